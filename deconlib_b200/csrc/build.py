@@ -19,7 +19,10 @@ ROOT = os.path.dirname(PKG)
 OBJ = os.path.join(ROOT, "_build", "obj")
 LIB = os.path.join(PKG, "libdecon_b200.so")
 SOURCES = ["capi.cu", "conv.cu", "reduce.cu", "ops.cu", "solvers.cu", "noalloc.cu", "batch.cu", "psf.cu", "nlcg.cu", "pdhg_run.cu", "pupil.cu",
-           "xstatic_r2c.cu", "xstatic_c2r.cu", "xstatic_col.cu"]
+           "fftplain.cu",
+           "colreg_a.cu", "colreg_b.cu", "colreg_c.cu", "colreg_d.cu", "colreg_e.cu",
+           "psf_any.cu", "psf_a.cu", "psf_b.cu", "psf_c.cu", "psf_d.cu", "psf_e.cu",
+           *(f"xreg_{d}_{g}.cu" for g in ("e", "d", "c", "b", "a", "odd") for d in ("c2r", "r2c"))]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -244,10 +244,7 @@ static int build_otf(decon_conv* p, const float* kernel, int normalize, cudaStre
     }
     Win3 none{0, 0, 0, 0, 0, 0};
     if ((st = launch_xr2c(*p, PRO_KERNEL, kernel, none, 0.f, 0.f, Fz, p->otf, s)) ||
-        (st = launch_col(*p, p->ax_y, p->T_y, COL_FWD, p->otf, Fy * p->P, p->P, (int)Fy, p->otf,
-                         Fy * p->P, p->P, (int)Fy, Fz, s)) ||
-        (st = launch_col(*p, p->ax_z, p->T_z, COL_FWD, p->otf, p->P, Fy * p->P, (int)Fz, p->otf,
-                         p->P, Fy * p->P, (int)Fz, Fy, s)) ||
+        (st = transform_otf(*p, 1, s)) || (st = transform_otf(*p, 0, s)) ||
         (st = max_abs2(p->otf, Fz * Fy, p->Hx, p->P, p->dscal + 1, p->partials, s)))
         return st;
     double nrm = 0;
@@ -325,7 +322,7 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
     p->ax_y.tws = 1;
     p->ax_z.tw = p->twz;
     p->ax_z.tws = 1;
-    p->npartials = std::max<int64_t>(reduce_partials_needed(), cdiv(nz * ny, p->T_x) + 1);
+    p->npartials = std::max<int64_t>(reduce_partials_needed(), cdiv(nz * ny, std::min(p->T_x, 4)) + 1);
     if ((st = dev_alloc((void**)&p->otf, (size_t)Fz * Fy * p->P * sizeof(float2), "OTF")) ||
         (st = dev_alloc((void**)&p->s1, (size_t)nz * ny * p->P * sizeof(float2), "spectrum S1")) ||
         (st = dev_alloc((void**)&p->s2, (size_t)nz * Fy * p->P * sizeof(float2), "spectrum S2")) ||
@@ -344,22 +341,9 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
         delete p;
         return st;
     }
-    // TMA tensor maps for the strided column passes (power-of-two lengths
-    // <= 512, 16-column tiles).  DECON_NO_TMA=1 selects the plain-load kernels.
-    {
-        const bool allow = getenv("DECON_NO_TMA") == nullptr;
-        const int64_t P = p->P;
-        p->s1_box = (int)std::min<int64_t>(ny, 256);
-        p->s2y_box = (int)std::min<int64_t>(Fy, 256);
-        p->s2z_box = (int)std::min<int64_t>(nz, 256);
-        p->otf_box = (int)std::min<int64_t>(Fz, 256);
-        p->tma_y = allow && tma_length_ok(p->ax_y.L) && p->T_y == 16 &&
-                   encode_spectrum_map(&p->tm_s1_j1, p->s1, P, ny, nz, p->s1_box, 1) &&
-                   encode_spectrum_map(&p->tm_s2_j1, p->s2, P, Fy, nz, p->s2y_box, 1);
-        p->tma_z = allow && tma_length_ok(p->ax_z.L) && p->T_z == 16 &&
-                   encode_spectrum_map(&p->tm_s2_j2, p->s2, P, Fy, nz, 1, p->s2z_box) &&
-                   encode_spectrum_map(&p->tm_otf_z, p->otf, P, Fy, Fz, 1, p->otf_box);
-    }
+    // DECON_NO_TMA=1: the plain-load column kernels
+    p->reg_ok = getenv("DECON_NO_TMA") == nullptr;
+    if (p->reg_ok) make_col_passes(*p);
     if ((st = build_otf(p, kernel, normalize, s))) {
         free_plan(p);
         delete p;
@@ -408,8 +392,7 @@ int decon_conv_set_precision(decon_conv* p, int precision, void* stream) {
     if (!p->otf_inv && (st = dev_alloc((void**)&p->otf_inv, (size_t)p->F[0] * sizeof(float), "OTF scales")))
         return st;
     DK_TRY(quantize_otf(*p, as_stream(stream)));
-    if (!p->tma_otf16)
-        p->tma_otf16 = encode_half_plane_map(&p->tm_otf16_z, p->otf16, p->P, p->F[1], p->F[0], p->otf_box);
+    if (!p->z_otf16.ok) make_z_otf16(*p);
     p->precision = 1;
     return DECON_OK;
 }
@@ -441,9 +424,7 @@ int decon_conv_set_schedule(decon_conv* p, int sched) {
         a.tw = axes[i]->tw;
         a.tws = axes[i]->tws;
         *axes[i] = a;
-        const bool runtime = !static_length(L);
-        *lines[i] = (runtime && (sched & DECON_SCHED_HALF_LINES) && lines0[i] >= 2) ? lines0[i] / 2
-                                                                                  : lines0[i];
+        *lines[i] = (sched & DECON_SCHED_HALF_LINES) && lines0[i] >= 2 ? lines0[i] / 2 : lines0[i];
     }
     if ((sched & DECON_SCHED_FUSED) && !p->otft && yz_supported(p->N, p->F) && p->F[0] != p->N[0]) {
         // the fused pass needs the kx-major OTF copy: allocate and fill it

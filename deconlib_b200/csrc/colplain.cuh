@@ -1,15 +1,13 @@
-// Plain-load column pass (passes 2-4 for lengths without a TMA kernel):
+// Plain-load column pass (passes 2-4 for lengths without a register kernel):
 // one CTA = T columns x L points of one plane, loaded with ordinary loads,
-// transformed in shared memory (compile-time radices for the static
-// lengths, the runtime-radix path otherwise), written back.
+// transformed in shared memory by the runtime-radix engine, written back.
 #pragma once
 
 #include "conv_impl.cuh"
 
 namespace dk {
 
-template <int LS>
-__global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, 1) k_colfft(ColArgs a) {
+__global__ void __launch_bounds__(kDynThreads, 1) k_colfft(ColArgs a) {
     extern __shared__ float2 sm[];
     const int T = a.T, L = a.ax.L, tid = threadIdx.x;
     const int64_t o = blockIdx.x / a.ntiles;
@@ -25,9 +23,9 @@ __global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, 1) k_colff
     __syncthreads();
     const int t = tid % T, jb = tid / T;
     if (a.mode == COL_INV) {
-        fft_lines<+1, LS>(sm, T, t, jb, a.ax);
+        fft_lines<+1>(sm, T, t, jb, a.ax);
     } else {
-        fft_lines<-1, LS>(sm, T, t, jb, a.ax);
+        fft_lines<-1>(sm, T, t, jb, a.ax);
     }
     if (a.mode == COL_OTF || a.mode == COL_OTF_CONJ) {
         const float2* otf = a.otf + o * a.otf_os + kx0;
@@ -40,7 +38,7 @@ __global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, 1) k_colff
             }
         }
         __syncthreads();
-        fft_lines<+1, LS>(sm, T, t, jb, a.ax);
+        fft_lines<+1>(sm, T, t, jb, a.ax);
     }
     float2* dst = a.dst + o * a.dst_os + kx0;
     for (int q = tid; q < a.nout * T; q += blockDim.x) {

@@ -1,0 +1,13 @@
+// Instantiations of the register column pass (colreg.cuh), lengths of DK_PAIR_LENGTHS_A.
+#include "colreg.cuh"
+
+namespace dk {
+
+ColRegKernel colreg_group_a(int L, int mode) {
+#define DK_CASE(n) if (L == n) return colreg_kernel<n>(mode);
+    DK_PAIR_LENGTHS_A(DK_CASE)
+#undef DK_CASE
+    return ColRegKernel{};
+}
+
+}  // namespace dk

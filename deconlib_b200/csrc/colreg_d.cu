@@ -1,0 +1,13 @@
+// Instantiations of the register column pass (colreg.cuh), lengths of DK_PAIR_LENGTHS_D.
+#include "colreg.cuh"
+
+namespace dk {
+
+ColRegKernel colreg_group_d(int L, int mode) {
+#define DK_CASE(n) if (L == n) return colreg_kernel<n>(mode);
+    DK_PAIR_LENGTHS_D(DK_CASE)
+#undef DK_CASE
+    return ColRegKernel{};
+}
+
+}  // namespace dk

@@ -27,76 +27,17 @@
 
 #include "conv_impl.cuh"
 #include "tma.cuh"
-#include "colpipe.cuh"
-#include "xpass.cuh"
+namespace dk {
+
+// Raised when a bounded mbarrier wait gives up (read by decon_device_status,
+// cleared by decon_device_status_clear); such a CTA skips its compute and store.
+static __device__ int g_wait_timeout = 0;
+
+}  // namespace dk
+
 #include "yzpass.cuh"
 
 namespace dk {
-
-// ---------------------------------------------------------------------------
-// passes 2-4 on TMA: the same column transform with the tile moved by
-// cp.async.bulk.tensor (one elected thread issues the boxes; an mbarrier with
-// a bounded wait signals arrival; results leave through a TMA store).
-// Power-of-two lengths L <= 512 with 16-column tiles (128-byte rows), so the
-// shared-memory tile uses the TMA 128-byte swizzle layout (physw<1>).
-// ---------------------------------------------------------------------------
-
-
-template <int LS>
-__global__ void __launch_bounds__(kFftThreads, (LS >= 512 ? 1 : 2)) k_colfft_tma(const __grid_constant__ ColTmaArgs a) {
-    extern __shared__ unsigned char smraw[];
-    float2* sm = reinterpret_cast<float2*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~uintptr_t(1023));
-    float2* so = sm + LS * 16;
-    __shared__ uint64_t bar;
-    const int tid = threadIdx.x;
-    const int o = blockIdx.x / a.ntiles;
-    const int c0 = (blockIdx.x - o * a.ntiles) * 32;  // float coordinate of the tile
-    const bool otf = a.mode == COL_OTF || a.mode == COL_OTF_CONJ;
-    const int nbox = (a.nin + a.src_box - 1) / a.src_box;
-    if (tid == 0) {
-        mbar_init(&bar, 1);
-        fence_proxy_async_smem();
-    }
-    __syncthreads();
-    if (tid == 0) {
-        const uint32_t bytes = (uint32_t)(nbox * a.src_box * 128) + (otf ? (uint32_t)(LS * 128) : 0u);
-        mbar_expect_tx(&bar, bytes);
-        for (int i = 0; i < nbox; ++i) {
-            const int r0 = i * a.src_box;
-            if (a.src_jdim == 1) tma_load_3d(sm + r0 * 16, &a.src, c0, r0, o, &bar);
-            else tma_load_3d(sm + r0 * 16, &a.src, c0, o, r0, &bar);
-        }
-        if (otf)
-            for (int r0 = 0; r0 < LS; r0 += a.otf_box) tma_load_3d(so + r0 * 16, &a.otf, c0, o, r0, &bar);
-    }
-    // rows the boxes do not cover are the implicit zero padding
-    for (int q = nbox * a.src_box * 16 + tid; q < LS * 16; q += blockDim.x) sm[q] = make_float2(0.f, 0.f);
-    const bool ok = __syncthreads_and(mbar_wait_bounded(&bar, 0));
-    if (!ok) return;
-    const int t = tid & 15, jb = tid >> 4;
-    if (a.mode == COL_INV) {
-        fft_lines_static<LS, +1, 1, 1>(sm, 16, t, jb, a.tw, a.tws);
-    } else {
-        fft_lines_static<LS, -1, 1, 1>(sm, 16, t, jb, a.tw, a.tws);
-    }
-    if (otf) {
-        for (int q = tid; q < LS * 16; q += blockDim.x) {
-            const float2 w = so[q];
-            sm[q] = a.mode == COL_OTF ? cmul(sm[q], w) : cmulc(sm[q], w);
-        }
-        __syncthreads();
-        fft_lines_static<LS, +1, 1, 1>(sm, 16, t, jb, a.tw, a.tws);
-    }
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-        for (int r0 = 0; r0 < a.nout; r0 += a.dst_box) {
-            if (a.dst_jdim == 1) tma_store_3d(&a.dst, c0, r0, o, sm + r0 * 16);
-            else tma_store_3d(&a.dst, c0, o, r0, sm + r0 * 16);
-        }
-        tma_store_commit_and_wait();
-    }
-}
 
 // ---------------------------------------------------------------------------
 // host: axis planning and launches
@@ -134,7 +75,7 @@ bool plan_axis(int L, Axis& ax, int order) {
     if (n != 1 || (int)r.size() > kMaxStages) return false;
     ax.nst = (int)r.size();
     for (int i = 0; i < ax.nst; ++i) ax.rad |= (unsigned long long)r[i] << (4 * i);
-    ax.tpl = static_length(L) ? (L + 31) / 32 : (L + kDynPPT - 1) / kDynPPT;
+    ax.tpl = (L + kDynPPT - 1) / kDynPPT;
     return true;
 }
 
@@ -192,11 +133,8 @@ int kernel_prepare(void* fn, size_t smem, int nthr, int* per_sm) {
     return DECON_OK;
 }
 
-static int launch(void* fn, int64_t nblk, int nthr, size_t smem, cudaStream_t st, void* args,
-                  int cls) {
+static int launch(void* fn, dim3 grid, int nthr, size_t smem, cudaStream_t st, void* args, int cls) {
     DK_TRY(kernel_prepare(fn, smem, nthr, nullptr));
-    if (nblk <= 0) return DECON_OK;
-    if (nblk > 0x7fffffffLL) return fail(DECON_ERR_UNSUPPORTED, "grid too large");
     void* params[] = {args};
     const bool prof = (g_prof.mask & cls) != 0;
     if (prof) {
@@ -208,13 +146,19 @@ static int launch(void* fn, int64_t nblk, int nthr, size_t smem, cudaStream_t st
         }
         DK_CUDA(cudaEventRecord(g_prof.ev[g_prof.used].first, st));
     }
-    DK_CUDA(cudaLaunchKernel(fn, dim3((unsigned)nblk), dim3(nthr), params, smem, st));
+    DK_CUDA(cudaLaunchKernel(fn, grid, dim3(nthr), params, smem, st));
     count_launch();
     if (prof) {
         DK_CUDA(cudaEventRecord(g_prof.ev[g_prof.used].second, st));
         ++g_prof.used;
     }
     return DECON_OK;
+}
+
+static int launch(void* fn, int64_t nblk, int nthr, size_t smem, cudaStream_t st, void* args, int cls) {
+    if (nblk <= 0) return kernel_prepare(fn, smem, nthr, nullptr);
+    if (nblk > 0x7fffffffLL) return fail(DECON_ERR_UNSUPPORTED, "grid too large");
+    return launch(fn, dim3((unsigned)nblk), nthr, smem, st, args, cls);
 }
 
 }  // namespace dk
@@ -249,7 +193,7 @@ __global__ void k_wait_probe(unsigned polls) {
         fence_proxy_async_smem();
     }
     __syncthreads();
-    if (threadIdx.x == 0) (void)mbar_wait_bounded(&bar, 0, polls);
+    if (threadIdx.x == 0) (void)mbar_wait_bounded(&bar, 0, &g_wait_timeout, polls);
 }
 
 }  // namespace dk
@@ -287,8 +231,66 @@ extern "C" int decon_profile_stop(double* ms_total, int64_t* launches) {
 
 namespace dk {
 
+#define DK_XREG_PICK(kind)                                        \
+    static XRegKernel pick_xreg_##kind(int L, bool odd, int what) { \
+        if (odd) return xreg_##kind##_odd(L, what);                 \
+        for (auto group : {xreg_##kind##_a, xreg_##kind##_b, xreg_##kind##_c, xreg_##kind##_d, xreg_##kind##_e}) { \
+            const XRegKernel k = group(L, what);                    \
+            if (k.fn) return k;                                     \
+        }                                                           \
+        return XRegKernel{};                                        \
+    }
+DK_XREG_PICK(r2c)
+DK_XREG_PICK(c2r)
+#undef DK_XREG_PICK
+
+static bool is_full_window(const ConvPlan& p, const Win3& w) {
+    return w.oz == 0 && w.oy == 0 && w.ox == 0 && w.wz == p.N[0] && w.wy == p.N[1] && w.wx == p.N[2];
+}
+
+static bool pair_aligned(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0; }
+
+// The fields both register X passes share.
+static XRegArgs xreg_args(const ConvPlan& p, int64_t nrows, int64_t Ny, int64_t Nx) {
+    XRegArgs a{};
+    const int L = p.ax_x.L;
+    a.Ny = Ny;
+    a.Nx = Nx;
+    a.P = p.P;
+    a.nrows = (uint32_t)nrows;
+    a.nlines = (uint32_t)(p.odd ? cdiv(nrows, 2) : nrows);
+    a.nin = a.nout = (int)std::min<int64_t>(p.odd ? Nx : cdiv(Nx, 2), L);
+    a.tw = p.ax_x.tw;
+    a.tws = p.ax_x.tws;
+    a.twx = p.twx;
+    return a;
+}
+
 int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cval, float bg,
                 int64_t nz_rows, float2* out, cudaStream_t st, int64_t kstride) {
+    const int src = pro == PRO_ARRAY ? 0 : pro == PRO_UP2 ? 1 : 2;
+    const XRegKernel k = p.reg_ok && kstride == 0 && (pro == PRO_KERNEL || pro == PRO_UP2 || is_full_window(p, win))
+                             ? pick_xreg_r2c(p.ax_x.L, p.odd, src)
+                             : XRegKernel{};
+    if (k.fn) {
+        const int64_t Ny = pro == PRO_KERNEL ? p.F[1] : p.N[1], Nx = pro == PRO_KERNEL ? p.F[2] : p.N[2];
+        XRegArgs a = xreg_args(p, nz_rows * Ny, Ny, Nx);
+        a.pro = pro;
+        a.in = in;
+        a.cval = cval;
+        a.bg = bg;
+        a.kdiv = p.kdiv;
+        a.Nz = nz_rows;
+        a.Kz = p.K[0];
+        a.Ky = p.K[1];
+        a.Kx = p.K[2];
+        a.pz = (p.K[0] + 1) / 2;
+        a.py = (p.K[1] + 1) / 2;
+        a.px = (p.K[2] + 1) / 2;
+        a.out = out;
+        a.vec = Nx % 2 == 0 && pair_aligned(in);
+        return launch(k.fn, cdiv(a.nlines, k.TL), k.nt, k.smem, st, &a, PROF_XR2C);
+    }
     XR2CArgs a{};
     a.kstride = kstride;
     a.in = in;
@@ -319,8 +321,6 @@ int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cva
     if (pro == PRO_UP2) a.vec4 = up2_vec;
     a.T = p.T_x;
     a.nrows = nz_rows * a.Ny;
-    if (static_length(a.ax.L))
-        if (a.T != x_lines(a.ax.L)) return fail(DECON_ERR_UNSUPPORTED, "X pass lines per CTA mismatch");
     {
         const int L = a.ax.L;
         const int64_t nin = p.odd ? std::min<int64_t>(a.Nx, L) : std::min<int64_t>((a.Nx + 1) / 2, L);
@@ -332,7 +332,7 @@ int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cva
     const int nthr = threads_for(a.T, a.ax);
     const int64_t nblk = cdiv(a.nrows, a.T);
     const size_t smem = (size_t)a.T * a.ax.L * sizeof(float2);
-    void* fn = pick_xr2c_kernel(pro, a.ax.L);
+    void* fn = pick_xr2c_kernel(pro);
     if (!fn) return fail(DECON_ERR_VALUE, "bad prologue %d", pro);
     return launch(fn, nblk, nthr, smem, st, &a, PROF_XR2C);
 }
@@ -360,13 +360,33 @@ int launch_col(const ConvPlan& p, const Axis& ax, int T, int mode, const float2*
     const int nthr = threads_for(T, ax);
     const int64_t nblk = nouter * a.ntiles;
     const size_t smem = (size_t)T * ax.L * sizeof(float2);
-    return launch(pick_colfft_kernel(ax.L), nblk, nthr, smem, st, &a,
+    return launch(pick_colfft_kernel(), nblk, nthr, smem, st, &a,
                   (mode == COL_OTF || mode == COL_OTF_CONJ) ? PROF_ZOTF : PROF_COL);
 }
 
 int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* out,
                 const float* aux0, const float* aux1, float bg, double* partials, int* nblk_out,
                 cudaStream_t st) {
+    const XRegKernel k = p.reg_ok && !use_yz(p) && is_full_window(p, win)
+                             ? pick_xreg_c2r(p.ax_x.L, p.odd, epi)
+                             : XRegKernel{};
+    if (k.fn) {
+        if (epi == EPI_DOWN2 && (p.odd || (p.N[0] | p.N[1] | p.N[2]) & 1))
+            return fail(DECON_ERR_UNSUPPORTED, "2x area-sum epilogue: extents must be even");
+        XRegArgs a = xreg_args(p, p.N[0] * p.N[1], p.N[1], p.N[2]);
+        a.spec = in;
+        a.out_real = out;
+        a.aux0 = aux0;
+        a.aux1 = aux1;
+        a.bg = bg;
+        a.pred = epi == EPI_PRED;
+        a.partials = partials;
+        a.scale = (float)(1.0 / ((double)p.F[0] * (double)p.F[1] * (double)p.F[2]));
+        a.vec = p.N[2] % 2 == 0 && pair_aligned(out) && pair_aligned(aux0) && pair_aligned(aux1);
+        const int64_t nblk = cdiv(a.nlines, k.TL);
+        if (nblk_out) *nblk_out = (int)nblk;
+        return launch(k.fn, nblk, k.nt, k.smem, st, &a, PROF_XC2R);
+    }
     XC2RArgs a{};
     a.in = in;
     a.P = p.P;
@@ -384,8 +404,6 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
         a.vec4 = full && !p.odd && (p.N[2] % 4) == 0 && al(out) && al(aux0) && al(aux1);
     }
     a.T = p.T_x;
-    if (static_length(a.ax.L))
-        if (a.T != x_lines(a.ax.L)) return fail(DECON_ERR_UNSUPPORTED, "X pass lines per CTA mismatch");
     a.scale = (float)(1.0 / ((double)p.F[0] * (double)p.F[1] * (double)p.F[2]));
     a.win = win;
     a.out = out;
@@ -413,32 +431,9 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
     const int64_t nblk = cdiv(a.nrows, a.T);
     if (nblk_out) *nblk_out = (int)nblk;
     const size_t smem = (size_t)a.T * a.ax.L * sizeof(float2);
-    void* fn = pick_xc2r_kernel(epi, a.ax.L);
+    void* fn = pick_xc2r_kernel(epi);
     if (!fn) return fail(DECON_ERR_VALUE, "bad epilogue %d", epi);
     return launch(fn, nblk, nthr, smem, st, &a, PROF_XC2R);
-}
-
-static void* pick_col_tma(int L) {
-    switch (L) {
-        case 64: return (void*)k_colfft_tma<64>;
-        case 128: return (void*)k_colfft_tma<128>;
-        case 256: return (void*)k_colfft_tma<256>;
-        case 512: return (void*)k_colfft_tma<512>;
-        case 80: return (void*)k_colfft_tma<80>;
-        case 96: return (void*)k_colfft_tma<96>;
-        case 160: return (void*)k_colfft_tma<160>;
-        case 192: return (void*)k_colfft_tma<192>;
-        case 240: return (void*)k_colfft_tma<240>;
-        default: return nullptr;
-    }
-}
-
-// Lengths with a TMA column kernel: the powers of two up to 512, and the
-// other compile-time lengths up to 256 (one TMA box spans the whole line, so
-// no box reaches past the tile).
-bool tma_length_ok(int L) {
-    return L == 64 || L == 128 || L == 256 || L == 512 || L == 80 || L == 96 || L == 160 || L == 192 ||
-           L == 240;
 }
 
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -458,170 +453,142 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return enc;
 }
 
-bool encode_half_plane_map(CUtensorMap* map, const __half2* base, int64_t pitch, int64_t d1, int64_t d2,
-                           int b2) {
+bool encode_tile_map(CUtensorMap* map, const void* base, int esize, int64_t pitch, int64_t d1, int64_t d2,
+                     int T, int b1, int b2) {
     const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
     if (!enc) return false;
-    // one half2 = one 4-byte element; rows of 16 elements (64 bytes), no swizzle
-    cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)d1, (cuuint64_t)d2};
-    cuuint64_t strides[2] = {(cuuint64_t)(pitch * sizeof(__half2)),
-                             (cuuint64_t)(pitch * sizeof(__half2) * d1)};
-    cuuint32_t box[3] = {16u, 1u, (cuuint32_t)b2};
+    const int f = esize / 4;  // 4-byte map elements per complex value
+    cuuint64_t dims[3] = {(cuuint64_t)(f * pitch), (cuuint64_t)d1, (cuuint64_t)d2};
+    cuuint64_t strides[2] = {(cuuint64_t)(pitch * esize), (cuuint64_t)(pitch * esize * d1)};
+    cuuint32_t box[3] = {(cuuint32_t)(f * T), (cuuint32_t)b1, (cuuint32_t)b2};
     cuuint32_t estr[3] = {1u, 1u, 1u};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<__half2*>(base), dims, strides,
-                     box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box,
+                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
 
-bool encode_spectrum_map(CUtensorMap* map, const float2* base, int64_t pitch, int64_t d1, int64_t d2,
-                         int b1, int b2) {
-    const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-    if (!enc) return false;
-    cuuint64_t dims[3] = {(cuuint64_t)(2 * pitch), (cuuint64_t)d1, (cuuint64_t)d2};
-    cuuint64_t strides[2] = {(cuuint64_t)(2 * pitch * sizeof(float)),
-                             (cuuint64_t)(2 * pitch * sizeof(float) * d1)};
-    cuuint32_t box[3] = {32u, (cuuint32_t)b1, (cuuint32_t)b2};
-    cuuint32_t estr[3] = {1u, 1u, 1u};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float2*>(base), dims, strides,
-                     box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
+// ---------------------------------------------------------------------------
+// register column passes (colreg.cuh)
+// ---------------------------------------------------------------------------
+
+// DECON_NO_PIPE / DECON_SCHED_NO_PIPE: the FP32 OTF also for a mixed plan.
+static bool no_pipe(const ConvPlan& p) {
+    return getenv("DECON_NO_PIPE") != nullptr || (p.sched & DECON_SCHED_NO_PIPE) != 0;
 }
 
-// One column pass on TMA.  src/dst/otf maps come from the plan.
-// Pipelined kernel for (L, mode, nin, nout), or nullptr.  R x R (SPLIT 1) for
-// L = 64, 256; the half-zero split (SPLIT 2) for L = 128, 512 when the
-// non-zero input / kept output fits in half the axis.
-// h16: the axial (OTF) modes read the FP16 OTF (mixed precision).
-static void* pick_pipe(int L, int mode, int nin, int nout, int* R, int* split, bool h16 = false,
-                       bool lean = false) {
-    const bool otf = mode == COL_OTF || mode == COL_OTF_CONJ;
-    const bool half_ok = (mode == COL_FWD && nin <= L / 2) || (mode == COL_INV && nout <= L / 2) ||
-                         (otf && nin <= L / 2 && nout <= L / 2);
-#define DK_PIPE(RR, SS)                                                                          \
-    do {                                                                                         \
-        *R = RR;                                                                                 \
-        *split = SS;                                                                             \
-        switch (mode) {                                                                          \
-            case COL_FWD: return (void*)k_col_pipe<RR, SS, COL_FWD>;                             \
-            case COL_INV: return (void*)k_col_pipe<RR, SS, COL_INV>;                             \
-            case COL_OTF:                                                                        \
-                return h16 ? (lean ? (void*)k_col_pipe<RR, SS, COL_OTF, true, true>              \
-                                   : (void*)k_col_pipe<RR, SS, COL_OTF, true>)                  \
-                           : (lean ? (void*)k_col_pipe<RR, SS, COL_OTF, false, true>            \
-                                   : (void*)k_col_pipe<RR, SS, COL_OTF>);                       \
-            case COL_OTF_CONJ:                                                                   \
-                return h16 ? (lean ? (void*)k_col_pipe<RR, SS, COL_OTF_CONJ, true, true>         \
-                                   : (void*)k_col_pipe<RR, SS, COL_OTF_CONJ, true>)             \
-                           : (lean ? (void*)k_col_pipe<RR, SS, COL_OTF_CONJ, false, true>       \
-                                   : (void*)k_col_pipe<RR, SS, COL_OTF_CONJ>);                  \
-        }                                                                                        \
-    } while (0)
-    if (L == 256) DK_PIPE(16, 1);
-    if (L == 64) DK_PIPE(8, 1);
-    if (L == 128 && half_ok) DK_PIPE(8, 2);
-#undef DK_PIPE
-    if (L == 512 && half_ok && !otf) {
-        *R = 16;
-        *split = 2;
-        return mode == COL_FWD ? (void*)k_col_pipe<16, 2, COL_FWD> : (void*)k_col_pipe<16, 2, COL_INV>;
+static ColRegKernel pick_colreg(int L, int mode) {
+    for (auto group : {colreg_group_a, colreg_group_b, colreg_group_c, colreg_group_d, colreg_group_e}) {
+        const ColRegKernel k = group(L, mode);
+        if (k.fn) return k;
     }
-    return nullptr;
+    return ColRegKernel{};
 }
 
-static bool launch_col_pipe(const ConvPlan& p, const Axis& ax, int mode, const CUtensorMap& src,
-                            int src_jdim, int src_box, int nin, const CUtensorMap& dst, int dst_jdim,
-                            int dst_box, int nout, int64_t nouter, cudaStream_t st, int* status) {
-    int R = 0, split = 0;
-    const bool otf_mode = mode == COL_OTF || mode == COL_OTF_CONJ;
-    const bool h16 = otf_mode && p.precision == 1 && p.otf16 != nullptr;
-    // axial pass of length 256: the lean two-CTA kernel (measured 153 vs 166 us
-    // at 128x256x256 on the B200); DECON_PIPE_LEAN=0 / 1 overrides.  Its FP16
-    // form stages the half OTF tile by TMA (needs the plan's half-OTF map).
-    const char* le = getenv("DECON_PIPE_LEAN");
-    const bool lean = otf_mode && (!h16 || p.tma_otf16) &&
-                      (le ? le[0] == '1' : (ax.L == 256 && !(p.sched & DECON_SCHED_LEAN_OFF)));
-    const bool no_pipe = getenv("DECON_NO_PIPE") || (p.sched & DECON_SCHED_NO_PIPE);
-    void* fn = no_pipe ? nullptr : pick_pipe(ax.L, mode, nin, nout, &R, &split, h16, lean);
-    if (!fn) return false;
-    PipeArgs a;
+// Boxes of at most 256 rows covering n rows, each a multiple of 128 bytes (the
+// shared-memory alignment of a TMA box); rows past the buffer read as zero.
+static void split_rows(int n, int row_bytes, int* box, int* nbox) {
+    *nbox = (n + 255) / 256;
+    const int even = 128 / std::min(128, row_bytes);
+    *box = (int)round_up(cdiv(n, *nbox), even);
+}
+
+// A column pass along dimension jdim (1: rows adjacent in a plane, 2: planes)
+// of src [s2][s1][P] into dst with the same dimension order.
+static bool make_col_pass(const ConvPlan& p, ColPass& c, const Axis& ax, int mode, int jdim,
+                          const float2* src, int64_t s1, int64_t s2, int nin, float2* dst, int64_t d1,
+                          int nout, int64_t nouter) {
+    c.ok = false;
+    c.k = pick_colreg(ax.L, mode);
+    if (!c.k.fn) return false;
+    ColRegArgs& a = c.a;
     memset(&a, 0, sizeof(a));
+    const int T = c.k.T;
     a.src = src;
     a.dst = dst;
-    a.otf = p.otf;
-    a.otf16 = p.otf16;
-    a.otf_inv = p.otf_inv;
-    a.otfmap = p.tm_otf_z;
-    a.otfmap16 = p.tm_otf16_z;
-    a.otf_box = p.otf_box;
-    a.otf_js = p.F[1] * p.P;
-    a.otf_os = p.P;
-    a.tw = ax.tw;
-    a.tws = ax.tws;
+    a.src_os = jdim == 1 ? s1 * p.P : p.P;
+    a.src_js = jdim == 1 ? p.P : s1 * p.P;
+    a.dst_os = jdim == 1 ? d1 * p.P : p.P;
+    a.dst_js = jdim == 1 ? p.P : d1 * p.P;
     a.nin = nin;
     a.nout = nout;
-    a.ntiles = (int)cdiv(p.Hx, 16);
     a.nouter = (int)nouter;
-    a.src_jdim = src_jdim;
-    a.dst_jdim = dst_jdim;
-    a.src_box = src_box;
-    a.dst_box = dst_box;
-    const int L = ax.L;
-    const int ns = pipe_slots(L, lean);
-    // OTF tile: FP32 in each ring slot, or (lean) one buffer of FP32 or FP16
-    const bool otf_tile = otf_mode && !h16;
-    const size_t tile_bytes = (size_t)L * 16 * sizeof(float2);
-    const size_t smem = 1024 + (size_t)ns * tile_bytes * (otf_tile && !lean ? 2 : 1) +
-                        (otf_mode && lean ? (h16 ? tile_bytes / 2 : tile_bytes) : 0);
-    const int nthr = 16 * R;
-    *status = DECON_OK;
-    int per_sm = 1;
-    if ((*status = kernel_prepare(fn, smem, nthr, &per_sm)) != DECON_OK) return true;
-    if (per_sm < 1) per_sm = 1;
-    const int64_t total = nouter * a.ntiles;
-    const int64_t grid = std::min<int64_t>(total, (int64_t)sm_count() * per_sm);
-    *status = launch(fn, grid, nthr, smem, st, &a,
-                     (mode == COL_OTF || mode == COL_OTF_CONJ) ? PROF_ZOTF : PROF_COL);
-    return true;
+    a.jdim = jdim;
+    a.tw = ax.tw;
+    a.tws = ax.tws;
+    a.conj = 1.f;
+    a.nfull = (int)(p.Hx / T);
+    a.rem = (int)(p.Hx - (int64_t)a.nfull * T);
+    a.per = a.rem ? T / a.rem : 1;
+    const int64_t nmain = nouter * a.nfull, ntiles = nmain + (a.rem ? cdiv(nouter, a.per) : 0);
+    if (ntiles > 0x7fffffffLL - 65536) return false;
+    a.nmain = (int)nmain;
+    a.ntiles = (int)ntiles;
+    split_rows(nin, T * 8, &a.box, &a.nbox);
+    a.in_bytes = a.nbox * a.box * T * 8;
+    if (!encode_tile_map(&a.srcmap, src, 8, p.P, s1, s2, T, jdim == 1 ? a.box : 1, jdim == 1 ? 1 : a.box))
+        return false;
+    c.smem = c.k.exch + a.in_bytes;
+    if (mode == 2 || mode == 3) {
+        const int esize = mode == 3 ? 4 : 8;
+        a.otf = p.otf;
+        a.otf16 = p.otf16;
+        a.otf_inv = p.otf_inv;
+        a.otf_os = p.P;
+        a.otf_js = p.F[1] * p.P;
+        split_rows(ax.L, T * esize, &a.obox, &a.onbox);
+        if (!encode_tile_map(&a.otfmap, mode == 3 ? (const void*)p.otf16 : (const void*)p.otf, esize, p.P,
+                             p.F[1], p.F[0], T, 1, a.obox))
+            return false;
+        c.smem += a.onbox * a.obox * T * esize;
+    }
+    void* flag = nullptr;
+    int per_sm = 0;
+    if (c.smem > 227 * 1024 || cudaGetSymbolAddress(&flag, g_wait_timeout) != cudaSuccess ||
+        kernel_prepare(c.k.fn, c.smem, c.k.nt, &per_sm) != DECON_OK || per_sm < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    a.flag = static_cast<int*>(flag);
+    c.grid = (int)std::min<int64_t>(ntiles, (int64_t)sm_count() * per_sm);
+    return c.ok = true;
+}
+
+void make_col_passes(ConvPlan& p) {
+    const int64_t Nz = p.N[0], Ny = p.N[1], Fy = p.F[1];
+    make_col_pass(p, p.y_fwd, p.ax_y, 0, 1, p.s1, Ny, Nz, (int)Ny, p.s2, Fy, (int)Fy, Nz);
+    make_col_pass(p, p.z_otf, p.ax_z, 2, 2, p.s2, Fy, Nz, (int)Nz, p.s2, Fy, (int)Nz, Fy);
+    make_col_pass(p, p.y_inv, p.ax_y, 1, 1, p.s2, Fy, Nz, (int)Fy, p.s1, Ny, (int)Ny, Nz);
+}
+
+void make_z_otf16(ConvPlan& p) {
+    const int64_t Nz = p.N[0], Fy = p.F[1];
+    make_col_pass(p, p.z_otf16, p.ax_z, 3, 2, p.s2, Fy, Nz, (int)Nz, p.s2, Fy, (int)Nz, Fy);
+}
+
+static int launch_col_pass(const ConvPlan&, const ColPass& c, bool conj, cudaStream_t st) {
+    ColRegArgs a = c.a;
+    if (conj) a.conj = -1.f;
+    return launch(c.k.fn, c.grid, c.k.nt, c.smem, st, &a, a.otf ? PROF_ZOTF : PROF_COL);
+}
+
+int transform_otf(const ConvPlan& p, int axis, cudaStream_t st) {
+    const int64_t Fz = p.F[0], Fy = p.F[1], P = p.P;
+    const int n = (int)p.F[axis];
+    const Axis& ax = axis == 1 ? p.ax_y : p.ax_z;
+    ColPass c;
+    if (p.reg_ok && make_col_pass(p, c, ax, 0, axis == 1 ? 1 : 2, p.otf, Fy, Fz, n, p.otf, Fy, n,
+                                  axis == 1 ? Fz : Fy))
+        return launch_col_pass(p, c, false, st);
+    if (axis == 1)
+        return launch_col(p, ax, p.T_y, COL_FWD, p.otf, Fy * P, P, n, p.otf, Fy * P, P, n, Fz, st);
+    return launch_col(p, ax, p.T_z, COL_FWD, p.otf, P, Fy * P, n, p.otf, P, Fy * P, n, Fy, st);
 }
 
 bool zpass_pipelined(const ConvPlan& p) {
-    if (!p.tma_z || getenv("DECON_NO_PIPE") || (p.sched & (DECON_SCHED_NO_PIPE | DECON_SCHED_NO_TMA)))
-        return false;
-    int R = 0, split = 0;
-    return pick_pipe(p.ax_z.L, COL_OTF, (int)p.N[0], (int)p.N[0], &R, &split) != nullptr;
-}
-
-static int launch_col_tma(const ConvPlan& p, const Axis& ax, int mode, const CUtensorMap& src,
-                          int src_jdim, int src_box, int nin, const CUtensorMap& dst, int dst_jdim,
-                          int dst_box, int nout, int64_t nouter, cudaStream_t st) {
-    int pst = DECON_OK;
-    if (launch_col_pipe(p, ax, mode, src, src_jdim, src_box, nin, dst, dst_jdim, dst_box, nout,
-                        nouter, st, &pst))
-        return pst;
-    ColTmaArgs a;
-    memset(&a, 0, sizeof(a));
-    a.src = src;
-    a.dst = dst;
-    if (mode == COL_OTF || mode == COL_OTF_CONJ) a.otf = p.tm_otf_z;
-    a.nin = nin;
-    a.nout = nout;
-    a.ntiles = (int)cdiv(p.Hx, 16);
-    a.mode = mode;
-    a.src_jdim = src_jdim;
-    a.dst_jdim = dst_jdim;
-    a.src_box = src_box;
-    a.dst_box = dst_box;
-    a.otf_box = p.otf_box;
-    a.tw = ax.tw;
-    a.tws = ax.tws;
-    const int L = ax.L;
-    const int nthr = std::max(64, 16 * ((L + 31) / 32));  // 16 lines x the static path's threads per line
-    const bool otf = mode == COL_OTF || mode == COL_OTF_CONJ;
-    const size_t smem = 1024 + (size_t)L * 16 * sizeof(float2) * (otf ? 2 : 1);
-    return launch(pick_col_tma(L), nouter * a.ntiles, nthr, smem, st, &a,
-                  otf ? PROF_ZOTF : PROF_COL);
+    if (!p.z_otf.ok || no_pipe(p) || (p.sched & DECON_SCHED_NO_TMA)) return false;
+    const int L = p.ax_z.L;
+    return L == 64 || L == 256 || (L == 128 && p.N[0] <= 64);
 }
 
 // ---------------------------------------------------------------------------
@@ -789,9 +756,8 @@ int spectrum_forward(const ConvPlan& p, int pro, const float* in, Win3 win, floa
     const int64_t Nz = p.N[0], Ny = p.N[1], Fy = p.F[1], P = p.P;
     if (use_yz(p)) return launch_xr2c(p, pro, in, win, cval, bg, Nz, p.s1, st, Nz * Ny);
     DK_TRY(launch_xr2c(p, pro, in, win, cval, bg, Nz, p.s1, st));
-    if (p.tma_y && !(p.sched & DECON_SCHED_NO_TMA)) {
-        DK_TRY(launch_col_tma(p, p.ax_y, COL_FWD, p.tm_s1_j1, 1, p.s1_box, (int)Ny, p.tm_s2_j1, 1,
-                              p.s2y_box, (int)Fy, Nz, st));
+    if (p.y_fwd.ok && !(p.sched & DECON_SCHED_NO_TMA)) {
+        DK_TRY(launch_col_pass(p, p.y_fwd, false, st));
     } else {
         DK_TRY(launch_col(p, p.ax_y, p.T_y, COL_FWD, p.s1, Ny * P, P, (int)Ny, p.s2, Fy * P, P,
                           (int)Fy, Nz, st));
@@ -804,17 +770,16 @@ int spectrum_filter_back(const ConvPlan& p, bool adjoint, cudaStream_t st) {
     if (use_yz(p)) return launch_yz(p, adjoint, st);
     const int64_t Nz = p.N[0], Ny = p.N[1], Fy = p.F[1], P = p.P;
     const int mode = adjoint ? COL_OTF_CONJ : COL_OTF;
-    const bool tma = !(p.sched & DECON_SCHED_NO_TMA);
-    if (p.tma_z && tma) {
-        DK_TRY(launch_col_tma(p, p.ax_z, mode, p.tm_s2_j2, 2, p.s2z_box, (int)Nz, p.tm_s2_j2, 2,
-                              p.s2z_box, (int)Nz, Fy, st));
+    const bool reg = !(p.sched & DECON_SCHED_NO_TMA);
+    if (p.z_otf.ok && reg) {
+        const bool h16 = p.precision == 1 && p.z_otf16.ok && !no_pipe(p);
+        DK_TRY(launch_col_pass(p, h16 ? p.z_otf16 : p.z_otf, adjoint, st));
     } else {
         DK_TRY(launch_col(p, p.ax_z, p.T_z, mode, p.s2, P, Fy * P, (int)Nz, p.s2, P, Fy * P,
                           (int)Nz, Fy, st));
     }
-    if (p.tma_y && tma) {
-        DK_TRY(launch_col_tma(p, p.ax_y, COL_INV, p.tm_s2_j1, 1, p.s2y_box, (int)Fy, p.tm_s1_j1, 1,
-                              p.s1_box, (int)Ny, Nz, st));
+    if (p.y_inv.ok && reg) {
+        DK_TRY(launch_col_pass(p, p.y_inv, false, st));
     } else {
         DK_TRY(launch_col(p, p.ax_y, p.T_y, COL_INV, p.s2, Fy * P, P, (int)Fy, p.s1, Ny * P, P,
                           (int)Ny, Nz, st));

@@ -11,17 +11,13 @@
 namespace dk {
 
 constexpr int kSmemElems = 8192;  // complex values per CTA (64 KB)
-// T lines x L points <= kSmemElems and ceil(L/32) threads per line bound a
-// CTA to kSmemElems / 32 threads.
-constexpr int kFftThreads = kSmemElems / 32;
 
-// Lines per CTA for an axis: the largest power of two <= cap whose tile fits
-// kSmemElems complex values and whose threads (T x tpl) fit the CTA limit of
-// the length's path.
+// Lines per CTA of the runtime-radix passes: the largest power of two <= cap
+// whose tile fits kSmemElems complex values and whose threads (T x tpl) fit a
+// CTA.
 inline int fft_lines_per_cta(const Axis& ax, int cap) {
-    const int lim = static_length(ax.L) ? kFftThreads : kDynThreads;
     int T = 1;
-    while (T * 2 <= cap && (T * 2) * ax.L <= kSmemElems && (T * 2) * ax.tpl <= lim) T *= 2;
+    while (T * 2 <= cap && (T * 2) * ax.L <= kSmemElems && (T * 2) * ax.tpl <= kDynThreads) T *= 2;
     return T;
 }
 
@@ -43,6 +39,22 @@ enum Epilogue { EPI_STORE = 0, EPI_RL_RATIO = 1, EPI_RL_UPDATE = 2, EPI_PRED = 3
 enum ColMode { COL_FWD = 0, COL_INV = 1, COL_OTF = 2, COL_OTF_CONJ = 3 };
 // kernel classes for decon_profile_start (bit mask)
 enum ProfClass { PROF_XR2C = 1, PROF_COL = 2, PROF_ZOTF = 4, PROF_XC2R = 8 };
+
+__device__ __forceinline__ bool kernel_src(int64_t c, int64_t F, int64_t m, int64_t npos,
+                                           int64_t& k) {
+    // Corner-origin embedding (utils/padding.py:142-190): canvas index c holds
+    // kernel index c (c < npos) or c - F + m (the wrapped negative offsets).
+    if (c < npos) {
+        k = c;
+        return c < m;
+    }
+    const int64_t nneg = m - npos;
+    if (c >= F - nneg) {
+        k = c - F + m;
+        return true;
+    }
+    return false;
+}
 
 struct XR2CArgs {
     const float* in;
@@ -72,29 +84,76 @@ struct ColArgs {
     int64_t otf_js, otf_os;
 };
 
-struct ColTmaArgs {
-    CUtensorMap src, dst, otf;  // 64-byte aligned descriptors
-    int nin, nout, ntiles, mode;
-    int src_jdim, dst_jdim, src_box, dst_box, otf_box;
+// Register column pass (k_colreg, colreg.cuh): tile geometry, tensor maps of
+// the rows that come by TMA, and the plain addresses of the same rows.
+struct ColRegArgs {
+    CUtensorMap srcmap, otfmap;
+    const float2* src;
+    float2* dst;
+    int64_t src_os, src_js, dst_os, dst_js;
+    int nin, nout, nouter;
+    int nfull, rem, per;   // full tiles per plane, columns past them, planes per tile of those
+    int nmain, ntiles;     // full tiles, all tiles
+    int jdim, box, nbox;   // source map: dimension of the rows, rows per box, boxes
+    int obox, onbox, in_bytes;
+    const float2* tw;      // W_L table, W_L^m = tw[m * tws]
     int tws;
-    const float2* tw;
-};
-
-// Persistent pipelined column pass (k_col_pipe).
-struct PipeArgs {
-    CUtensorMap src, dst;
-    CUtensorMap otfmap;     // FP32 OTF [Fz][Fy][P] as TMA boxes (axial pass)
-    CUtensorMap otfmap16;   // FP16 OTF [Fz][Fy][P] half2, (16, 1, otf_box) boxes (lean mixed axial pass)
-    int otf_box;
-    const float2* otf;      // OTF base for the axial pass
-    const __half2* otf16;   // mixed precision: FP16 OTF, OTF = otf16 * otf_inv[kz]
+    float conj;            // -1: multiply by conj(OTF)
+    const float2* otf;
+    const __half2* otf16;  // mixed precision: OTF = otf16 * otf_inv[kz]
     const float* otf_inv;
-    int64_t otf_js, otf_os; // complex-element strides of OTF rows (kz) and planes (ky)
-    const float2* tw;       // W_L table, W_L^m = tw[m * tws]
-    int tws;
-    int nin, nout, ntiles, nouter;
-    int src_jdim, dst_jdim, src_box, dst_box;
+    int64_t otf_os, otf_js;
+    int* flag;             // raised when a bounded wait gives up
 };
+struct ColRegKernel {
+    void* fn = nullptr;
+    int T = 0, nt = 0, exch = 0;
+};
+// One column pass of a plan, ready to launch.
+struct ColPass {
+    ColRegKernel k;
+    ColRegArgs a;
+    int smem = 0, grid = 0;
+    bool ok = false;
+};
+ColRegKernel colreg_group_a(int L, int mode);
+ColRegKernel colreg_group_b(int L, int mode);
+ColRegKernel colreg_group_c(int L, int mode);
+ColRegKernel colreg_group_d(int L, int mode);
+ColRegKernel colreg_group_e(int L, int mode);
+
+// Register X passes (xreg.cuh).
+struct XRegArgs {
+    int pro;               // prologue of XS_OTHER
+    const float* in;       // R2C input
+    float cval, bg, kdiv;
+    int64_t Nz, Ny, Nx;
+    int64_t Kz, Ky, Kx, pz, py, px;  // kernel embedding (PRO_KERNEL)
+    float2* out;           // R2C output spectrum
+    const float2* spec;    // C2R input spectrum
+    float* out_real;       // C2R output
+    const float *aux0, *aux1;
+    double* partials;
+    int pred;              // EPI_RL_RATIO kernel: store the model, not the ratio
+    float scale;
+    int64_t P;
+    uint32_t nrows, nlines;  // rows of the volume; lines (rows, or pairs of rows for odd Fx)
+    int nin, nout;           // points of a line that can be non-zero / are kept
+    int vec;                 // rows are 8-byte aligned pairs
+    const float2* tw;        // W_L table, W_L^m = tw[m * tws]
+    int tws;
+    const float2* twx;       // W_Fx table
+};
+struct XRegKernel {
+    void* fn = nullptr;
+    int TL = 0, nt = 0, smem = 0;
+};
+#define DK_XREG_GROUPS(X) X(a) X(b) X(c) X(d) X(e) X(odd)
+#define DK_XREG_DECL(g)                       \
+    XRegKernel xreg_r2c_##g(int L, int src);  \
+    XRegKernel xreg_c2r_##g(int L, int epi);
+DK_XREG_GROUPS(DK_XREG_DECL)
+#undef DK_XREG_DECL
 
 struct XC2RArgs {
     const float2* in;
@@ -128,18 +187,16 @@ struct ConvPlan {
     float kdiv;
     double norm_sq;
     int device;
-    // TMA descriptors of the column passes (valid when tma_y / tma_z)
-    bool tma_y = false, tma_z = false;
-    CUtensorMap tm_s1_j1, tm_s2_j1, tm_s2_j2, tm_otf_z;
-    int s1_box = 0, s2y_box = 0, s2z_box = 0, otf_box = 0;
+    // Register column passes (ok when the axis length has one): Y forward
+    // S1 -> S2, axial in S2 (FP32 and FP16 OTF), Y inverse S2 -> S1
+    ColPass y_fwd, z_otf, z_otf16, y_inv;
+    bool reg_ok = false;
     // Mixed precision (decon_conv_set_precision): the OTF also stored as FP16
     // complex, scaled per kz plane by a power of two (OTF = otf16 * otf_inv[kz]),
     // read by the pipelined axial pass instead of the FP32 OTF.
     int precision = 0;
     __half2* otf16 = nullptr;
     float* otf_inv = nullptr;
-    CUtensorMap tm_otf16_z;   // valid when tma_otf16
-    bool tma_otf16 = false;
     // Fused Y / axial pass (yzpass.cuh): the OTF also stored kx-major
     // [Hx][Fy][Fz]; the spectrum between the X passes is then kx-major too
     // ([Hx][Nz][Ny] in s1).  nullptr: the canvas takes the unfused passes.
@@ -161,28 +218,24 @@ int build_otf_kmajor(const ConvPlan& p, cudaStream_t st);
 
 // Quantise p.otf into p.otf16 / p.otf_inv (capi.cu).
 int quantize_otf(const ConvPlan& p, cudaStream_t st);
-// True when the axial pass of this plan runs the pipelined kernel (conv.cu).
+// True when this plan's axial pass can take an FP16 OTF (conv.cu).
 bool zpass_pipelined(const ConvPlan& p);
 
 // Shared-memory opt-in (only ever raised per device and kernel) and cached
 // occupancy for a launch shape (conv.cu).
 int kernel_prepare(void* fn, size_t smem, int nthr, int* per_sm);
 
-bool tma_length_ok(int L);
-// Kernels of the X R2C / X C2R / plain column passes for one axis length
-// (the static-length instantiation, or the runtime-radix one), by prologue /
-// epilogue code; nullptr for an unknown code.  One translation unit each
-// (xstatic_r2c.cu, xstatic_c2r.cu, xstatic_col.cu), so they build in parallel.
-void* pick_xr2c_kernel(int pro, int L);
-void* pick_xc2r_kernel(int epi, int L);
-void* pick_colfft_kernel(int L);
+// Runtime-radix kernels (fftplain.cu) by prologue / epilogue code; nullptr for
+// an unknown code.
+void* pick_xr2c_kernel(int pro);
+void* pick_xc2r_kernel(int epi);
+void* pick_colfft_kernel();
 
-// Rank-3 map over an FP16 complex [d2][d1][pitch] buffer (one half2 = one
-// 4-byte element) with (16, 1, b2) boxes and no swizzle.
-bool encode_half_plane_map(CUtensorMap* map, const __half2* base, int64_t pitch, int64_t d1, int64_t d2,
-                           int b2);
-bool encode_spectrum_map(CUtensorMap* map, const float2* base, int64_t pitch, int64_t d1, int64_t d2,
-                         int b1, int b2);
+// Column passes of the plan's buffers (after they are allocated), and the
+// transform of the OTF buffer along an axis (1: y, 0: z) in place.
+void make_col_passes(ConvPlan& p);
+void make_z_otf16(ConvPlan& p);
+int transform_otf(const ConvPlan& p, int axis, cudaStream_t st);
 
 int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cval, float bg,
                 int64_t nz_rows, float2* out, cudaStream_t st, int64_t kstride = 0);

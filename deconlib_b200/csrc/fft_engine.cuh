@@ -1,4 +1,6 @@
-// Shared-memory Stockham FFT engine for batches of lines.
+// Shared-memory Stockham FFT engine for batches of lines of any 7-smooth
+// length, radices chosen at run time; the 5-smooth lengths up to 1024 have
+// register kernels instead (codelets.cuh).
 //
 // A CTA holds T lines of L complex points in shared memory, element (j, t)
 // (point j of line t) at phys(j, t) = j*T + (t ^ (j & (T-1))).  The XOR
@@ -8,14 +10,14 @@
 //
 // Each radix-R stage of the self-sorting (Stockham) algorithm reads point
 // j + r*L/R, multiplies by the twiddle W_{Ns R}^{r (j mod Ns)}, applies a
-// radix-R DFT and writes point (j div Ns) Ns R + (j mod Ns) + r Ns.  Every
-// thread owns at most ceil(32/R) butterflies per stage, so it holds <= 35
-// complex values in registers; a stage is read-all / barrier / write-all / barrier,
-// which lets the transform run in place.  Threads per line: ceil(L / 32).
+// radix-R DFT and writes point (j div Ns) Ns R + (j mod Ns) + r Ns; a stage is
+// read-all / barrier / write-all / barrier, which lets the transform run in
+// place.
 //
 // Twiddles come from a table of exp(-2 pi i m / Lt) computed on the host in
 // double precision (W_L^m = tw[m * tws]); no sin/cos is evaluated on the GPU.
 // Radices 2, 3, 4, 5, 7, 8 and 16 are implemented.
+// dft<16> and dft<8> also serve the warp transforms of the fused Y / axial pass.
 #pragma once
 
 #include "common.cuh"
@@ -24,24 +26,11 @@ namespace dk {
 
 constexpr int kMaxStages = 16;
 
-// Lengths with a compile-time radix sequence (fft_lines_static): 2^a x {1, 3,
-// 5, 15} from 64 to 1024, so that a canvas rounded up to one of them grows an
-// axis by at most 1/3; every other 7-smooth length takes the runtime-radix
-// path.
-#define DK_STATIC_LENGTHS(X) \
-    X(64) X(80) X(96) X(128) X(160) X(192) X(240) X(256) X(320) X(384) X(480) X(512) X(640) X(768) \
-    X(960) X(1024)
-__host__ __device__ constexpr bool static_length(int L) {
-#define DK_IS(n) L == n ||
-    return DK_STATIC_LENGTHS(DK_IS) false;
-#undef DK_IS
-}
 // Runtime-radix path: each thread holds ceil(kDynPPT / R) butterflies per
 // stage (<= 14 values, all in registers), so a line takes ceil(L / kDynPPT)
 // threads and a CTA up to kDynThreads.  (Holding 32 points per thread across
-// a stage's barrier, as the compile-time path does, spilled every value to
-// local memory on the runtime path and ran the strided passes at ~7 % of
-// HBM bandwidth.)
+// a stage's barrier spilled every value to local memory and ran the strided
+// passes at ~7 % of HBM bandwidth.)
 constexpr int kDynPPT = 8;
 constexpr int kDynThreads = 1024;
 
@@ -49,30 +38,13 @@ struct Axis {
     int L;                  // complex points per line
     int nst;                // radix stages
     unsigned long long rad; // radix of stage s in bits [4s, 4s+4), product == L
-    int tpl;                // threads per line: ceil(L / 32), runtime path ceil(L / kDynPPT)
+    int tpl;                // threads per line: ceil(L / kDynPPT)
     int tws;                // table stride: W_L^m = tw[m * tws]
     const float2* tw;       // twiddle table (device)
     __host__ __device__ int radix(int s) const { return (int)((rad >> (4 * s)) & 15ull); }
 };
 
 __device__ __forceinline__ int phys(int j, int t, int T) { return j * T + (t ^ (j & (T - 1))); }
-
-// Layout selector.  SW = 0: the XOR swizzle above (any power-of-two T).
-// SW = 1: T = 16 lines whose rows are exactly 128 bytes, laid out as the TMA
-// 128-byte swizzle writes them: 16-byte chunk (t / 2) XOR (j mod 8).  Both
-// keep a warp's accesses to consecutive lines at one point conflict-free.
-// SW >= 2: the XOR swizzle with a compile-time T = SW (the shifts and masks
-// fold into the address arithmetic).
-template <int SW>
-__device__ __forceinline__ int physw(int j, int t, int T) {
-    if constexpr (SW == 0) {
-        return phys(j, t, T);
-    } else if constexpr (SW == 1) {
-        return j * 16 + ((((t >> 1) ^ (j & 7)) << 1) | (t & 1));
-    } else {
-        return j * SW + (t ^ (j & (SW - 1)));
-    }
-}
 
 // multiply by -i (DIR < 0, forward) or +i (DIR > 0, inverse)
 template <int DIR>
@@ -232,18 +204,14 @@ __device__ __forceinline__ void dft(float2* v) {
     else if constexpr (R == 8) dft8<DIR>(v);
 }
 
-// One Stockham stage.  (t, jb): this thread's line and first butterfly.
-template <int R, int DIR, int NS_STATIC, int SW = 0, int PPT = 32>
-__device__ __forceinline__ void stage_body(float2* buf, int T, int L, int Ns_dyn, int t, int jb,
-                                           int tpl, const float2* __restrict__ tw, int tws,
-                                           int nin = 1 << 30, int nout = 1 << 30) {
-    // nin: points >= nin are known zeros (only meaningful in a first stage,
-    // where point index = input index); nout: points >= nout are not stored
-    // (only in a last stage, where point index = output index).
-    // ceil(PPT / R) butterflies per thread cover L / R butterflies with
-    // ceil(L / PPT) threads per line for every radix (<= PPT + R - 1 values held).
-    constexpr int K = (PPT + R - 1) / R;
-    const int Ns = NS_STATIC > 0 ? NS_STATIC : Ns_dyn;
+// One Stockham stage.  (t, jb): this thread's line and first butterfly.  Not
+// inlined, so each radix keeps its own register allocation.
+template <int R, int DIR>
+__device__ __noinline__ void fft_stage(float2* buf, int T, int L, int Ns, int t, int jb, int tpl,
+                                       const float2* __restrict__ tw, int tws) {
+    // ceil(kDynPPT / R) butterflies per thread cover L / R butterflies with
+    // ceil(L / kDynPPT) threads per line for every radix
+    constexpr int K = (kDynPPT + R - 1) / R;
     const int nb = L / R;
     const int step = L / (Ns * R);  // twiddle index step in units of W_L
     float2 v[K][R];
@@ -252,8 +220,7 @@ __device__ __forceinline__ void stage_body(float2* buf, int T, int L, int Ns_dyn
         const int j = jb + k * tpl;
         if (jb < tpl && j < nb) {
 #pragma unroll
-            for (int r = 0; r < R; ++r)
-                v[k][r] = (j + r * nb < nin) ? buf[physw<SW>(j + r * nb, t, T)] : make_float2(0.f, 0.f);
+            for (int r = 0; r < R; ++r) v[k][r] = buf[phys(j + r * nb, t, T)];
             if (Ns > 1) {
                 const int kk = j % Ns;
 #pragma unroll
@@ -272,77 +239,30 @@ __device__ __forceinline__ void stage_body(float2* buf, int T, int L, int Ns_dyn
         if (jb < tpl && j < nb) {
             const int base = (j / Ns) * Ns * R + (j % Ns);
 #pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (base + r * Ns < nout) buf[physw<SW>(base + r * Ns, t, T)] = v[k][r];
+            for (int r = 0; r < R; ++r) buf[phys(base + r * Ns, t, T)] = v[k][r];
         }
     }
     __syncthreads();
 }
 
-// Runtime-dispatched stage for arbitrary 7-smooth lengths.  Not inlined, so
-// each radix keeps its own register allocation.
-template <int R, int DIR>
-__device__ __noinline__ void fft_stage_dyn(float2* buf, int T, int L, int Ns, int t, int jb,
-                                           int tpl, const float2* tw, int tws) {
-    stage_body<R, DIR, 0, 0, kDynPPT>(buf, T, L, Ns, t, jb, tpl, tw, tws);
-}
-
+// Full transform of the T lines held in buf.  DIR = -1 forward
+// (exp(-2 pi i ...)), +1 inverse, both unnormalised.  All threads of the CTA
+// must call it (it contains barriers).  t = tid % T, jb = tid / T.
 template <int DIR>
-__device__ __forceinline__ void fft_lines_dyn(float2* buf, int T, int t, int jb, const Axis ax) {
+__device__ __forceinline__ void fft_lines(float2* buf, int T, int t, int jb, const Axis ax) {
     int Ns = 1;
     for (int s = 0; s < ax.nst; ++s) {
         const int R = ax.radix(s);
         switch (R) {
-            case 8: fft_stage_dyn<8, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
-            case 4: fft_stage_dyn<4, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
-            case 2: fft_stage_dyn<2, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
-            case 3: fft_stage_dyn<3, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
-            case 5: fft_stage_dyn<5, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
-            case 7: fft_stage_dyn<7, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
+            case 8: fft_stage<8, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
+            case 4: fft_stage<4, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
+            case 2: fft_stage<2, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
+            case 3: fft_stage<3, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
+            case 5: fft_stage<5, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
+            case 7: fft_stage<7, DIR>(buf, T, ax.L, Ns, t, jb, ax.tpl, ax.tw, ax.tws); break;
             default: break;
         }
         Ns *= R;
-    }
-}
-
-// Static lengths with the radix sequence fixed at compile time
-// (static_radix): straight-line stages, constant divisors for j div Ns.  The
-// runtime path (plan_axis, for non-instantiated lengths) uses radices <= 8.
-// The power-of-two part first, radix-16 stages first (fewest shared-memory
-// round trips), then 8 / 4 / 2, then the odd factors 5 and 3:
-// 64 = 16.4, 128 = 16.8, 256 = 16.16, 512 = 16.8.4, 1024 = 16.16.4,
-// 80 = 16.5, 96 = 8.4.3, 160 = 8.4.5, 192 = 16.4.3, 240 = 16.5.3,
-// 320 = 16.4.5, 384 = 16.8.3, 480 = 8.4.5.3, 640 = 16.8.5, 768 = 16.16.3,
-// 960 = 16.4.5.3.
-constexpr int static_radix(int rem) {
-    const int p = rem & -rem;  // power-of-two part
-    if (p > 1) return p >= 16 && p != 32 ? 16 : (p == 32 ? 8 : p);
-    return rem % 5 == 0 ? 5 : (rem % 3 == 0 ? 3 : (rem % 7 == 0 ? 7 : rem));
-}
-
-template <int L, int DIR, int NS, int SW = 0>
-__device__ __forceinline__ void fft_lines_static(float2* buf, int T, int t, int jb,
-                                                 const float2* __restrict__ tw, int tws,
-                                                 int nin = 1 << 30, int nout = 1 << 30) {
-    if constexpr (NS < L) {
-        constexpr int R = static_radix(L / NS);
-        stage_body<R, DIR, NS, SW>(buf, T, L, NS, t, jb, (L + 31) / 32, tw, tws,
-                                   NS == 1 ? nin : (1 << 30), NS * R == L ? nout : (1 << 30));
-        fft_lines_static<L, DIR, NS * R, SW>(buf, T, t, jb, tw, tws, nin, nout);
-    }
-}
-
-// Full transform of the T lines held in buf.  DIR = -1 forward
-// (exp(-2 pi i ...)), +1 inverse, both unnormalised.  All threads of the CTA
-// must call it (it contains barriers).  t = tid % T, jb = tid / T.
-// LS > 0 selects the compile-time path for length LS (== ax.L).
-template <int DIR, int LS>
-__device__ __forceinline__ void fft_lines(float2* buf, int T, int t, int jb, const Axis ax,
-                                          int nin = 1 << 30, int nout = 1 << 30) {
-    if constexpr (LS > 0) {
-        fft_lines_static<LS, DIR, 1>(buf, T, t, jb, ax.tw, ax.tws, nin, nout);
-    } else {
-        fft_lines_dyn<DIR>(buf, T, t, jb, ax);
     }
 }
 

@@ -1,126 +1,114 @@
 // Widefield PSF synthesis on the device: PSF(z) = |IFFT2(P(kx, ky) e^{2 pi i kz z})|^2.
 //
 // Replaces the NumPy loop of deconlib's pupil_to_psf (psf/widefield.py:18-73)
-// with two FFT passes per chunk of z planes, built on the library's own
-// shared-memory FFT engine:
+// with two FFT passes per chunk of z planes (psf_passes.cuh):
 //
-//   pass 1 (k_psf_cols): defocus P(ky, kx) e^{2 pi i kz z} on load (phase in
-//     FP64 with sincospi; pupil and kz are re-read per plane from L2), inverse
-//     FFT along y over tiles of T columns, complex planes written to scratch;
-//   pass 2 (k_psf_rows): inverse FFT along x over T contiguous rows, intensity
-//     |.|^2 times the final scale, written straight into the PSF.
+//   pass 1: defocus P(ky, kx) e^{2 pi i kz z} on load (phase in FP64 with
+//     sincospi; pupil and kz are re-read per plane from L2), inverse FFT along
+//     y over tiles of columns, complex columns written to scratch;
+//   pass 2: inverse FFT along x over rows, intensity |.|^2 times the final
+//     scale, written straight into the PSF.
 //
-// 20 bytes of HBM traffic per voxel (complex write + read, float write).  The
-// unit-sum normalisation needs no pass over the PSF: |e^{i phi}| = 1, so by
+// A pupil is zero outside the aperture, a disc that covers 4 % of the plane
+// and 23 % of its columns at the sampling of a 2x refined grid, and a zero
+// column stays zero under the defocus: k_psf_support lists the columns that
+// hold anything, pass 1 transforms those only (packed side by side in the
+// scratch) and pass 2 takes the others as zeros.  128x256x256 at 0.0425 um,
+// NA 1.4: passes 83 + 67 us without the list and on the shared-memory engine.
+// The unit-sum normalisation needs no pass over the PSF: |e^{i phi}| = 1, so by
 // Parseval every plane's unnormalised intensity sums to ny nx sum|P|^2, and
-// the total is nz ny nx sum|P|^2, an FP64 reduction over the pupil alone
-// (k_psf_energy).  numpy's ifft2 divides by ny nx; without normalisation the
-// PSF carries that factor squared.
+// the total is nz ny nx sum|P|^2, an FP64 reduction over the pupil alone.
+// numpy's ifft2 divides by ny nx; without normalisation the PSF carries that
+// factor squared.
 #include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
 #include <vector>
 
-#include "conv_impl.cuh"
+#include "psf_passes.cuh"
 
 namespace dk {
 
 // Complex scratch per chunk of planes: at most this many voxels (256 MB), or
 // one plane when a plane is larger.
 constexpr int64_t kPsfChunkVoxels = int64_t(1) << 25;
-constexpr int kPsfEnergyBlocks = 256;
 
-struct PsfColArgs {
-    const float2* pupil;
-    const double* kz;
-    const double* z;  // this chunk's first plane
-    float2* a;
-    int64_t nyx;
-    int nx, ntiles, T;
-    Axis ax;  // y axis, L = ny
-};
-
-struct PsfRowArgs {
-    const float2* a;
-    float* psf;  // this chunk's first plane
-    int64_t nrows;
-    int T;
-    FastDiv fd_L;
-    Axis ax;               // x axis, L = nx
-    const double* energy;  // sum |P|^2 (normalize) or nullptr
-    double norm_div;       // nz ny nx (normalize)
-    float fixed_scale;     // 1 / (ny nx)^2 (no normalisation)
-};
-
-// sum |P|^2 in FP64, one partial per CTA
-__global__ void k_psf_energy(const float2* __restrict__ pupil, int64_t n, double* __restrict__ partials) {
+// Per column x: flags[x] = 1 if the column of the pupil holds a non-zero (or
+// its phase may not be finite: |kz| > 1e100), and the column block's share of
+// sum |P|^2 in FP64.  32 columns per CTA.
+__global__ void k_psf_support(const float2* __restrict__ pupil, const double* __restrict__ kz, int ny, int nx,
+                              int* __restrict__ flags, double* __restrict__ partials) {
+    __shared__ int any[32];
+    if (threadIdx.y == 0) any[threadIdx.x] = 0;
+    __syncthreads();
+    const int x = blockIdx.x * 32 + threadIdx.x;
     double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float2 v = pupil[i];
-        acc += (double)v.x * v.x + (double)v.y * v.y;
-    }
-    const double s = block_sum(acc);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
-}
-
-// Pass 1: one CTA = T columns of one plane; defocus on load, inverse FFT along y.
-template <int LS>
-__global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, 1) k_psf_cols(const PsfColArgs a) {
-    extern __shared__ float2 sm[];
-    const int T = a.T, L = a.ax.L, tid = threadIdx.x;
-    const int64_t o = blockIdx.x / a.ntiles;
-    const int x0 = (int)(blockIdx.x - o * a.ntiles) * T;
-    const double zz = a.z[o];
-    const int lgT = 31 - __clz(T);  // T is a power of two
-    for (int q = tid; q < L * T; q += blockDim.x) {
-        const int j = q >> lgT, t = q & (T - 1);
-        float2 v = make_float2(0.f, 0.f);
-        if (x0 + t < a.nx) {
-            const int64_t p = (int64_t)j * a.nx + x0 + t;
-            double sn, cs;
-            sincospi(2.0 * a.kz[p] * zz, &sn, &cs);
-            const float2 pv = a.pupil[p];
-            v = make_float2((float)((double)pv.x * cs - (double)pv.y * sn),
-                            (float)((double)pv.x * sn + (double)pv.y * cs));
+    bool on = false;
+    if (x < nx) {
+#pragma unroll 4
+        for (int y = threadIdx.y; y < ny; y += blockDim.y) {
+            const int64_t p = (int64_t)y * nx + x;
+            const float2 v = pupil[p];
+            acc += (double)v.x * v.x + (double)v.y * v.y;
+            on = on || !(v.x == 0.f && v.y == 0.f) || !(fabs(kz[p]) <= 1e100);
         }
-        sm[phys(j, t, T)] = v;
     }
+    if (on) any[threadIdx.x] = 1;
+    // block_sum numbers threads by threadIdx.x: fold the rows first
+    __shared__ double part[32][33];
+    part[threadIdx.y][threadIdx.x] = acc;
     __syncthreads();
-    fft_lines<+1, LS>(sm, T, tid % T, tid / T, a.ax);
-    float2* dst = a.a + o * a.nyx + x0;
-    for (int q = tid; q < L * T; q += blockDim.x) {
-        const int j = q >> lgT, t = q & (T - 1);
-        if (x0 + t < a.nx) dst[(int64_t)j * a.nx + t] = sm[phys(j, t, T)];
+    if (threadIdx.y == 0) {
+        if (x < nx) flags[x] = any[threadIdx.x];
+        double t = 0.0;
+        for (int i = 0; i < 32; ++i) t += part[i][threadIdx.x];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (threadIdx.x == 0) partials[blockIdx.x] = t;
     }
 }
 
-// Pass 2: one CTA = T contiguous rows; inverse FFT along x, |.|^2 * scale.
-template <int LS>
-__global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, 1) k_psf_rows(const PsfRowArgs a) {
-    extern __shared__ float2 sm[];
-    const int T = a.T, L = a.ax.L, tid = threadIdx.x;
-    const int64_t row0 = (int64_t)blockIdx.x * T;
-    const int64_t left = a.nrows - row0;
-    const int nr = left < T ? (int)left : T;
-    const float2* src = a.a + row0 * L;
-    for (int q = tid; q < T * L; q += blockDim.x) {
-        const int t = fdiv(q, a.fd_L), j = q - t * L;
-        sm[phys(j, t, T)] = t < nr ? src[q] : make_float2(0.f, 0.f);
-    }
+// One CTA: the columns in use as a list (act) and each column's place in it
+// (pos, -1 for a zero column), and the energy.  Every column is in use when a
+// z is not finite or huge.
+__global__ void __launch_bounds__(1024) k_psf_scan(const int* __restrict__ flags, int nx, const double* __restrict__ z,
+                                                   int64_t nz, const double* __restrict__ partials, int nparts,
+                                                   int* __restrict__ act, int* __restrict__ pos, int* __restrict__ nact,
+                                                   double* __restrict__ energy) {
+    __shared__ int warp_base[32];
+    __shared__ int base, all;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (tid == 0) base = all = 0;
     __syncthreads();
-    fft_lines<+1, LS>(sm, T, tid % T, tid / T, a.ax);
-    float scale = a.fixed_scale;
-    if (a.energy) {
-        const double tot = a.norm_div * *a.energy;
-        scale = tot > 0.0 ? (float)(1.0 / tot) : 1.f;
+    for (int64_t i = tid; i < nz; i += blockDim.x)
+        if (!(fabs(z[i]) <= 1e100)) all = 1;
+    __syncthreads();
+    for (int x0 = 0; x0 < nx; x0 += blockDim.x) {
+        const int x = x0 + tid;
+        const bool on = x < nx && (all || flags[x]);
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) warp_base[w] = __popc(m);
+        __syncthreads();
+        if (tid == 0) {
+            int t = base;
+            for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
+                const int c = warp_base[i];
+                warp_base[i] = t;
+                t += c;
+            }
+            base = t;
+        }
+        __syncthreads();
+        const int at = warp_base[w] + __popc(m & ((1u << lane) - 1));
+        if (x < nx) pos[x] = on ? at : -1;
+        if (on) act[at] = x;
+        __syncthreads();
     }
-    float* dst = a.psf + row0 * L;
-    for (int q = tid; q < nr * L; q += blockDim.x) {
-        const int t = fdiv(q, a.fd_L), j = q - t * L;
-        const float2 v = sm[phys(j, t, T)];
-        dst[q] = (v.x * v.x + v.y * v.y) * scale;
+    if (tid == 0) {
+        *nact = base;
+        double t = 0.0;
+        for (int i = 0; i < nparts; ++i) t += partials[i];
+        *energy = t;
     }
 }
 
@@ -177,21 +165,12 @@ static int psf_pool(cudaMemPool_t* out) {
 }
 
 
-static int threads_for_lines(int T, const Axis& ax) {
-    return std::max(64, (int)round_up((int64_t)T * ax.tpl, 32));
-}
-
-template <int LS>
-static void* cols_ptr() { return (void*)k_psf_cols<LS>; }
-template <int LS>
-static void* rows_ptr() { return (void*)k_psf_rows<LS>; }
-
-static void* pick(int L, bool cols) {
-#define DK_CASE(n) \
-    if (L == n) return cols ? cols_ptr<n>() : rows_ptr<n>();
-    DK_STATIC_LENGTHS(DK_CASE)
-#undef DK_CASE
-    return cols ? cols_ptr<0>() : rows_ptr<0>();
+static PsfKernel pick(const Axis& ax, bool cols) {
+    for (auto group : {psf_group_a, psf_group_b, psf_group_c, psf_group_d, psf_group_e}) {
+        const PsfKernel k = group(ax.L, cols);
+        if (k.fn) return k;
+    }
+    return psf_any_kernel(ax, cols);
 }
 
 static int launch_args(void* fn, int64_t nblk, int nthr, size_t smem, cudaStream_t st, void* args) {
@@ -230,51 +209,51 @@ extern "C" int decon_pupil_to_psf(const float* pupil, const double* kz, const do
     axx.tws = axy.tws = 1;
     cudaMemPool_t pool;
     DK_TRY(psf_pool(&pool));
-    float2* a = nullptr;
-    double* red = nullptr;
+    // scratch: complex chunk, then energy, partials, and the column lists
+    const int nparts = (int)cdiv(nx, 32);
+    const size_t chunk_bytes = (size_t)round_up(chunk * nyx * (int64_t)sizeof(float2), 256);
+    const size_t bytes = chunk_bytes + (1 + nparts) * sizeof(double) + (3 * nx + 1) * sizeof(int);
+    char* buf = nullptr;
     auto run = [&]() -> int {
-        DK_CUDA(cudaMallocFromPoolAsync((void**)&a, (size_t)(chunk * nyx) * sizeof(float2), pool, st));
+        DK_CUDA(cudaMallocFromPoolAsync((void**)&buf, bytes, pool, st));
+        PsfArgs a{};
+        a.pupil = reinterpret_cast<const float2*>(pupil);
+        a.kz = kz;
+        a.a = reinterpret_cast<float2*>(buf);
+        double* energy = reinterpret_cast<double*>(buf + chunk_bytes);
+        double* partials = energy + 1;
+        int* flags = reinterpret_cast<int*>(partials + nparts);
+        int *act = flags + nx, *pos = act + nx, *nact = pos + nx;
+        k_psf_support<<<nparts, dim3(32, 32), 0, st>>>(a.pupil, kz, (int)ny, (int)nx, flags, partials);
+        DK_LAUNCHED();
+        k_psf_scan<<<1, 1024, 0, st>>>(flags, (int)nx, z, nz, partials, nparts, act, pos, nact, energy);
+        DK_LAUNCHED();
         const double inv_n = 1.0 / ((double)nx * (double)ny);
-        PsfRowArgs ra{};
-        ra.fixed_scale = (float)(inv_n * inv_n);
-        if (normalize) {
-            DK_CUDA(cudaMallocFromPoolAsync((void**)&red, (kPsfEnergyBlocks + 1) * sizeof(double), pool, st));
-            const int nb = (int)std::min<int64_t>(kPsfEnergyBlocks, cdiv(nyx, 256));
-            k_psf_energy<<<nb, 256, 0, st>>>(reinterpret_cast<const float2*>(pupil), nyx, red);
-            DK_LAUNCHED();
-            DK_TRY(finish_partials(red, nb, red + kPsfEnergyBlocks, st));
-            ra.energy = red + kPsfEnergyBlocks;
-            ra.norm_div = (double)nz * (double)nyx;
-        }
-        PsfColArgs ca{};
-        ca.pupil = reinterpret_cast<const float2*>(pupil);
-        ca.kz = kz;
-        ca.a = a;
-        ca.nyx = nyx;
-        ca.nx = (int)nx;
-        ca.ax = axy;
-        ca.T = fft_lines_per_cta(axy, 32);
-        ca.ntiles = (int)cdiv(nx, ca.T);
-        ra.a = a;
-        ra.ax = axx;
-        ra.T = fft_lines_per_cta(axx, 32);
-        ra.fd_L = make_fastdiv(nx);
-        void* fc = pick((int)ny, true);
-        void* fr = pick((int)nx, false);
-        const int tc = threads_for_lines(ca.T, axy), tr = threads_for_lines(ra.T, axx);
-        const size_t sc = (size_t)ca.T * ny * sizeof(float2), sr = (size_t)ra.T * nx * sizeof(float2);
+        a.energy = normalize ? energy : nullptr;
+        a.norm_div = (double)nz * (double)nyx;
+        a.fixed_scale = (float)(inv_n * inv_n);
+        a.act = act;
+        a.pos = pos;
+        a.nact = nact;
+        a.nx = (int)nx;
+        a.ny = (int)ny;
+        const PsfKernel kc = pick(axy, true), kr = pick(axx, false);
         for (int64_t z0 = 0; z0 < nz; z0 += chunk) {
             const int64_t nzc = std::min(chunk, nz - z0);
-            ca.z = z + z0;
-            DK_TRY(launch_args(fc, nzc * ca.ntiles, tc, sc, st, &ca));
-            ra.psf = psf + z0 * nyx;
-            ra.nrows = nzc * ny;
-            DK_TRY(launch_args(fr, cdiv(ra.nrows, ra.T), tr, sr, st, &ra));
+            a.z = z + z0;
+            a.psf = psf + z0 * nyx;
+            a.nrows = nzc * ny;
+            a.ax = axy;
+            a.T = kc.T;
+            a.ntiles = (int)cdiv(nx, kc.T);
+            DK_TRY(launch_args(kc.fn, nzc * a.ntiles, kc.nt, kc.smem, st, &a));
+            a.ax = axx;
+            a.T = kr.T;
+            DK_TRY(launch_args(kr.fn, cdiv(a.nrows, kr.T), kr.nt, kr.smem, st, &a));
         }
         return DECON_OK;
     };
     const int status = run();
-    if (a) cudaFreeAsync(a, st);
-    if (red) cudaFreeAsync(red, st);
+    if (buf) cudaFreeAsync(buf, st);
     return status;
 }

@@ -10,12 +10,6 @@
 
 namespace dk {
 
-// Device-side flag set when a bounded mbarrier wait gives up (read by
-// decon_device_status, cleared by decon_device_status_clear); such a CTA
-// skips its compute and store.  Only the translation unit with the TMA
-// kernels (conv.cu) includes this header.
-static __device__ int g_wait_timeout = 0;
-
 constexpr unsigned kWaitLimit = 1u << 22;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -49,12 +43,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Bounded wait: gives up after `limit` polls (kWaitLimit in the kernels) and
-// raises g_wait_timeout.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
+// raises *flag, the device's flag that decon_device_status reads (conv.cu);
+// the CTA then skips its compute and store.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* flag,
                                                   unsigned limit = kWaitLimit) {
     for (unsigned i = 0; i < limit; ++i)
         if (mbar_try_wait(bar, parity)) return true;
-    atomicExch(&g_wait_timeout, 1);
+    atomicExch(flag, 1);
     return false;
 }
 
@@ -68,26 +63,11 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
-// 3-D tiled bulk tensor store shared -> global (bulk-group completion).
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int c0, int c1, int c2,
-                                             const void* src) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
-            reinterpret_cast<uint64_t>(map)),
-        "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(src))
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_store_commit_and_wait() {
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-
-// Host: encode a rank-3 float32 tensor map over a spectrum buffer viewed as
-// [d2][d1][2 * pitch floats] with a (32 floats, b1, b2) box and 128-byte
-// swizzle.  Returns false if the driver entry point is unavailable or the
-// encode fails.
-bool encode_spectrum_map(CUtensorMap* map, const float2* base, int64_t pitch, int64_t d1, int64_t d2,
-                         int b1, int b2);
+// Host: rank-3 tensor map over a spectrum buffer [d2][d1][pitch] of elements
+// of esize bytes (8: complex64 as two floats, 4: half2) with boxes of T
+// elements x b1 x b2, no swizzle.  False if the driver entry point is
+// unavailable or the encode fails.
+bool encode_tile_map(CUtensorMap* map, const void* base, int esize, int64_t pitch, int64_t d1, int64_t d2,
+                     int T, int b1, int b2);
 
 }  // namespace dk

@@ -1,5 +1,7 @@
-// X passes: real-to-complex FFT of signal rows (pass 1) and complex-to-real
-// FFT back to rows with the fused element-wise epilogues (pass 5).
+// X passes of the lengths without a register kernel (xreg.cuh), and of the
+// kx-major spectrum of the fused Y / axial pass: real-to-complex FFT of signal
+// rows (pass 1) and complex-to-real FFT back to rows with the fused
+// element-wise epilogues (pass 5), on the runtime-radix engine.
 //
 // A row of Fx reals is packed as Fx/2 complex points z[n] = x[2n] + i x[2n+1]
 // (even Fx), transformed with the shared-memory engine and unpacked with the
@@ -8,31 +10,12 @@
 //
 // I/O: when a row is a plain, 16-byte aligned float array (Nx % 4 == 0, the
 // whole signal window) each thread moves float4 vectors, several in flight,
-// straight into the swizzled tile.  Points that are known zeros (the padding
-// beyond Nx / 2) are never written or read: the first FFT stage of pass 1
-// treats them as zeros and the last stage of pass 5 skips outputs beyond the
-// crop.
+// straight into the swizzled tile.
 #pragma once
 
 #include "conv_impl.cuh"
 
 namespace dk {
-
-__device__ __forceinline__ bool kernel_src(int64_t c, int64_t F, int64_t m, int64_t npos,
-                                           int64_t& k) {
-    // Corner-origin embedding (utils/padding.py:142-190): canvas index c holds
-    // kernel index c (c < npos) or c - F + m (the wrapped negative offsets).
-    if (c < npos) {
-        k = c;
-        return c < m;
-    }
-    const int64_t nneg = m - npos;
-    if (c >= F - nneg) {
-        k = c - F + m;
-        return true;
-    }
-    return false;
-}
 
 struct RowSrc {
     const float* p;  // row base (nullptr: row outside the window or constant input)
@@ -82,22 +65,11 @@ __device__ __forceinline__ float fetch_x(const XR2CArgs& a, const RowSrc& r, int
 // pass 1: X R2C
 // ---------------------------------------------------------------------------
 
-// Lines per CTA of the X passes for a compile-time length (the host's rule,
-// fft_lines_per_cta: T x L <= kSmemElems complex values and T x ceil(L / 32)
-// <= kFftThreads threads, T <= 32, a power of two).
-__host__ __device__ constexpr int x_lines(int LS) {
-    int T = 1;
-    while (T * 2 <= 32 && T * 2 * LS <= kSmemElems && T * 2 * ((LS + 31) / 32) <= kFftThreads) T *= 2;
-    return T;
-}
-
-template <int PRO, int LS>
-__global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, LS > 0 ? 3 : 1) k_xr2c(XR2CArgs a) {
+template <int PRO>
+__global__ void __launch_bounds__(kDynThreads, 1) k_xr2c(XR2CArgs a) {
     extern __shared__ float2 sm[];
     __shared__ RowSrc rsrc[32];  // per-row source (general path)
-    constexpr int TC = LS > 0 ? x_lines(LS) : 0;  // compile-time lines per CTA
-    const int T = TC > 0 ? TC : a.T, L = LS > 0 ? LS : a.ax.L, tid = threadIdx.x;
-    auto phys = [&](int j, int t, int) { return physw<TC>(j, t, T); };
+    const int T = a.T, L = a.ax.L, tid = threadIdx.x;
     const int64_t row0 = (int64_t)blockIdx.x * T;
     // packed points that can be non-zero
     const int nin = a.odd ? (int)(a.Nx < L ? a.Nx : L) : (int)(((a.Nx + 1) >> 1) < L ? ((a.Nx + 1) >> 1) : L);
@@ -203,18 +175,15 @@ __global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, LS > 0 ? 3
             sm[phys(n, t, T)] = v;
         }
     }
-    if constexpr (LS == 0) {
-        // the runtime-radix path reads every point: zero the padding
-        const int nz = L - nin;
-        #pragma unroll 1
-        for (int q = tid; q < T * nz; q += blockDim.x) {
-            const int t = q / nz;
-            sm[phys(nin + (q - t * nz), t, T)] = make_float2(0.f, 0.f);
-        }
+    // the stages read every point: zero the padding
+    const int nz = L - nin;
+    #pragma unroll 1
+    for (int q = tid; q < T * nz; q += blockDim.x) {
+        const int t = q / nz;
+        sm[phys(nin + (q - t * nz), t, T)] = make_float2(0.f, 0.f);
     }
     __syncthreads();
-    if constexpr (LS > 0) fft_lines_static<LS, -1, 1, TC>(sm, T, tid % T, tid / T, a.ax.tw, a.ax.tws, nin);
-    else fft_lines<-1, LS>(sm, T, tid % T, tid / T, a.ax, nin);
+    fft_lines<-1>(sm, T, tid % T, tid / T, a.ax);
     const int H = a.Hx;
     const int lgT = 31 - __clz(T);  // T is a power of two
     if (a.odd) {
@@ -318,20 +287,13 @@ __device__ __forceinline__ void epilogue(const XC2RArgs& a, int64_t i, float v, 
     }
 }
 
-// Three CTAs per SM below length 512 (80 registers, no spills; at 256 the
-// PDHG iteration measured 1.04-1.05 vs 1.06-1.07 ms with two); from 512 on
-// the compile-time lines per CTA need more registers, so two.
-template <int EPI, int LS>
-__global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, LS > 0 ? (LS < 512 ? 3 : 2) : 1) k_xc2r(XC2RArgs a) {
+template <int EPI>
+__global__ void __launch_bounds__(kDynThreads, 1) k_xc2r(XC2RArgs a) {
     extern __shared__ float2 sm[];
     __shared__ float2 nyq[32];    // X[M] of each row (even Fx)
     __shared__ int64_t obase[32];  // output index of x = 0 of each row (general path)
     constexpr int64_t kOutside = INT64_MIN;
-    // compile-time lines per CTA from L = 512 on (measured 211 -> 198 us at
-    // Fx = 1024); at L = 256 it brought no gain and spilled the loss epilogues
-    constexpr int TC = LS >= 512 ? x_lines(LS) : 0;
-    const int T = TC > 0 ? TC : a.T, L = LS > 0 ? LS : a.ax.L, tid = threadIdx.x;
-    auto phys = [&](int j, int t, int) { return physw<TC>(j, t, T); };
+    const int T = a.T, L = a.ax.L, tid = threadIdx.x;
     const int64_t row0 = (int64_t)blockIdx.x * T;
     const int lgT = 31 - __clz(T);  // T is a power of two
     if (a.odd) {
@@ -447,10 +409,7 @@ __global__ void __launch_bounds__(LS > 0 ? kFftThreads : kDynThreads, LS > 0 ? (
         }
         __syncthreads();
     }
-    // outputs beyond the kept x range are not needed
-    const int nout = a.odd ? (int)(a.Nx < L ? a.Nx : L) : (int)(((a.Nx + 1) >> 1) < L ? ((a.Nx + 1) >> 1) : L);
-    if constexpr (LS > 0) fft_lines_static<LS, +1, 1, TC>(sm, T, tid % T, tid / T, a.ax.tw, a.ax.tws, 1 << 30, nout);
-    else fft_lines<+1, LS>(sm, T, tid % T, tid / T, a.ax, 1 << 30, nout);
+    fft_lines<+1>(sm, T, tid % T, tid / T, a.ax);
 
     double acc = 0.0;
     const int64_t Nx = a.Nx;

@@ -1,0 +1,472 @@
+// X passes (real-to-complex and back) with the transform in registers.
+//
+// Even Fx: a row is packed as L = M = Fx / 2 complex points z[n] = x[2n] +
+// i x[2n+1].  Odd Fx: two rows make one line z[n] = xa[n] + i xb[n] of L = Fx
+// points.  L = B x S runs as two register DFTs around one exchange through
+// shared memory, and the packing is undone (or done) in the same registers:
+// spectrum points k and L - k lie in butterflies u and B - u of the radix-S
+// stage, so one thread takes both and no second pass over shared memory is
+// needed.  Rows are read and written by the threads that transform them, 8 or
+// 16 bytes a lane in whole row pieces.
+//
+//   R2C  stage 1: radix B over n = j + r S (global rows -> exchange)
+//        stage 2: radix S, butterflies u and B - u -> X[k], X[L - k]
+//   C2R  stage 1: X[k], X[L - k] -> radix S, butterflies u and B - u
+//        stage 2: radix B -> x, with the element-wise epilogues
+//
+// The self-paired butterflies (u = 0, and B / 2 for even B) go through the same
+// code: their second half repeats the first and is not stored.
+#pragma once
+
+#include "codelets.cuh"
+#include "conv_impl.cuh"
+
+namespace dk {
+
+// Lines, threads and exchange layout of a CTA.
+template <int L, bool ODD>
+struct XRegShape {
+    static constexpr int S = small_radix(L, ODD ? 27 : 20), B = L / S;
+    static constexpr int TPL = B / 2 + 1;  // threads per line in the paired stage
+    static constexpr int TL = 32 * TPL <= 160 ? 32 : (16 * TPL <= 160 ? 16 : (8 * TPL <= 160 ? 8 : 4));
+    static constexpr int NT = (TL * TPL + 31) / 32 * 32;
+    // one exchange row per butterfly of the first stage, an odd number of
+    // points apart: consecutive lanes hit different banks
+    template <int R>
+    struct Ex {
+        static constexpr int step = R | 1;               // row length
+        static constexpr int need = (L / R) * step;
+        // lines start TPL points apart modulo 16, so a half-warp that spans
+        // two lines still covers distinct banks
+        static constexpr int pitch = need + (((TPL - need) % 16) + 16) % 16;
+        static constexpr int bytes = TL * pitch * (int)sizeof(float2);
+    };
+    static constexpr int blocks_for(int regs) {
+        const int b = 65536 / (NT * ((regs + 7) / 8 * 8));
+        return b < 1 ? 1 : (b > 10 ? 10 : b);
+    }
+};
+
+// ---------------------------------------------------------------------------
+// pass 1: X R2C
+// ---------------------------------------------------------------------------
+
+enum XRegSrc { XS_ARRAY = 0, XS_UP2 = 1, XS_OTHER = 2 };
+
+// Source of a row for the set-up prologues (constant, kernel embedding,
+// max(y - b, 1e-6)): nullptr where the row is zero, any address for a constant.
+__device__ __forceinline__ const float* other_row(const XRegArgs& a, int64_t row) {
+    if (row >= a.nrows) return nullptr;
+    if (a.pro == PRO_CONST) return &a.cval;
+    if (a.pro == PRO_RLINIT) return a.in + row * a.Nx;
+    // PRO_KERNEL: corner-origin embedding of the kernel in the canvas
+    int64_t kz, ky;
+    const int64_t z = row / a.Ny, y = row - z * a.Ny;
+    if (!kernel_src(z, a.Nz, a.Kz, a.pz, kz) || !kernel_src(y, a.Ny, a.Ky, a.py, ky)) return nullptr;
+    return a.in + (kz * a.Ky + ky) * a.Kx;
+}
+__device__ __forceinline__ float other_value(const XRegArgs& a, const float* p, int x) {
+    if (p == nullptr || x >= a.Nx) return 0.f;
+    if (a.pro == PRO_CONST) return a.cval;
+    if (a.pro == PRO_RLINIT) return fmaxf(__ldg(p + x) - a.bg, 1e-6f);
+    int64_t kx;
+    if (!kernel_src(x, a.Nx, a.Kx, a.px, kx)) return 0.f;
+    return __ldg(p + kx) / a.kdiv;
+}
+
+template <int L, bool ODD, int SRC>
+__global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::blocks_for(4 * XRegShape<L, ODD>::S + 44))
+    k_xreg_r2c(const XRegArgs a) {
+    using H = XRegShape<L, ODD>;
+    constexpr int S = H::S, B = H::B, TL = H::TL, NT = H::NT, TPL = H::TPL;
+    using E = typename H::template Ex<B>;
+    extern __shared__ float2 sm[];
+    const int tid = threadIdx.x;
+    const uint32_t line0 = blockIdx.x * TL;
+    float2* stg = sm + TL * E::pitch;  // staged rows (XS_OTHER)
+    if constexpr (SRC == XS_OTHER) {
+        __shared__ const float* rows[2 * TL];
+        constexpr int W = ODD ? 2 : 1;  // rows per line
+        for (int i = tid; i < W * TL; i += NT) rows[i] = other_row(a, (int64_t)W * line0 + i);
+        __syncthreads();
+        for (int l = 0; l < TL; ++l)
+            for (int n = tid; n < a.nin; n += NT)
+                stg[l * L + n] = ODD ? make_float2(other_value(a, rows[2 * l], n), other_value(a, rows[2 * l + 1], n))
+                                     : make_float2(other_value(a, rows[l], 2 * n), other_value(a, rows[l], 2 * n + 1));
+        __syncthreads();
+    }
+
+    // stage 1
+#pragma unroll 1
+    for (int q = tid; q < TL * S; q += NT) {
+        const int l = q / S, j = q - l * S;
+        const uint32_t line = line0 + l;
+        C1 v[B];
+        if constexpr (SRC == XS_OTHER) {
+#pragma unroll
+            for (int r = 0; r < B; ++r) v[r] = j + r * S < a.nin ? as_c1(stg[l * L + j + r * S]) : C1{0.f, 0.f};
+        } else if constexpr (SRC == XS_UP2) {
+            // fine row (z, y) of the adjoint of the 2x area sum: fine x = 2n and
+            // 2n + 1 both take coarse value n of coarse row (z / 2, y / 2)
+            const uint32_t z = line / (uint32_t)a.Ny, y = line - z * (uint32_t)a.Ny;
+            const float* p = a.in + ((int64_t)(z >> 1) * (a.Ny >> 1) + (y >> 1)) * (a.Nx >> 1);
+            const int lim = line < a.nrows ? a.nin : 0;
+#pragma unroll
+            for (int r = 0; r < B; ++r) {
+                const float w = j + r * S < lim ? __ldg(p + j + r * S) : 0.f;
+                v[r] = C1{w, w};
+            }
+        } else if constexpr (ODD) {
+            const float* p = a.in + (int64_t)line * 2 * a.Nx;
+            const int lim = 2 * line < a.nrows ? a.nin : 0, lim2 = 2 * line + 1 < a.nrows ? a.nin : 0;
+#pragma unroll
+            for (int r = 0; r < B; ++r) {
+                const int n = j + r * S;
+                v[r] = C1{n < lim ? __ldg(p + n) : 0.f, n < lim2 ? __ldg(p + a.Nx + n) : 0.f};
+            }
+        } else if (a.vec) {
+            const float2* p = reinterpret_cast<const float2*>(a.in + (int64_t)line * a.Nx);
+            const int lim = line < a.nrows ? a.nin : 0;
+#pragma unroll
+            for (int r = 0; r < B; ++r) v[r] = j + r * S < lim ? as_c1(__ldg(p + j + r * S)) : C1{0.f, 0.f};
+        } else {
+            const float* p = a.in + (int64_t)line * a.Nx;
+            const int lim = line < a.nrows ? (int)a.Nx : 0;
+#pragma unroll
+            for (int r = 0; r < B; ++r) {
+                const int x = 2 * (j + r * S);
+                v[r] = C1{x < lim ? __ldg(p + x) : 0.f, x + 1 < lim ? __ldg(p + x + 1) : 0.f};
+            }
+        }
+        dftn<B, -1>(v);
+        float2* e = sm + l * E::pitch + j * E::step;
+#pragma unroll
+        for (int r = 0; r < B; ++r) e[r] = as_f2(v[r]);
+    }
+    __syncthreads();
+
+    // stage 2
+    const int l = tid / TPL, u = tid - l * TPL;
+    const uint32_t line = line0 + l;
+    if (l >= TL || line >= a.nlines) return;
+    C1 va[S], vb[S];
+    {
+        const float2* e = sm + l * E::pitch;
+        const int m = u == 0 ? 0 : B - u;
+#pragma unroll
+        for (int r = 0; r < S; ++r) {
+            va[r] = as_c1(e[u + r * E::step]);
+            vb[r] = as_c1(e[m + r * E::step]);
+            if (r > 0) {
+                const float2 w = __ldg(&a.tw[(r * u) * a.tws]);
+                va[r] = twist<false>(va[r], w);
+                // W^(r (B - u)) without its factor W_S^r, which shifts the
+                // outputs by one (read below at index + 1)
+                vb[r] = twist<true>(vb[r], w);
+            }
+        }
+    }
+    dftn<S, -1>(va);
+    dftn<S, -1>(vb);
+    if constexpr (!ODD) {
+        // X[k] = e + W^k o, X[M-k] = conj(e - W^k o) with e = (Z[k] + conj
+        // Z[M-k]) / 2, o = -i (Z[k] - conj Z[M-k]) / 2
+        float2* out = a.out + (int64_t)line * a.P;
+        const bool second = u > 0 && 2 * u < B;
+#pragma unroll
+        for (int r = 0; r < S; ++r) {
+            const int k = u + r * B;
+            const C1 zk = va[r], zm = conj_of(vb[(S - r) % S]);
+            const C1 s = zk + zm, d = zk - zm;
+            const C1 e{0.5f * s.re, 0.5f * s.im}, o{0.5f * d.im, -0.5f * d.re};
+            const C1 t = twist<false>(o, __ldg(&a.twx[k]));
+            out[k] = as_f2(e + t);
+            if (second || (u == 0 && r == 0)) out[L - k] = as_f2(conj_of(e - t));
+        }
+    } else {
+        // Xa = (Z[k] + conj Z[L-k]) / 2, Xb = -i (Z[k] - conj Z[L-k]) / 2
+        float2* out = a.out + (int64_t)line * 2 * a.P;
+        const bool two = 2 * line + 1 < a.nrows;
+#pragma unroll
+        for (int r = 0; r < S; ++r) {
+            int k = u + r * B;
+            const C1 zk = va[r], zm = conj_of(vb[(S - r) % S]);
+            const C1 s = zk + zm, d = zk - zm;
+            C1 xa{0.5f * s.re, 0.5f * s.im}, xb{0.5f * d.im, -0.5f * d.re};
+            if (2 * k > L) {
+                if (u == 0) continue;
+                k = L - k;
+                xa = conj_of(xa);
+                xb = conj_of(xb);
+            }
+            out[k] = as_f2(xa);
+            if (two) out[a.P + k] = as_f2(xb);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// pass 5: X C2R with fused epilogues
+// ---------------------------------------------------------------------------
+
+// Element-wise epilogue on N voxels from index i on (v already scaled).
+template <int EPI, int N>
+__device__ __forceinline__ void x_epilogue(const XRegArgs& a, int64_t i, const float* v, double& acc) {
+    typedef typename std::conditional<N == 2, float2, float>::type V;
+    float o[N];
+    if constexpr (EPI == EPI_STORE) {
+#pragma unroll
+        for (int e = 0; e < N; ++e) o[e] = v[e];
+    } else if constexpr (EPI == EPI_RL_UPDATE) {
+        // rl_mlx.py:149-150  x = max(x * where(active, A^T ratio / sens, 0), 1e-10)
+        const V s = __ldg(reinterpret_cast<const V*>(a.aux1 + i));
+        const V x = *reinterpret_cast<const V*>(a.aux0 + i);
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            const float se = reinterpret_cast<const float*>(&s)[e];
+            const float c = se > 0.f ? v[e] / se : 0.f;
+            o[e] = fmaxf(reinterpret_cast<const float*>(&x)[e] * c, 1e-10f);
+        }
+    } else {
+        // rl_mlx.py:147-148  model = A x + b ; ratio = y / max(model, 1e-10)
+        const V y = __ldg(reinterpret_cast<const V*>(a.aux0 + i));
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            const float yv = reinterpret_cast<const float*>(&y)[e];
+            const float m = v[e] + a.bg;
+            o[e] = a.pred ? m : yv / fmaxf(m, 1e-10f);
+            if (a.partials) {
+                // rl_mlx.py:75-79: y log(max(y,eps)/max(m,eps)) - (y - max(m,eps))
+                const float ys = fmaxf(yv, 1e-6f), ms = fmaxf(m, 1e-6f);
+                acc += (double)(yv * logf(ys / ms) - (yv - ms));
+            }
+        }
+    }
+    V w;
+#pragma unroll
+    for (int e = 0; e < N; ++e) reinterpret_cast<float*>(&w)[e] = o[e];
+    *reinterpret_cast<V*>(a.out_real + i) = w;
+}
+
+// Spectrum row of line l: consecutive rows, or, for the 2x area sum, the four
+// rows of one 2 x 2 (z, y) block in lines 4q .. 4q + 3.
+template <int EPI>
+__device__ __forceinline__ uint32_t c2r_line(const XRegArgs& a, uint32_t line) {
+    if constexpr (EPI == EPI_DOWN2) {
+        const uint32_t q = line >> 2, my = (uint32_t)a.Ny >> 1;
+        const uint32_t k = q / my, y = q - k * my;
+        return (2 * k + (line & 1)) * (uint32_t)a.Ny + 2 * y + ((line >> 1) & 1);
+    } else {
+        return line;
+    }
+}
+
+template <int L, bool ODD, int EPI>
+__global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
+                                  XRegShape<L, ODD>::blocks_for(EPI == EPI_DOWN2 && XRegShape<L, ODD>::B > 12
+                                                                    ? 4 * XRegShape<L, ODD>::B + 44
+                                                                    : 4 * XRegShape<L, ODD>::S + 44))
+    k_xreg_c2r(const XRegArgs a) {
+    using H = XRegShape<L, ODD>;
+    constexpr int S = H::S, B = H::B, TL = H::TL, NT = H::NT, TPL = H::TPL;
+    using E = typename H::template Ex<S>;
+    extern __shared__ float2 sm[];
+    const int tid = threadIdx.x;
+    const uint32_t line0 = blockIdx.x * TL;
+
+    // stage 1
+    {
+        const int l = tid / TPL, u = tid - l * TPL;
+        const uint32_t line = line0 + l;
+        if (l < TL && line < a.nlines) {
+            C1 va[S], vb[S];
+            if constexpr (!ODD) {
+                // Z[k] = e + i d W^-k, Z[M-k] = conj(e) + i conj(d W^-k) with e = X[k] +
+                // conj X[M-k], d = X[k] - conj X[M-k]; irfft ignores Im of DC and Nyquist
+                const float2* in = a.spec + (int64_t)c2r_line<EPI>(a, line) * a.P;
+#pragma unroll
+                for (int r = 0; r < S; ++r) {
+                    va[r] = as_c1(__ldg(in + u + r * B));
+                    vb[r] = as_c1(__ldg(in + L - u - r * B));
+                }
+                if (u == 0) va[0].im = vb[0].im = 0.f;
+#pragma unroll
+                for (int r = 0; r < S; ++r) {
+                    const C1 xm = conj_of(vb[r]);
+                    const C1 e = va[r] + xm, d = va[r] - xm;
+                    const C1 t = twist<true>(d, __ldg(&a.twx[u + r * B]));
+                    va[r] = C1{e.re - t.im, e.im + t.re};
+                    vb[r] = C1{e.re + t.im, t.re - e.im};
+                }
+            } else {
+                // Z[k] = Xa[k] + i Xb[k], Z[L-k] = conj(Xa[k]) + i conj(Xb[k])
+                const float2* in = a.spec + (int64_t)line * 2 * a.P;
+                const bool two = 2 * line + 1 < a.nrows;
+#pragma unroll
+                for (int r = 0; r < S; ++r) {
+                    const int k = u + r * B;
+                    const bool up = 2 * k > L;
+                    const int h = up ? L - k : k;
+                    va[r] = as_c1(__ldg(in + h));
+                    vb[r] = two ? as_c1(__ldg(in + a.P + h)) : C1{0.f, 0.f};
+                    if (up) {
+                        va[r].im = -va[r].im;
+                        vb[r].im = -vb[r].im;
+                    }
+                }
+                if (u == 0) va[0].im = vb[0].im = 0.f;
+#pragma unroll
+                for (int r = 0; r < S; ++r) {
+                    const C1 xa = va[r], xb = vb[r];
+                    va[r] = C1{xa.re - xb.im, xa.im + xb.re};
+                    vb[r] = C1{xa.re + xb.im, xb.re - xa.im};
+                }
+            }
+            float2* e = sm + l * E::pitch;
+            dftn<S, +1>(va);
+#pragma unroll
+            for (int r = 0; r < S; ++r) e[u * E::step + r] = as_f2(va[r]);
+            if (u > 0 && 2 * u < B) {
+                // butterfly B - u holds Z[L-k] in reverse order
+#pragma unroll
+                for (int r = 0; r < S / 2; ++r) {
+                    const C1 t = vb[r];
+                    vb[r] = vb[S - 1 - r];
+                    vb[S - 1 - r] = t;
+                }
+                dftn<S, +1>(vb);
+#pragma unroll
+                for (int r = 0; r < S; ++r) e[(B - u) * E::step + r] = as_f2(vb[r]);
+            }
+        }
+    }
+    __syncthreads();
+
+    // stage 2
+    double acc = 0.0;
+    auto transform = [&](int l, int j, C1 (&v)[B]) {
+        const float2* e = sm + l * E::pitch + j;
+#pragma unroll
+        for (int r = 0; r < B; ++r) {
+            v[r] = as_c1(e[r * E::step]);
+            if (r > 0) v[r] = twist<true>(v[r], __ldg(&a.tw[(r * j) * a.tws]));
+        }
+        dftn<B, +1>(v);
+    };
+    const float s = a.scale;
+    if constexpr (EPI == EPI_DOWN2) {
+        // 2x area sum of the scaled output, in the order of the three banded
+        // passes (z pairs, then y pairs, then x pairs; unit weights).  Lines
+        // 4q, 4q+1: planes 2k, 2k+1 at y = 2j; 4q+2, 4q+3: at y = 2j+1.
+        // Round-to-nearest intrinsics: every product and sum is rounded as the
+        // stored output and the separate passes round it (no fma).
+#pragma unroll 1
+        for (int q = tid; q < TL / 4 * S; q += NT) {
+            const int b = q / S, j = q - b * S;
+            const uint32_t line = line0 + 4 * b;
+            if (line >= a.nlines) continue;
+            float sx[B], sy[B];
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                C1 v[B];
+                float px[B], py[B];
+                transform(4 * b + 2 * h, j, v);
+#pragma unroll
+                for (int r = 0; r < B; ++r) {
+                    px[r] = __fmul_rn(v[r].re, s);
+                    py[r] = __fmul_rn(v[r].im, s);
+                }
+                transform(4 * b + 2 * h + 1, j, v);
+#pragma unroll
+                for (int r = 0; r < B; ++r) {
+                    px[r] = __fadd_rn(px[r], __fmul_rn(v[r].re, s));
+                    py[r] = __fadd_rn(py[r], __fmul_rn(v[r].im, s));
+                    sx[r] = h == 0 ? px[r] : __fadd_rn(sx[r], px[r]);
+                    sy[r] = h == 0 ? py[r] : __fadd_rn(sy[r], py[r]);
+                }
+            }
+            float* out = a.out_real + (int64_t)(line >> 2) * (a.Nx >> 1) + j;
+#pragma unroll
+            for (int r = 0; r < B; ++r)
+                if (j + r * S < a.nout) out[r * S] = __fadd_rn(sx[r], sy[r]);
+        }
+    } else {
+#pragma unroll 1
+        for (int q = tid; q < TL * S; q += NT) {
+            const int l = q / S, j = q - l * S;
+            const uint32_t line = line0 + l;
+            if (line >= a.nlines) continue;
+            C1 v[B];
+            transform(l, j, v);
+            if constexpr (ODD) {
+                const int64_t i = (int64_t)line * 2 * a.Nx + j;
+                const bool two = 2 * line + 1 < a.nrows;
+#pragma unroll
+                for (int r = 0; r < B; ++r) {
+                    if (j + r * S >= a.nout) continue;
+                    const float xa = v[r].re * s, xb = v[r].im * s;
+                    x_epilogue<EPI, 1>(a, i + r * S, &xa, acc);
+                    if (two) x_epilogue<EPI, 1>(a, i + a.Nx + r * S, &xb, acc);
+                }
+            } else if (a.vec) {
+                const int64_t i = (int64_t)line * a.Nx + 2 * j;
+#pragma unroll
+                for (int r = 0; r < B; ++r) {
+                    if (j + r * S >= a.nout) continue;
+                    const float x[2] = {v[r].re * s, v[r].im * s};
+                    x_epilogue<EPI, 2>(a, i + 2 * r * S, x, acc);
+                }
+            } else {
+                const int64_t i = (int64_t)line * a.Nx + 2 * j;
+#pragma unroll
+                for (int r = 0; r < B; ++r) {
+                    const int x0 = 2 * (j + r * S);
+                    if (x0 >= a.Nx) continue;
+                    const float xa = v[r].re * s, xb = v[r].im * s;
+                    x_epilogue<EPI, 1>(a, i + 2 * r * S, &xa, acc);
+                    if (x0 + 1 < a.Nx) x_epilogue<EPI, 1>(a, i + 2 * r * S + 1, &xb, acc);
+                }
+            }
+        }
+    }
+    if constexpr (EPI == EPI_RL_RATIO) {
+        if (a.partials) {
+            const double t = block_sum(acc);
+            if (tid == 0) a.partials[blockIdx.x] = t;
+        }
+    }
+}
+
+template <int L, bool ODD>
+XRegKernel xreg_r2c_of(int src) {
+    using H = XRegShape<L, ODD>;
+    constexpr int smem = H::template Ex<H::B>::bytes;
+    switch (src) {
+        case XS_ARRAY: return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_ARRAY>, H::TL, H::NT, smem};
+        case XS_UP2:
+            if constexpr (!ODD) return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_UP2>, H::TL, H::NT, smem};
+            break;
+        case XS_OTHER:
+            return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_OTHER>, H::TL, H::NT,
+                              smem + H::TL * L * (int)sizeof(float2)};
+    }
+    return XRegKernel{};
+}
+
+template <int L, bool ODD>
+XRegKernel xreg_c2r_of(int epi) {
+    using H = XRegShape<L, ODD>;
+    constexpr int smem = H::template Ex<H::S>::bytes;
+    switch (epi) {
+        case EPI_STORE: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_STORE>, H::TL, H::NT, smem};
+        case EPI_PRED:
+        case EPI_RL_RATIO: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_RL_RATIO>, H::TL, H::NT, smem};
+        case EPI_RL_UPDATE: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_RL_UPDATE>, H::TL, H::NT, smem};
+        case EPI_DOWN2:
+            if constexpr (!ODD) return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_DOWN2>, H::TL, H::NT, smem};
+            break;
+    }
+    return XRegKernel{};
+}
+
+}  // namespace dk

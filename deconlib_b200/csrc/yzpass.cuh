@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_yz(const __grid_constant__ YZA
                 bulk_prefetch_l2(reinterpret_cast<const char*>(o) + off, kBytes - off < kChunk ? kBytes - off : kChunk);
         }
         // ---- A: forward Y transform of this CTA's rows: B (input) -> A ----
-        ok = mbar_wait_bounded(&bar, (uint32_t)(it & 1)) && ok;
+        ok = mbar_wait_bounded(&bar, (uint32_t)(it & 1), &g_wait_timeout) && ok;
         {
             const int sub = lane % (2 * NLY), h = sub / NLY, j = sub % NLY;
             const int xs = NLY == 8 ? 8 * h : 0;
