@@ -260,6 +260,7 @@ static XRegArgs xreg_args(const ConvPlan& p, int64_t nrows, int64_t Ny, int64_t 
     a.nrows = (uint32_t)nrows;
     a.nlines = (uint32_t)(p.odd ? cdiv(nrows, 2) : nrows);
     a.nin = a.nout = (int)std::min<int64_t>(p.odd ? Nx : cdiv(Nx, 2), L);
+    a.Hx = (int)p.Hx;
     a.tw = p.ax_x.tw;
     a.tws = p.ax_x.tws;
     a.twx = p.twx;
@@ -268,7 +269,7 @@ static XRegArgs xreg_args(const ConvPlan& p, int64_t nrows, int64_t Ny, int64_t 
 
 int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cval, float bg,
                 int64_t nz_rows, float2* out, cudaStream_t st, int64_t kstride) {
-    const int src = pro == PRO_ARRAY ? 0 : pro == PRO_UP2 ? 1 : 2;
+    const int src = pro == PRO_KERNEL ? 2 : pro == PRO_UP2 ? 1 : 0;
     const XRegKernel k = p.reg_ok && kstride == 0 && (pro == PRO_KERNEL || pro == PRO_UP2 || is_full_window(p, win))
                              ? pick_xreg_r2c(p.ax_x.L, p.odd, src)
                              : XRegKernel{};

@@ -124,7 +124,7 @@ ColRegKernel colreg_group_e(int L, int mode);
 
 // Register X passes (xreg.cuh).
 struct XRegArgs {
-    int pro;               // prologue of XS_OTHER
+    int pro;               // Prologue (array, constant or RL start in the array kernel)
     const float* in;       // R2C input
     float cval, bg, kdiv;
     int64_t Nz, Ny, Nx;
@@ -139,6 +139,7 @@ struct XRegArgs {
     int64_t P;
     uint32_t nrows, nlines;  // rows of the volume; lines (rows, or pairs of rows for odd Fx)
     int nin, nout;           // points of a line that can be non-zero / are kept
+    int Hx;                  // spectrum points of a row
     int vec;                 // rows are 8-byte aligned pairs
     const float2* tw;        // W_L table, W_L^m = tw[m * tws]
     int tws;
