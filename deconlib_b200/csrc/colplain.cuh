@@ -9,6 +9,7 @@ namespace dk {
 
 __global__ void __launch_bounds__(kDynThreads, 1) k_colfft(ColArgs a) {
     extern __shared__ float2 sm[];
+    chain_enter();
     const int T = a.T, L = a.ax.L, tid = threadIdx.x;
     const int64_t o = blockIdx.x / a.ntiles;
     const int64_t kx0 = (int64_t)(blockIdx.x - o * a.ntiles) * T;

@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
         fence_proxy_async_smem();
     }
     __syncthreads();
+    chain_enter();
 
     // full tiles come by TMA; the tiles of the last Hx % T columns, which hold
     // several planes side by side, by plain loads

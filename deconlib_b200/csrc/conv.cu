@@ -133,9 +133,23 @@ int kernel_prepare(void* fn, size_t smem, int nthr, int* per_sm) {
     return DECON_OK;
 }
 
-static int launch(void* fn, dim3 grid, int nthr, size_t smem, cudaStream_t st, void* args, int cls) {
-    DK_TRY(kernel_prepare(fn, smem, nthr, nullptr));
+// Dynamic shared memory that needs no opt-in, whatever the kernel's static part
+// (at most a few hundred bytes in the FFT passes; the default limit is 48 KB).
+constexpr size_t kNoOptIn = 44 * 1024;
+
+// Launches an FFT pass as a chained kernel.  prepared: its shared memory is
+// already opted in (a plan's column passes), or needs no opt-in.
+static int launch_chained(void* fn, dim3 grid, int nthr, size_t smem, bool prepared, cudaStream_t st, void* args,
+                          int cls) {
+    if (!prepared && smem > kNoOptIn) DK_TRY(kernel_prepare(fn, smem, nthr, nullptr));
     void* params[] = {args};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(nthr);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    chain_attribute(&cfg, at);
     const bool prof = (g_prof.mask & cls) != 0;
     if (prof) {
         if (g_prof.used == g_prof.ev.size()) {
@@ -146,7 +160,7 @@ static int launch(void* fn, dim3 grid, int nthr, size_t smem, cudaStream_t st, v
         }
         DK_CUDA(cudaEventRecord(g_prof.ev[g_prof.used].first, st));
     }
-    DK_CUDA(cudaLaunchKernel(fn, grid, dim3(nthr), params, smem, st));
+    DK_CUDA(cudaLaunchKernelExC(&cfg, fn, params));
     count_launch();
     if (prof) {
         DK_CUDA(cudaEventRecord(g_prof.ev[g_prof.used].second, st));
@@ -158,7 +172,7 @@ static int launch(void* fn, dim3 grid, int nthr, size_t smem, cudaStream_t st, v
 static int launch(void* fn, int64_t nblk, int nthr, size_t smem, cudaStream_t st, void* args, int cls) {
     if (nblk <= 0) return kernel_prepare(fn, smem, nthr, nullptr);
     if (nblk > 0x7fffffffLL) return fail(DECON_ERR_UNSUPPORTED, "grid too large");
-    return launch(fn, dim3((unsigned)nblk), nthr, smem, st, args, cls);
+    return launch_chained(fn, dim3((unsigned)nblk), nthr, smem, false, st, args, cls);
 }
 
 }  // namespace dk
@@ -570,7 +584,7 @@ void make_z_otf16(ConvPlan& p) {
 static int launch_col_pass(const ConvPlan&, const ColPass& c, bool conj, cudaStream_t st) {
     ColRegArgs a = c.a;
     if (conj) a.conj = -1.f;
-    return launch(c.k.fn, c.grid, c.k.nt, c.smem, st, &a, a.otf ? PROF_ZOTF : PROF_COL);
+    return launch_chained(c.k.fn, dim3((unsigned)c.grid), c.k.nt, c.smem, true, st, &a, a.otf ? PROF_ZOTF : PROF_COL);
 }
 
 int transform_otf(const ConvPlan& p, int axis, cudaStream_t st) {

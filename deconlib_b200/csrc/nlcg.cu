@@ -134,6 +134,7 @@ __device__ __forceinline__ void ew4(int64_t n, const float* const (&in)[NI], flo
 // f0 = max(x, 1e-6), s = sqrt(f0), f = s s; or (from_s) f = s s alone.
 __global__ void k_nlcg_init(const float* __restrict__ x, float* __restrict__ s, float* __restrict__ f,
                             int64_t n, int from_s, int vec) {
+    chain_enter();
     const float* in[1] = {x};
     float* out[2] = {from_s ? nullptr : s, f};
     ew4(n, in, out, vec, [&](const float* v, float* o) {
@@ -156,6 +157,7 @@ __device__ __forceinline__ void model_terms(float m, float g, float eps, float& 
 
 __global__ void k_nlcg_model(const float* __restrict__ m, const float* __restrict__ g, float eps,
                              float* __restrict__ w, int64_t n, int vec, double* part, NlcgDev* dev) {
+    chain_enter();
     double v[3] = {0.0, 0.0, 0.0};
     const float* in[2] = {m, g};
     float* out[1] = {w};
@@ -169,6 +171,7 @@ __global__ void k_nlcg_products(int mode, float gamma, const float* __restrict__
                                 const float* __restrict__ d, const float* __restrict__ r,
                                 float* __restrict__ d_out, float* __restrict__ sd,
                                 float* __restrict__ dd, int64_t n, int vec, NlcgDev* dev) {
+    chain_enter();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         dev->lam = 0.0;
         dev->done = 0;
@@ -186,6 +189,7 @@ __global__ void k_nlcg_products(int mode, float gamma, const float* __restrict__
 
 __global__ void k_nlcg_gram(const float* __restrict__ a, const float* __restrict__ b,
                             const float* __restrict__ c, int64_t n, int vec, double* part, NlcgDev* dev) {
+    chain_enter();
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     const float* in[3] = {a, b, c};
     float* out[1] = {nullptr};
@@ -207,6 +211,7 @@ __global__ void k_nlcg_newton(const float* __restrict__ m, const float* __restri
                               const float* __restrict__ kdd, const float* __restrict__ g, float b,
                               float eps, double beta, int use_reg, int64_t n, int vec, double* part,
                               NlcgDev* dev) {
+    chain_enter();
     if (dev->done) return;  // every CTA reads the same flag: all return or none
     const double lam = dev->lam;
     const float c1 = (float)(2.0 * lam), c2 = (float)(lam * lam), lf = (float)lam;
@@ -252,6 +257,7 @@ __global__ void k_nlcg_accept_d(const float* __restrict__ m, const float* __rest
                                 const float* __restrict__ kdd, const float* __restrict__ g, float b,
                                 float eps, float* __restrict__ m_new, float* __restrict__ w_new,
                                 int64_t n, int vec, double* part, NlcgDev* dev) {
+    chain_enter();
     const double lam = dev->lam;
     const float c1 = (float)(2.0 * lam), c2 = (float)(lam * lam);
     double v[3] = {0.0, 0.0, 0.0};
@@ -269,6 +275,7 @@ __global__ void k_nlcg_accept_d(const float* __restrict__ m, const float* __rest
 __global__ void k_nlcg_accept_o(const float* __restrict__ s, const float* __restrict__ d,
                                 float* __restrict__ s_new, float* __restrict__ f_new, int64_t n, int vec,
                                 const NlcgDev* dev) {
+    chain_enter();
     const float lf = (float)dev->lam;
     const float* in[2] = {s, d};
     float* out[2] = {s_new, f_new};
@@ -280,6 +287,7 @@ __global__ void k_nlcg_accept_o(const float* __restrict__ s, const float* __rest
 }
 
 __global__ void k_nlcg_energy(const float* __restrict__ a, int64_t n, int vec, double* part, NlcgDev* dev) {
+    chain_enter();
     double v[1] = {0.0};
     const float* in[1] = {a};
     float* out[1] = {nullptr};
@@ -297,6 +305,7 @@ __global__ void k_nlcg_gradient(const float* __restrict__ s, const float* __rest
                                 const float* __restrict__ f_prev, const float* __restrict__ ktw,
                                 const float* __restrict__ ctcf, float c4b, float eps,
                                 float* __restrict__ r, int64_t n, int vec, double* part, NlcgDev* dev) {
+    chain_enter();
     double v[3] = {0.0, 0.0, 0.0};
     const bool has_g = ktw != nullptr, has_c = ctcf != nullptr, has_p = f_prev != nullptr;
     const float* in[5] = {has_g ? s : nullptr, f, f_prev, ktw, ctcf};
@@ -334,6 +343,7 @@ __global__ void __launch_bounds__(256) k_nlcg_hess_gram(const float* __restrict_
                                                         const float* __restrict__ sd,
                                                         const float* __restrict__ dd, Dims d, W6 w,
                                                         double* part, NlcgDev* dev) {
+    chain_enter();
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     hess_zwalk<IDX, 3>(
         d, w, [&](IDX i) { return Fields3{__ldg(f + i), __ldg(sd + i), __ldg(dd + i)}; },
@@ -361,6 +371,7 @@ __global__ void __launch_bounds__(256) k_nlcg_hess_gram(const float* __restrict_
 template <class IDX>
 __global__ void __launch_bounds__(256) k_nlcg_hess_energy(const float* __restrict__ f, Dims d, W6 w,
                                                           double* part, NlcgDev* dev) {
+    chain_enter();
     double v[1] = {0.0};
     hess_zwalk<IDX, 1>(
         d, w, [&](IDX i) { return __ldg(f + i); }, [](const float& r, int) { return r; },
@@ -379,6 +390,7 @@ __global__ void k_nlcg_quad(const float* __restrict__ g, const float* __restrict
                             const float* __restrict__ ksd, int64_t nd, const float* __restrict__ a,
                             const float* __restrict__ d, int64_t no, float eps, double* part,
                             NlcgDev* dev) {
+    chain_enter();
     double v[2] = {0.0, 0.0};
     for (int64_t i = gtid(); i < nd; i += gstride()) {
         const float mv = m[i], kv = ksd[i];
@@ -447,7 +459,7 @@ int decon_nlcg_destroy(decon_nlcg* h) { return nl_free(h); }
 int decon_nlcg_init(const float* x, float* s, float* f, int64_t n, int from_s, void* stream) {
     if (!x || !f || (!from_s && !s)) return fail(DECON_ERR_NULL, "null pointer");
     if (n <= 0) return DECON_OK;
-    k_nlcg_init<<<nl_blocks(n), kNlThreads, 0, as_stream(stream)>>>(x, s, f, n, from_s, al16({x, s, f}));
+    DK_TRY(chain(k_nlcg_init, nl_blocks(n), kNlThreads, 0, as_stream(stream), x, s, f, n, from_s, al16({x, s, f})));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -456,8 +468,8 @@ int decon_nlcg_model(decon_nlcg* h, const float* m, const float* g, float eps, f
                      void* stream) {
     if (!h || !m || !g) return fail(DECON_ERR_NULL, "null pointer");
     if (n <= 0) return fail(DECON_ERR_VALUE, "decon_nlcg_model: empty data");
-    k_nlcg_model<<<nl_blocks(n), kNlThreads, 0, as_stream(stream)>>>(m, g, eps, w, n, al16({m, g, w}),
-                                                                     h->part, h->dev);
+    DK_TRY(chain(k_nlcg_model, nl_blocks(n), kNlThreads, 0, as_stream(stream), m, g, eps, w, n, al16({m, g, w}),
+                                                                     h->part, h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -469,8 +481,8 @@ int decon_nlcg_products(decon_nlcg* h, int mode, float gamma, const float* s, co
     if (mode != 0 && mode != 1) return fail(DECON_ERR_VALUE, "decon_nlcg_products: mode must be 0 or 1");
     if (n <= 0) return fail(DECON_ERR_VALUE, "decon_nlcg_products: empty object");
     const int vec = al16({s, d, mode == 1 ? r : nullptr, mode == 1 ? d_out : nullptr, sd, dd});
-    k_nlcg_products<<<nl_blocks(n), kNlThreads, 0, as_stream(stream)>>>(mode, gamma, s, d, r, d_out, sd,
-                                                                        dd, n, vec, h->dev);
+    DK_TRY(chain(k_nlcg_products, nl_blocks(n), kNlThreads, 0, as_stream(stream), mode, gamma, s, d, r, d_out, sd,
+                                                                        dd, n, vec, h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -479,8 +491,8 @@ int decon_nlcg_gram(decon_nlcg* h, const float* a, const float* b, const float* 
                     void* stream) {
     if (!h || !a || !b || !c) return fail(DECON_ERR_NULL, "null pointer");
     if (n <= 0) return fail(DECON_ERR_VALUE, "decon_nlcg_gram: empty");
-    k_nlcg_gram<<<nl_blocks(n), kNlThreads, 0, as_stream(stream)>>>(a, b, c, n, al16({a, b, c}), h->part,
-                                                                    h->dev);
+    DK_TRY(chain(k_nlcg_gram, nl_blocks(n), kNlThreads, 0, as_stream(stream), a, b, c, n, al16({a, b, c}), h->part,
+                                                                    h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -492,8 +504,8 @@ int decon_nlcg_newton(decon_nlcg* h, const float* m, const float* ksd, const flo
     if (n <= 0) return fail(DECON_ERR_VALUE, "decon_nlcg_newton: empty data");
     const cudaStream_t st = as_stream(stream);
     for (int it = 0; it < newton_iters; ++it) {
-        k_nlcg_newton<<<nl_blocks(n), kNlThreads, 0, st>>>(m, ksd, kdd, g, background, eps, beta, use_reg,
-                                                          n, al16({m, ksd, kdd, g}), h->part, h->dev);
+        DK_TRY(chain(k_nlcg_newton, nl_blocks(n), kNlThreads, 0, st, m, ksd, kdd, g, background, eps, beta, use_reg,
+                                                          n, al16({m, ksd, kdd, g}), h->part, h->dev));
         DK_LAUNCHED();
     }
     return DECON_OK;
@@ -506,14 +518,14 @@ int decon_nlcg_accept(decon_nlcg* h, const float* m, const float* ksd, const flo
     if (!h || !m || !ksd || !kdd || !g || !m_new) return fail(DECON_ERR_NULL, "null pointer");
     if (nd <= 0) return fail(DECON_ERR_VALUE, "decon_nlcg_accept: empty data");
     const cudaStream_t st = as_stream(stream);
-    k_nlcg_accept_d<<<nl_blocks(nd), kNlThreads, 0, st>>>(m, ksd, kdd, g, background, eps, m_new, w_new,
+    DK_TRY(chain(k_nlcg_accept_d, nl_blocks(nd), kNlThreads, 0, st, m, ksd, kdd, g, background, eps, m_new, w_new,
                                                          nd, al16({m, ksd, kdd, g, m_new, w_new}), h->part,
-                                                         h->dev);
+                                                         h->dev));
     DK_LAUNCHED();
     if (s) {
         if (!d || !s_new || !f_new) return fail(DECON_ERR_NULL, "null pointer");
-        k_nlcg_accept_o<<<nl_blocks(no), kNlThreads, 0, st>>>(s, d, s_new, f_new, no,
-                                                             al16({s, d, s_new, f_new}), h->dev);
+        DK_TRY(chain(k_nlcg_accept_o, nl_blocks(no), kNlThreads, 0, st, s, d, s_new, f_new, no,
+                                                             al16({s, d, s_new, f_new}), h->dev));
         DK_LAUNCHED();
     }
     return DECON_OK;
@@ -522,7 +534,7 @@ int decon_nlcg_accept(decon_nlcg* h, const float* m, const float* ksd, const flo
 int decon_nlcg_energy(decon_nlcg* h, const float* a, int64_t n, void* stream) {
     if (!h || !a) return fail(DECON_ERR_NULL, "null pointer");
     if (n <= 0) return fail(DECON_ERR_VALUE, "decon_nlcg_energy: empty");
-    k_nlcg_energy<<<nl_blocks(n), kNlThreads, 0, as_stream(stream)>>>(a, n, al16({a}), h->part, h->dev);
+    DK_TRY(chain(k_nlcg_energy, nl_blocks(n), kNlThreads, 0, as_stream(stream), a, n, al16({a}), h->part, h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -533,8 +545,8 @@ int decon_nlcg_gradient(decon_nlcg* h, const float* s, const float* f, const flo
     if (!h || !f || (ktw && (!s || !r))) return fail(DECON_ERR_NULL, "null pointer");
     if (n <= 0) return fail(DECON_ERR_VALUE, "decon_nlcg_gradient: empty object");
     const int vec = al16({ktw ? s : nullptr, f, f_prev, ktw, ctcf, ktw ? r : nullptr});
-    k_nlcg_gradient<<<nl_blocks(n), kNlThreads, 0, as_stream(stream)>>>(s, f, f_prev, ktw, ctcf, c4b, eps,
-                                                                       r, n, vec, h->part, h->dev);
+    DK_TRY(chain(k_nlcg_gradient, nl_blocks(n), kNlThreads, 0, as_stream(stream), s, f, f_prev, ktw, ctcf, c4b, eps,
+                                                                       r, n, vec, h->part, h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -557,11 +569,11 @@ int decon_nlcg_hess_gram(decon_nlcg* h, const float* f, const float* sd, const f
     W6 w;
     hessian_weights(r, w.w);
     if (offsets_fit_u32(d))
-        k_nlcg_hess_gram<uint32_t><<<hess_grid(d, (const void*)k_nlcg_hess_gram<uint32_t>), 256, 0, as_stream(stream)>>>(
-            f, sd, dd, d, w, h->part, h->dev);
+        DK_TRY(chain(k_nlcg_hess_gram<uint32_t>, hess_grid(d, (const void*)k_nlcg_hess_gram<uint32_t>), 256, 0, as_stream(stream), 
+            f, sd, dd, d, w, h->part, h->dev));
     else
-        k_nlcg_hess_gram<int64_t><<<hess_grid(d, (const void*)k_nlcg_hess_gram<int64_t>), 256, 0, as_stream(stream)>>>(
-            f, sd, dd, d, w, h->part, h->dev);
+        DK_TRY(chain(k_nlcg_hess_gram<int64_t>, hess_grid(d, (const void*)k_nlcg_hess_gram<int64_t>), 256, 0, as_stream(stream), 
+            f, sd, dd, d, w, h->part, h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -573,11 +585,11 @@ int decon_nlcg_hess_energy(decon_nlcg* h, const float* f, const int64_t shape[3]
     W6 w;
     hessian_weights(r, w.w);
     if (offsets_fit_u32(d))
-        k_nlcg_hess_energy<uint32_t><<<hess_grid(d, (const void*)k_nlcg_hess_energy<uint32_t>), 256, 0,
-                                       as_stream(stream)>>>(f, d, w, h->part, h->dev);
+        DK_TRY(chain(k_nlcg_hess_energy<uint32_t>, hess_grid(d, (const void*)k_nlcg_hess_energy<uint32_t>), 256, 0,
+                                       as_stream(stream), f, d, w, h->part, h->dev));
     else
-        k_nlcg_hess_energy<int64_t><<<hess_grid(d, (const void*)k_nlcg_hess_energy<int64_t>), 256, 0,
-                                      as_stream(stream)>>>(f, d, w, h->part, h->dev);
+        DK_TRY(chain(k_nlcg_hess_energy<int64_t>, hess_grid(d, (const void*)k_nlcg_hess_energy<int64_t>), 256, 0,
+                                      as_stream(stream), f, d, w, h->part, h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -587,8 +599,8 @@ int decon_nlcg_quad(decon_nlcg* h, const float* g, const float* m, const float* 
     if (!h || !g || !m || !ksd || !a || !d) return fail(DECON_ERR_NULL, "null pointer");
     if (nd <= 0 || no <= 0) return fail(DECON_ERR_VALUE, "decon_nlcg_quad: empty");
     const int64_t big = std::max(nd, no);
-    k_nlcg_quad<<<nl_blocks(big), kNlThreads, 0, as_stream(stream)>>>(g, m, ksd, nd, a, d, no, eps,
-                                                                     h->part, h->dev);
+    DK_TRY(chain(k_nlcg_quad, nl_blocks(big), kNlThreads, 0, as_stream(stream), g, m, ksd, nd, a, d, no, eps,
+                                                                     h->part, h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }

@@ -27,6 +27,7 @@ struct Box4 {
 
 __global__ void k_window_copy(const float* __restrict__ src, float* __restrict__ dst, Box4 b,
                               int64_t n) {
+    chain_enter();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         int64_t r = i, c[4];
@@ -54,6 +55,7 @@ __global__ void k_banded_inner(const float* __restrict__ in, float* __restrict__
                                int64_t n_in, int64_t inner, int64_t n_out,
                                const int32_t* __restrict__ idx, const float* __restrict__ w,
                                int width) {
+    chain_enter();
     const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= inner) return;
     const int64_t j = blockIdx.y;
@@ -74,6 +76,7 @@ __global__ void k_banded_inner4(const float* __restrict__ in, float* __restrict_
                                 int64_t n_in, int64_t inner, int64_t n_out,
                                 const int32_t* __restrict__ idx, const float* __restrict__ w,
                                 int width) {
+    chain_enter();
     const int64_t q4 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t inner4 = inner >> 2;
     if (q4 >= inner4) return;
@@ -101,6 +104,7 @@ constexpr int kBandW = 8;
 __global__ void k_banded_last_rows(const float* __restrict__ in, float* __restrict__ out, int64_t outer,
                                    int64_t n_in, int64_t n_out, const int32_t* __restrict__ idx,
                                    const float* __restrict__ w, int width) {
+    chain_enter();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n_out) return;
     int32_t ij[kBandW];
@@ -126,6 +130,7 @@ __global__ void k_banded_last_rows(const float* __restrict__ in, float* __restri
 __global__ void k_banded_last(const float* __restrict__ in, float* __restrict__ out, int64_t outer,
                               int64_t n_in, int64_t n_out, const int32_t* __restrict__ idx,
                               const float* __restrict__ w, int width) {
+    chain_enter();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n_out) return;
     const int32_t* ij = idx + j * width;
@@ -160,6 +165,7 @@ struct Vol {
 template <class IDX>
 __global__ void __launch_bounds__(256) k_hessian_fwd_z(const float* __restrict__ x, float* __restrict__ h,
                                                        Dims d, W6 w) {
+    chain_enter();
     const IDX n = (IDX)(d.nz * d.ny * d.nx);
     hess_zwalk<IDX, 1>(
         d, w, [&](IDX i) { return __ldg(x + i); }, [](const float& r, int) { return r; },
@@ -170,6 +176,7 @@ __global__ void __launch_bounds__(256) k_hessian_fwd_z(const float* __restrict__
 }
 
 __global__ void k_gradient_fwd(Vol f, float* __restrict__ g, float r) {
+    chain_enter();
     const int64_t n = f.nz * f.ny * f.nx;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -191,6 +198,7 @@ __device__ __forceinline__ float d1f_adj(const float* g, int64_t i, int64_t n, i
 
 __global__ void k_gradient_adj(const float* __restrict__ g, float* __restrict__ out, int64_t nz,
                                int64_t ny, int64_t nx, float r) {
+    chain_enter();
     const int64_t n = nz * ny * nx, sz = ny * nx, sy = nx;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -234,7 +242,7 @@ int decon_window_copy(const float* src, const int64_t* src_shape, const int64_t*
         n *= b.ds[d];
     }
     if (n == 0) return DECON_OK;
-    k_window_copy<<<grid1d(n, 256), 256, 0, as_stream(stream)>>>(src, dst, b, n);
+    DK_TRY(chain(k_window_copy, grid1d(n, 256), 256, 0, as_stream(stream), src, dst, b, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -293,10 +301,10 @@ int decon_banded_axis(const float* in, float* out, int64_t outer, int64_t n_in, 
             const int64_t gx = cdiv(n_out, 256);
             const int64_t gy = std::max<int64_t>(1, std::min<int64_t>(outer, cdiv((int64_t)sm_count() * 16, gx)));
             dim3 g((unsigned)gx, (unsigned)gy);
-            k_banded_last_rows<<<g, 256, 0, st>>>(in, out, outer, n_in, n_out, idx, w, width);
+            DK_TRY(chain(k_banded_last_rows, g, 256, 0, st, in, out, outer, n_in, n_out, idx, w, width));
         } else {
             dim3 g((unsigned)cdiv(n_out, 256), (unsigned)std::min<int64_t>(outer, 65535));
-            k_banded_last<<<g, 256, 0, st>>>(in, out, outer, n_in, n_out, idx, w, width);
+            DK_TRY(chain(k_banded_last, g, 256, 0, st, in, out, outer, n_in, n_out, idx, w, width));
         }
     } else {
         if (n_out > 65535) return fail(DECON_ERR_UNSUPPORTED, "resampled axis longer than 65535");
@@ -305,8 +313,8 @@ int decon_banded_axis(const float* in, float* out, int64_t outer, int64_t n_in, 
         const int64_t cols = v4 ? inner / 4 : inner;
         const int thr = cols >= 256 ? 256 : (int)round_up(cols, 32);
         dim3 g((unsigned)cdiv(cols, thr), (unsigned)n_out, (unsigned)std::min<int64_t>(outer, 65535));
-        if (v4) k_banded_inner4<<<g, thr, 0, st>>>(in, out, outer, n_in, inner, n_out, idx, w, width);
-        else k_banded_inner<<<g, thr, 0, st>>>(in, out, outer, n_in, inner, n_out, idx, w, width);
+        if (v4) DK_TRY(chain(k_banded_inner4, g, thr, 0, st, in, out, outer, n_in, inner, n_out, idx, w, width));
+        else DK_TRY(chain(k_banded_inner, g, thr, 0, st, in, out, outer, n_in, inner, n_out, idx, w, width));
     }
     DK_LAUNCHED();
     return DECON_OK;
@@ -321,9 +329,9 @@ int decon_hessian3d_forward(const float* x, float* h, const int64_t shape[3], fl
     const Dims d{shape[0], shape[1], shape[2]};
     const int64_t grid = std::min<int64_t>(TileGeo(d).ntiles, (int64_t)sm_count() * 8);
     if (offsets_fit_u32(d))
-        k_hessian_fwd_z<uint32_t><<<(unsigned)std::max<int64_t>(grid, 1), 256, 0, as_stream(stream)>>>(x, h, d, w);
+        DK_TRY(chain(k_hessian_fwd_z<uint32_t>, (unsigned)std::max<int64_t>(grid, 1), 256, 0, as_stream(stream), x, h, d, w));
     else
-        k_hessian_fwd_z<int64_t><<<(unsigned)std::max<int64_t>(grid, 1), 256, 0, as_stream(stream)>>>(x, h, d, w);
+        DK_TRY(chain(k_hessian_fwd_z<int64_t>, (unsigned)std::max<int64_t>(grid, 1), 256, 0, as_stream(stream), x, h, d, w));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -343,7 +351,7 @@ int decon_gradient3d_forward(const float* x, float* g, const int64_t shape[3], f
     if (!x || !g || !shape) return fail(DECON_ERR_NULL, "null pointer");
     Vol f{x, shape[0], shape[1], shape[2]};
     const int64_t n = shape[0] * shape[1] * shape[2];
-    k_gradient_fwd<<<grid1d(n, 256), 256, 0, as_stream(stream)>>>(f, g, r);
+    DK_TRY(chain(k_gradient_fwd, grid1d(n, 256), 256, 0, as_stream(stream), f, g, r));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -351,7 +359,7 @@ int decon_gradient3d_forward(const float* x, float* g, const int64_t shape[3], f
 int decon_gradient3d_adjoint(const float* g, float* x, const int64_t shape[3], float r, void* stream) {
     if (!g || !x || !shape) return fail(DECON_ERR_NULL, "null pointer");
     const int64_t n = shape[0] * shape[1] * shape[2];
-    k_gradient_adj<<<grid1d(n, 256), 256, 0, as_stream(stream)>>>(g, x, shape[0], shape[1], shape[2], r);
+    DK_TRY(chain(k_gradient_adj, grid1d(n, 256), 256, 0, as_stream(stream), g, x, shape[0], shape[1], shape[2], r));
     DK_LAUNCHED();
     return DECON_OK;
 }

@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(256) k_hess_dual_p(PdhgDev* s, float* y2,
                                                      const float* __restrict__ xc,
                                                      const float* __restrict__ xp, Dims d, W6 w,
                                                      float alpha) {
+    chain_enter();
     if (s->stop) return;
     const float sg = (float)s->sigma, th = (float)s->theta;
     const int64_t n = d.nz * d.ny * d.nx;
@@ -330,6 +331,7 @@ __global__ void __launch_bounds__(256) k_hess_dk_r(PdhgDev* s, const float* __re
                                                    const float* __restrict__ xn,
                                                    const float* __restrict__ xc, Dims d, W6 w,
                                                    int slot_a, int slot_l) {
+    chain_enter();
     if (s->stop) return;
     double a2 = 0.0, l2 = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
@@ -354,6 +356,7 @@ __global__ void __launch_bounds__(256) k_hess_dk_r(PdhgDev* s, const float* __re
 template <int NORM>
 __global__ void __launch_bounds__(256) k_hess_regloss_p(PdhgDev* s, const float* __restrict__ x,
                                                         Dims d, W6 w, int kk, int slot) {
+    chain_enter();
     if (!(kk < s->final_iter && !(s->converged && kk == s->final_iter - 1))) return;
     double acc = 0.0;
     Ptrs<1> hs{{x}};
@@ -518,6 +521,7 @@ __global__ void __launch_bounds__(256) k_hess_primal_t(PdhgDev* s, const float* 
                                                        const float* __restrict__ y2,
                                                        float* __restrict__ xn, Dims d, W6 w,
                                                        int s_dx2, int s_xc2, int s_xn2) {
+    chain_enter();
     if (s->stop) return;
     const float tau = (float)s->tau;
     double dx2 = 0.0, xc2 = 0.0, xn2 = 0.0;
@@ -542,6 +546,7 @@ __global__ void __launch_bounds__(256) k_hess_primal_t(PdhgDev* s, const float* 
 template <class IDX>
 __global__ void __launch_bounds__(256) k_hessian_adj_t(const float* __restrict__ hw, float* __restrict__ out,
                                                        Dims d, W6 w) {
+    chain_enter();
     hess_adj_walk<IDX>(hw, d, w, [&](IDX i, float lt) { out[i] = lt; });
 }
 
@@ -592,6 +597,7 @@ __global__ void __launch_bounds__(256) k_hess_dual_primal(
     PdhgDev* s, const float* __restrict__ y2_in, float* __restrict__ y2_out,
     const float* __restrict__ xc, const float* __restrict__ xp, const float* __restrict__ aty,
     float* __restrict__ xn, Dims d, W6 w, float alpha, int s_dx2, int s_xc2, int s_xn2) {
+    chain_enter();
     if (s->stop) return;
     __shared__ float xb[4][kPL2];     // x_bar planes, ring slot = plane & 3
     __shared__ float yn[6][4][kPL];   // y2_out planes, ring slot = plane & 3

@@ -24,6 +24,7 @@ template <int OP>
 __global__ void __launch_bounds__(kRedThreads) k_reduce1(const float* __restrict__ a,
                                                          const float* __restrict__ b, int64_t n,
                                                          double* __restrict__ partials) {
+    chain_enter();
     double acc = OP == DECON_RED_MAX ? -DBL_MAX : 0.0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce1(const float* __restrict
 template <bool MAX>
 __global__ void __launch_bounds__(kRedThreads) k_reduce2(const double* __restrict__ partials, int n,
                                                          double* __restrict__ out) {
+    chain_enter();
     double acc = MAX ? -DBL_MAX : 0.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) acc = MAX ? fmax(acc, partials[i]) : acc + partials[i];
     if (MAX) {
@@ -79,22 +81,22 @@ int reduce_f32(const float* a, const float* b, int64_t n, int op, double* out, d
     const int g = red_blocks(n);
     if (g > npartials) return fail(DECON_ERR_VALUE, "reduce: partials buffer too small");
     switch (op) {
-        case DECON_RED_SUM: k_reduce1<DECON_RED_SUM><<<g, kRedThreads, 0, st>>>(a, b, n, partials); break;
-        case DECON_RED_SUMSQ: k_reduce1<DECON_RED_SUMSQ><<<g, kRedThreads, 0, st>>>(a, b, n, partials); break;
-        case DECON_RED_DIFFSQ: k_reduce1<DECON_RED_DIFFSQ><<<g, kRedThreads, 0, st>>>(a, b, n, partials); break;
-        case DECON_RED_DOT: k_reduce1<DECON_RED_DOT><<<g, kRedThreads, 0, st>>>(a, b, n, partials); break;
-        case DECON_RED_MAX: k_reduce1<DECON_RED_MAX><<<g, kRedThreads, 0, st>>>(a, b, n, partials); break;
+        case DECON_RED_SUM: DK_TRY(chain(k_reduce1<DECON_RED_SUM>, g, kRedThreads, 0, st, a, b, n, partials)); break;
+        case DECON_RED_SUMSQ: DK_TRY(chain(k_reduce1<DECON_RED_SUMSQ>, g, kRedThreads, 0, st, a, b, n, partials)); break;
+        case DECON_RED_DIFFSQ: DK_TRY(chain(k_reduce1<DECON_RED_DIFFSQ>, g, kRedThreads, 0, st, a, b, n, partials)); break;
+        case DECON_RED_DOT: DK_TRY(chain(k_reduce1<DECON_RED_DOT>, g, kRedThreads, 0, st, a, b, n, partials)); break;
+        case DECON_RED_MAX: DK_TRY(chain(k_reduce1<DECON_RED_MAX>, g, kRedThreads, 0, st, a, b, n, partials)); break;
         default: return fail(DECON_ERR_VALUE, "reduce: unknown op %d", op);
     }
     DK_LAUNCHED();
-    if (op == DECON_RED_MAX) k_reduce2<true><<<1, kRedThreads, 0, st>>>(partials, g, out);
-    else k_reduce2<false><<<1, kRedThreads, 0, st>>>(partials, g, out);
+    if (op == DECON_RED_MAX) DK_TRY(chain(k_reduce2<true>, 1, kRedThreads, 0, st, partials, g, out));
+    else DK_TRY(chain(k_reduce2<false>, 1, kRedThreads, 0, st, partials, g, out));
     DK_LAUNCHED();
     return DECON_OK;
 }
 
 int finish_partials(const double* partials, int n, double* out, cudaStream_t st) {
-    k_reduce2<false><<<1, kRedThreads, 0, st>>>(partials, n, out);
+    DK_TRY(chain(k_reduce2<false>, 1, kRedThreads, 0, st, partials, n, out));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -103,6 +105,7 @@ int finish_partials(const double* partials, int n, double* out, cudaStream_t st)
 __global__ void __launch_bounds__(kRedThreads) k_maxabs2(const float2* __restrict__ z, int64_t rows,
                                                          int64_t cols, int64_t pitch,
                                                          double* __restrict__ partials) {
+    chain_enter();
     double acc = 0.0;
     const int64_t n = rows * cols, stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -126,9 +129,9 @@ __global__ void __launch_bounds__(kRedThreads) k_maxabs2(const float2* __restric
 int max_abs2(const float2* z, int64_t rows, int64_t cols, int64_t pitch, double* out,
              double* partials, cudaStream_t st) {
     const int g = red_blocks(rows * cols);
-    k_maxabs2<<<g, kRedThreads, 0, st>>>(z, rows, cols, pitch, partials);
+    DK_TRY(chain(k_maxabs2, g, kRedThreads, 0, st, z, rows, cols, pitch, partials));
     DK_LAUNCHED();
-    k_reduce2<true><<<1, kRedThreads, 0, st>>>(partials, g, out);
+    DK_TRY(chain(k_reduce2<true>, 1, kRedThreads, 0, st, partials, g, out));
     DK_LAUNCHED();
     return DECON_OK;
 }

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256) k_dual_data(PdhgDev* s, float* __restrict
                                                    const float* __restrict__ axp,
                                                    const float* __restrict__ data, float bg,
                                                    int64_t m) {
+    chain_enter();
     if (s->stop) return;
     const float sg = (float)s->sigma, th = (float)s->theta;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
@@ -72,6 +73,7 @@ template <int NORM>
 __global__ void __launch_bounds__(256) k_dual_reg(PdhgDev* s, float* __restrict__ y2,
                                                   const float* __restrict__ lxbar, float alpha,
                                                   int ncomp, int64_t n) {
+    chain_enter();
     if (s->stop) return;
     const float sg = (float)s->sigma;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -101,6 +103,7 @@ __global__ void __launch_bounds__(256) k_dual_reg(PdhgDev* s, float* __restrict_
 __global__ void __launch_bounds__(256) k_xbar(PdhgDev* s, const float* __restrict__ xc,
                                               const float* __restrict__ xp, float* __restrict__ xb,
                                               int64_t n) {
+    chain_enter();
     if (s->stop) return;
     const float th = (float)s->theta;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -116,6 +119,7 @@ __global__ void __launch_bounds__(256) k_primal(PdhgDev* s, const float* __restr
                                                 const float* __restrict__ aty,
                                                 const float* __restrict__ lty,
                                                 float* __restrict__ xn, int64_t n) {
+    chain_enter();
     if (s->stop) return;
     const float tau = (float)s->tau;
     double dx2 = 0.0, xc2 = 0.0, xn2 = 0.0;
@@ -139,6 +143,7 @@ __global__ void __launch_bounds__(256) k_primal(PdhgDev* s, const float* __restr
 __global__ void __launch_bounds__(256) k_diffsq_slot(PdhgDev* s, const float* __restrict__ a,
                                                      const float* __restrict__ b, int64_t n,
                                                      int slot) {
+    chain_enter();
     if (s->stop) return;
     double acc = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -153,6 +158,7 @@ __global__ void __launch_bounds__(256) k_diffsq_slot(PdhgDev* s, const float* __
 __global__ void __launch_bounds__(256) k_sub(PdhgDev* s, const float* __restrict__ a,
                                              const float* __restrict__ b, float* __restrict__ d,
                                              int64_t n) {
+    chain_enter();
     if (s->stop) return;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -164,6 +170,7 @@ template <int LOSS>
 __global__ void __launch_bounds__(256) k_loss_data(PdhgDev* s, const float* __restrict__ ax,
                                                    const float* __restrict__ data, float bg,
                                                    int64_t m, int kk) {
+    chain_enter();
     if (!loss_active(s, kk)) return;
     double acc = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
@@ -185,6 +192,7 @@ __global__ void __launch_bounds__(256) k_loss_data(PdhgDev* s, const float* __re
 template <int NORM>
 __global__ void __launch_bounds__(256) k_loss_reg(PdhgDev* s, const float* __restrict__ lx,
                                                   int ncomp, int64_t n, int kk) {
+    chain_enter();
     if (!loss_active(s, kk)) return;
     double acc = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -219,6 +227,7 @@ __device__ double fold_slot(const PdhgDev* s, int slot) {
 
 // The Malitsky-Pock scalar step (pdhg_mlx.py:749-857) in FP64, one CTA.
 __global__ void __launch_bounds__(256) k_step(PdhgDev* s) {
+    chain_enter();
     if (s->stop) return;
     // the five FP64 sums folded at once, one warp per slot (fixed order)
     __shared__ double red[5];
@@ -287,6 +296,7 @@ __global__ void __launch_bounds__(256) k_step(PdhgDev* s) {
 
 // Records alpha-weighted loss for iteration k-1 (called after k_step).
 __global__ void k_record_loss(PdhgDev* s, double alpha, int kk) {
+    chain_enter();
     if (!loss_active(s, kk)) return;
     const double dl = fold_slot(s, kSlotData);
     const double rl = fold_slot(s, kSlotReg);
@@ -334,6 +344,7 @@ __global__ void __launch_bounds__(256) k_hess_dual(PdhgDev* s, float* __restrict
                                                    const float* __restrict__ xc,
                                                    const float* __restrict__ xp, Dims d, W6 w,
                                                    float alpha) {
+    chain_enter();
     if (s->stop) return;
     const float sg = (float)s->sigma;
     const XbarField f{xc, xp, (float)s->theta, d.ny, d.nx};
@@ -369,6 +380,7 @@ __global__ void __launch_bounds__(256) k_hess_primal(PdhgDev* s, const float* __
                                                      const float* __restrict__ aty,
                                                      const float* __restrict__ y2,
                                                      float* __restrict__ xn, Dims d, W6 w) {
+    chain_enter();
     if (s->stop) return;
     const float tau = (float)s->tau;
     const int64_t n = d.nz * d.ny * d.nx;
@@ -395,6 +407,7 @@ __global__ void __launch_bounds__(256) k_hess_dk(PdhgDev* s, const float* __rest
                                                  const float* __restrict__ axc, int64_t m,
                                                  const float* __restrict__ xn,
                                                  const float* __restrict__ xc, Dims d, W6 w) {
+    chain_enter();
     if (s->stop) return;
     double a2 = 0.0, l2 = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
@@ -420,6 +433,7 @@ __global__ void __launch_bounds__(256) k_hess_dk(PdhgDev* s, const float* __rest
 template <int NORM>
 __global__ void __launch_bounds__(256) k_hess_regloss(PdhgDev* s, const float* __restrict__ x,
                                                       Dims d, W6 w, int kk) {
+    chain_enter();
     if (!loss_active(s, kk)) return;
     const PlainField f{x, d.ny, d.nx};
     const int64_t n = d.nz * d.ny * d.nx;
@@ -446,6 +460,7 @@ __global__ void __launch_bounds__(256) k_hess_regloss(PdhgDev* s, const float* _
 
 __global__ void k_rl_ratio(const float* __restrict__ model, const float* __restrict__ y, float bg,
                            float* __restrict__ ratio, int64_t n, double* __restrict__ partials) {
+    chain_enter();
     double acc = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -465,6 +480,7 @@ __global__ void k_rl_ratio(const float* __restrict__ model, const float* __restr
 
 __global__ void k_rl_update(float* __restrict__ x, const float* __restrict__ corr,
                             const float* __restrict__ sens, int64_t n) {
+    chain_enter();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const float s = sens[i];
@@ -474,6 +490,7 @@ __global__ void k_rl_update(float* __restrict__ x, const float* __restrict__ cor
 }
 
 __global__ void k_sub_floor(const float* __restrict__ y, float bg, float* __restrict__ out, int64_t n) {
+    chain_enter();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
         out[i] = fmaxf(y[i] - bg, 1e-6f);  // rl_mlx.py:123
@@ -481,6 +498,7 @@ __global__ void k_sub_floor(const float* __restrict__ y, float bg, float* __rest
 
 __global__ void k_rl_mask_generic(float* __restrict__ x, float* __restrict__ sens,
                                   const double* smax, int64_t n) {
+    chain_enter();
     const float fl = fmaxf((float)(*smax) * 1e-6f, 1e-10f);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -492,6 +510,7 @@ __global__ void k_rl_mask_generic(float* __restrict__ x, float* __restrict__ sen
 }
 
 __global__ void k_fill(float* __restrict__ p, float v, int64_t n) {
+    chain_enter();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
         p[i] = v;
@@ -499,12 +518,14 @@ __global__ void k_fill(float* __restrict__ p, float v, int64_t n) {
 
 __global__ void k_affine(const float* __restrict__ a, float alpha, float beta,
                          float* __restrict__ out, int64_t n) {
+    chain_enter();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
         out[i] = alpha * a[i] + beta;
 }
 
 __global__ void k_clamp_min(const float* __restrict__ a, float lo, float* __restrict__ out, int64_t n) {
+    chain_enter();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
         out[i] = fmaxf(a[i], lo);
@@ -513,9 +534,9 @@ __global__ void k_clamp_min(const float* __restrict__ a, float lo, float* __rest
 int hess_adjoint_tiled(const float* hw, float* out, const Dims& d, const W6& w, cudaStream_t st) {
     const int64_t grid = std::min<int64_t>(TileGeo(d).ntiles, (int64_t)sm_count() * 4);
     if (offsets_fit_u32(d))
-        k_hessian_adj_t<uint32_t><<<(unsigned)std::max<int64_t>(grid, 1), 256, 0, st>>>(hw, out, d, w);
+        DK_TRY(chain(k_hessian_adj_t<uint32_t>, (unsigned)std::max<int64_t>(grid, 1), 256, 0, st, hw, out, d, w));
     else
-        k_hessian_adj_t<int64_t><<<(unsigned)std::max<int64_t>(grid, 1), 256, 0, st>>>(hw, out, d, w);
+        DK_TRY(chain(k_hessian_adj_t<int64_t>, (unsigned)std::max<int64_t>(grid, 1), 256, 0, st, hw, out, d, w));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -645,9 +666,9 @@ int decon_pdhg_dual_data(decon_pdhg* h, float* y1, const float* ax_cur, const fl
     if (!h || !y1 || !ax_cur || !ax_prev || !data) return fail(DECON_ERR_NULL, "null pointer");
     const cudaStream_t s = as_stream(stream);
     if (loss_type == 0)
-        k_dual_data<0><<<g1(m), 256, 0, s>>>(h->dev, y1, ax_cur, ax_prev, data, background, m);
+        DK_TRY(chain(k_dual_data<0>, g1(m), 256, 0, s, h->dev, y1, ax_cur, ax_prev, data, background, m));
     else
-        k_dual_data<1><<<g1(m), 256, 0, s>>>(h->dev, y1, ax_cur, ax_prev, data, background, m);
+        DK_TRY(chain(k_dual_data<1>, g1(m), 256, 0, s, h->dev, y1, ax_cur, ax_prev, data, background, m));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -658,9 +679,9 @@ int decon_pdhg_dual_reg(decon_pdhg* h, float* y2, const float* lxbar, float alph
     if (ncomp < 1 || ncomp > 8) return fail(DECON_ERR_VALUE, "ncomp must be 1..8");
     const cudaStream_t s = as_stream(stream);
     if (norm == 0)
-        k_dual_reg<0><<<g1(n), 256, 0, s>>>(h->dev, y2, lxbar, alpha, ncomp, n);
+        DK_TRY(chain(k_dual_reg<0>, g1(n), 256, 0, s, h->dev, y2, lxbar, alpha, ncomp, n));
     else
-        k_dual_reg<1><<<g1(n), 256, 0, s>>>(h->dev, y2, lxbar, alpha, ncomp, n);
+        DK_TRY(chain(k_dual_reg<1>, g1(n), 256, 0, s, h->dev, y2, lxbar, alpha, ncomp, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -668,7 +689,7 @@ int decon_pdhg_dual_reg(decon_pdhg* h, float* y2, const float* lxbar, float alph
 int decon_pdhg_xbar(decon_pdhg* h, const float* xc, const float* xp, float* xbar, int64_t n,
                     void* stream) {
     if (!h || !xc || !xp || !xbar) return fail(DECON_ERR_NULL, "null pointer");
-    k_xbar<<<g1(n), 256, 0, as_stream(stream)>>>(h->dev, xc, xp, xbar, n);
+    DK_TRY(chain(k_xbar, g1(n), 256, 0, as_stream(stream), h->dev, xc, xp, xbar, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -676,14 +697,14 @@ int decon_pdhg_xbar(decon_pdhg* h, const float* xc, const float* xp, float* xbar
 int decon_pdhg_primal(decon_pdhg* h, const float* xc, const float* aty, const float* lty,
                       float* xn, int64_t n, void* stream) {
     if (!h || !xc || !aty || !xn) return fail(DECON_ERR_NULL, "null pointer");
-    k_primal<<<kPdhgGrid, 256, 0, as_stream(stream)>>>(h->dev, xc, aty, lty, xn, n);
+    DK_TRY(chain(k_primal, kPdhgGrid, 256, 0, as_stream(stream), h->dev, xc, aty, lty, xn, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
 
 int decon_pdhg_sub(decon_pdhg* h, const float* a, const float* b, float* d, int64_t n, void* stream) {
     if (!h || !a || !b || !d) return fail(DECON_ERR_NULL, "null pointer");
-    k_sub<<<g1(n), 256, 0, as_stream(stream)>>>(h->dev, a, b, d, n);
+    DK_TRY(chain(k_sub, g1(n), 256, 0, as_stream(stream), h->dev, a, b, d, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -692,10 +713,10 @@ int decon_pdhg_dk(decon_pdhg* h, const float* ax_new, const float* ax_cur, int64
                   const float* l_dx, int64_t nl, void* stream) {
     if (!h || !ax_new || !ax_cur) return fail(DECON_ERR_NULL, "null pointer");
     const cudaStream_t s = as_stream(stream);
-    k_diffsq_slot<<<kPdhgGrid, 256, 0, s>>>(h->dev, ax_new, ax_cur, m, kSlotDA2);
+    DK_TRY(chain(k_diffsq_slot, kPdhgGrid, 256, 0, s, h->dev, ax_new, ax_cur, m, kSlotDA2));
     DK_LAUNCHED();
     if (l_dx) {
-        k_diffsq_slot<<<kPdhgGrid, 256, 0, s>>>(h->dev, l_dx, nullptr, nl, kSlotDL2);
+        DK_TRY(chain(k_diffsq_slot, kPdhgGrid, 256, 0, s, h->dev, l_dx, nullptr, nl, kSlotDL2));
         DK_LAUNCHED();
     }
     return DECON_OK;
@@ -703,7 +724,7 @@ int decon_pdhg_dk(decon_pdhg* h, const float* ax_new, const float* ax_cur, int64
 
 int decon_pdhg_step(decon_pdhg* h, void* stream) {
     if (!h) return fail(DECON_ERR_NULL, "null pointer");
-    k_step<<<1, 256, 0, as_stream(stream)>>>(h->dev);
+    DK_TRY(chain(k_step, 1, 256, 0, as_stream(stream), h->dev));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -714,13 +735,13 @@ int decon_pdhg_loss(decon_pdhg* h, const float* ax, const float* data, float bac
     if (!h || !ax || !data || !lx) return fail(DECON_ERR_NULL, "null pointer");
     if (k < 0 || k >= std::max(h->num_iter, 1)) return fail(DECON_ERR_VALUE, "loss index out of range");
     const cudaStream_t s = as_stream(stream);
-    if (loss_type == 0) k_loss_data<0><<<kPdhgGrid, 256, 0, s>>>(h->dev, ax, data, background, m, k);
-    else k_loss_data<1><<<kPdhgGrid, 256, 0, s>>>(h->dev, ax, data, background, m, k);
+    if (loss_type == 0) DK_TRY(chain(k_loss_data<0>, kPdhgGrid, 256, 0, s, h->dev, ax, data, background, m, k));
+    else DK_TRY(chain(k_loss_data<1>, kPdhgGrid, 256, 0, s, h->dev, ax, data, background, m, k));
     DK_LAUNCHED();
-    if (norm == 0) k_loss_reg<0><<<kPdhgGrid, 256, 0, s>>>(h->dev, lx, ncomp, n, k);
-    else k_loss_reg<1><<<kPdhgGrid, 256, 0, s>>>(h->dev, lx, ncomp, n, k);
+    if (norm == 0) DK_TRY(chain(k_loss_reg<0>, kPdhgGrid, 256, 0, s, h->dev, lx, ncomp, n, k));
+    else DK_TRY(chain(k_loss_reg<1>, kPdhgGrid, 256, 0, s, h->dev, lx, ncomp, n, k));
     DK_LAUNCHED();
-    k_record_loss<<<1, 256, 0, s>>>(h->dev, alpha, k);
+    DK_TRY(chain(k_record_loss, 1, 256, 0, s, h->dev, alpha, k));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -739,9 +760,9 @@ int decon_pdhg_hess_dual(decon_pdhg* h, float* y2, const float* xc, const float*
     DK_TRY(smem_prepare(fn, DualLayout::bytes, &per_sm));
     const int grid = (int)std::min<int64_t>(tg.ntiles, (int64_t)sm_count() * per_sm);
     if (norm == 0)
-        k_hess_dual_p<0><<<grid, 256, DualLayout::bytes, as_stream(stream)>>>(h->dev, y2, xc, xp, d, w, alpha);
+        DK_TRY(chain(k_hess_dual_p<0>, grid, 256, DualLayout::bytes, as_stream(stream), h->dev, y2, xc, xp, d, w, alpha));
     else
-        k_hess_dual_p<1><<<grid, 256, DualLayout::bytes, as_stream(stream)>>>(h->dev, y2, xc, xp, d, w, alpha);
+        DK_TRY(chain(k_hess_dual_p<1>, grid, 256, DualLayout::bytes, as_stream(stream), h->dev, y2, xc, xp, d, w, alpha));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -753,11 +774,11 @@ int decon_pdhg_hess_primal(decon_pdhg* h, const float* xc, const float* aty, con
     hessian_weights(r, w.w);
     const Dims d{shape[0], shape[1], shape[2]};
     if (offsets_fit_u32(d))
-        k_hess_primal_t<uint32_t><<<kPdhgGrid, 256, 0, as_stream(stream)>>>(h->dev, xc, aty, y2, xn, d, w, kSlotDx2,
-                                                                           kSlotXc2, kSlotXn2);
+        DK_TRY(chain(k_hess_primal_t<uint32_t>, kPdhgGrid, 256, 0, as_stream(stream), h->dev, xc, aty, y2, xn, d, w, kSlotDx2,
+                                                                           kSlotXc2, kSlotXn2));
     else
-        k_hess_primal_t<int64_t><<<kPdhgGrid, 256, 0, as_stream(stream)>>>(h->dev, xc, aty, y2, xn, d, w, kSlotDx2,
-                                                                          kSlotXc2, kSlotXn2);
+        DK_TRY(chain(k_hess_primal_t<int64_t>, kPdhgGrid, 256, 0, as_stream(stream), h->dev, xc, aty, y2, xn, d, w, kSlotDx2,
+                                                                          kSlotXc2, kSlotXn2));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -775,11 +796,11 @@ int decon_pdhg_hess_dual_primal(decon_pdhg* h, const float* y2_in, float* y2_out
     const int grid = (int)std::min<int64_t>(kPdhgGrid, std::max<int64_t>(TileGeo(d).ntiles, 1));
     const cudaStream_t s = as_stream(stream);
     if (norm == 0)
-        k_hess_dual_primal<0><<<grid, 256, 0, s>>>(h->dev, y2_in, y2_out, xc, xp, aty, xn, d, w, alpha,
-                                                   kSlotDx2, kSlotXc2, kSlotXn2);
+        DK_TRY(chain(k_hess_dual_primal<0>, grid, 256, 0, s, h->dev, y2_in, y2_out, xc, xp, aty, xn, d, w, alpha,
+                                                   kSlotDx2, kSlotXc2, kSlotXn2));
     else
-        k_hess_dual_primal<1><<<grid, 256, 0, s>>>(h->dev, y2_in, y2_out, xc, xp, aty, xn, d, w, alpha,
-                                                   kSlotDx2, kSlotXc2, kSlotXn2);
+        DK_TRY(chain(k_hess_dual_primal<1>, grid, 256, 0, s, h->dev, y2_in, y2_out, xc, xp, aty, xn, d, w, alpha,
+                                                   kSlotDx2, kSlotXc2, kSlotXn2));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -799,11 +820,11 @@ int decon_pdhg_hess_dk(decon_pdhg* h, const float* ax_new, const float* ax_cur, 
     // from decon_pdhg_dk with l_dx = NULL); the empty A sum goes to the spare
     // slot 7 so that the two kernels may run concurrently
     if (u32)
-        k_hess_dk_r<uint32_t><<<grid, 256, 0, as_stream(stream)>>>(h->dev, ax_new, ax_cur, ax_new ? m : 0, xn, xc,
-                                                                  d, w, ax_new ? kSlotDA2 : kPdhgSlots - 1, kSlotDL2);
+        DK_TRY(chain(k_hess_dk_r<uint32_t>, grid, 256, 0, as_stream(stream), h->dev, ax_new, ax_cur, ax_new ? m : 0, xn, xc,
+                                                                  d, w, ax_new ? kSlotDA2 : kPdhgSlots - 1, kSlotDL2));
     else
-        k_hess_dk_r<int64_t><<<grid, 256, 0, as_stream(stream)>>>(h->dev, ax_new, ax_cur, ax_new ? m : 0, xn, xc,
-                                                                 d, w, ax_new ? kSlotDA2 : kPdhgSlots - 1, kSlotDL2);
+        DK_TRY(chain(k_hess_dk_r<int64_t>, grid, 256, 0, as_stream(stream), h->dev, ax_new, ax_cur, ax_new ? m : 0, xn, xc,
+                                                                 d, w, ax_new ? kSlotDA2 : kPdhgSlots - 1, kSlotDL2));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -817,17 +838,17 @@ int decon_pdhg_hess_loss(decon_pdhg* h, const float* ax, const float* data, floa
     hessian_weights(r, w.w);
     const Dims d{shape[0], shape[1], shape[2]};
     const cudaStream_t s = as_stream(stream);
-    if (loss_type == 0) k_loss_data<0><<<kPdhgGrid, 256, 0, s>>>(h->dev, ax, data, background, m, k);
-    else k_loss_data<1><<<kPdhgGrid, 256, 0, s>>>(h->dev, ax, data, background, m, k);
+    if (loss_type == 0) DK_TRY(chain(k_loss_data<0>, kPdhgGrid, 256, 0, s, h->dev, ax, data, background, m, k));
+    else DK_TRY(chain(k_loss_data<1>, kPdhgGrid, 256, 0, s, h->dev, ax, data, background, m, k));
     DK_LAUNCHED();
     int per_sm = 1;
     DK_TRY(smem_prepare(norm == 0 ? (const void*)k_hess_regloss_p<0> : (const void*)k_hess_regloss_p<1>,
                         LossLayout::bytes, &per_sm));
     const int grid = std::min(kPdhgGrid, sm_count() * per_sm);
-    if (norm == 0) k_hess_regloss_p<0><<<grid, 256, LossLayout::bytes, s>>>(h->dev, x, d, w, k, kSlotReg);
-    else k_hess_regloss_p<1><<<grid, 256, LossLayout::bytes, s>>>(h->dev, x, d, w, k, kSlotReg);
+    if (norm == 0) DK_TRY(chain(k_hess_regloss_p<0>, grid, 256, LossLayout::bytes, s, h->dev, x, d, w, k, kSlotReg));
+    else DK_TRY(chain(k_hess_regloss_p<1>, grid, 256, LossLayout::bytes, s, h->dev, x, d, w, k, kSlotReg));
     DK_LAUNCHED();
-    k_record_loss<<<1, 256, 0, s>>>(h->dev, alpha, k);
+    DK_TRY(chain(k_record_loss, 1, 256, 0, s, h->dev, alpha, k));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -885,7 +906,7 @@ int decon_rl_ratio(const float* model, const float* observed, float background, 
     const cudaStream_t s = as_stream(stream);
     const int g = std::min<int>(g1(n), (int)reduce_partials_needed());
     double* part = loss_sum ? static_cast<double*>(workspace) : nullptr;
-    k_rl_ratio<<<g, 256, 0, s>>>(model, observed, background, ratio, n, part);
+    DK_TRY(chain(k_rl_ratio, g, 256, 0, s, model, observed, background, ratio, n, part));
     DK_LAUNCHED();
     if (loss_sum) DK_TRY(finish_partials(part, g, loss_sum, s));
     return DECON_OK;
@@ -893,14 +914,14 @@ int decon_rl_ratio(const float* model, const float* observed, float background, 
 
 int decon_rl_update(float* x, const float* corr, const float* sens_masked, int64_t n, void* stream) {
     if (!x || !corr || !sens_masked) return fail(DECON_ERR_NULL, "null pointer");
-    k_rl_update<<<g1(n), 256, 0, as_stream(stream)>>>(x, corr, sens_masked, n);
+    DK_TRY(chain(k_rl_update, g1(n), 256, 0, as_stream(stream), x, corr, sens_masked, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
 
 int decon_rl_data_floor(const float* observed, float background, float* out, int64_t n, void* stream) {
     if (!observed || !out) return fail(DECON_ERR_NULL, "null pointer");
-    k_sub_floor<<<g1(n), 256, 0, as_stream(stream)>>>(observed, background, out, n);
+    DK_TRY(chain(k_sub_floor, g1(n), 256, 0, as_stream(stream), observed, background, out, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -911,7 +932,7 @@ int decon_rl_mask(float* x, float* sens, int64_t n, void* workspace, void* strea
     double* ws = static_cast<double*>(workspace);
     // the max lands in ws[0]; partials use the rest
     DK_TRY(reduce_f32(sens, nullptr, n, DECON_RED_MAX, ws, ws + 1, reduce_partials_needed() - 1, s));
-    k_rl_mask_generic<<<g1(n), 256, 0, s>>>(x, sens, ws, n);
+    DK_TRY(chain(k_rl_mask_generic, g1(n), 256, 0, s, x, sens, ws, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -919,7 +940,7 @@ int decon_rl_mask(float* x, float* sens, int64_t n, void* workspace, void* strea
 int decon_fill(float* p, float value, int64_t n, void* stream) {
     if (!p) return fail(DECON_ERR_NULL, "null pointer");
     if (n <= 0) return DECON_OK;
-    k_fill<<<g1(n), 256, 0, as_stream(stream)>>>(p, value, n);
+    DK_TRY(chain(k_fill, g1(n), 256, 0, as_stream(stream), p, value, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -927,7 +948,7 @@ int decon_fill(float* p, float value, int64_t n, void* stream) {
 int decon_affine(const float* a, float alpha, float beta, float* out, int64_t n, void* stream) {
     if (!a || !out) return fail(DECON_ERR_NULL, "null pointer");
     if (n <= 0) return DECON_OK;
-    k_affine<<<g1(n), 256, 0, as_stream(stream)>>>(a, alpha, beta, out, n);
+    DK_TRY(chain(k_affine, g1(n), 256, 0, as_stream(stream), a, alpha, beta, out, n));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -935,7 +956,7 @@ int decon_affine(const float* a, float alpha, float beta, float* out, int64_t n,
 int decon_clamp_min(const float* a, float lo, float* out, int64_t n, void* stream) {
     if (!a || !out) return fail(DECON_ERR_NULL, "null pointer");
     if (n <= 0) return DECON_OK;
-    k_clamp_min<<<g1(n), 256, 0, as_stream(stream)>>>(a, lo, out, n);
+    DK_TRY(chain(k_clamp_min, g1(n), 256, 0, as_stream(stream), a, lo, out, n));
     DK_LAUNCHED();
     return DECON_OK;
 }

@@ -68,6 +68,7 @@ __device__ __forceinline__ float fetch_x(const XR2CArgs& a, const RowSrc& r, int
 template <int PRO>
 __global__ void __launch_bounds__(kDynThreads, 1) k_xr2c(XR2CArgs a) {
     extern __shared__ float2 sm[];
+    chain_enter();
     __shared__ RowSrc rsrc[32];  // per-row source (general path)
     const int T = a.T, L = a.ax.L, tid = threadIdx.x;
     const int64_t row0 = (int64_t)blockIdx.x * T;
@@ -290,6 +291,7 @@ __device__ __forceinline__ void epilogue(const XC2RArgs& a, int64_t i, float v, 
 template <int EPI>
 __global__ void __launch_bounds__(kDynThreads, 1) k_xc2r(XC2RArgs a) {
     extern __shared__ float2 sm[];
+    chain_enter();
     __shared__ float2 nyq[32];    // X[M] of each row (even Fx)
     __shared__ int64_t obase[32];  // output index of x = 0 of each row (general path)
     constexpr int64_t kOutside = INT64_MIN;

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
     extern __shared__ float2 sm[];
     const int tid = threadIdx.x;
     const uint32_t line0 = blockIdx.x * TL;
+    chain_enter();
     float2* stg = sm + TL * E::pitch;  // staged rows (XS_KERNEL)
     if constexpr (SRC == XS_KERNEL) {
         __shared__ const float* rows[2 * TL];
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
     extern __shared__ float2 sm[];
     const int tid = threadIdx.x;
     const uint32_t line0 = blockIdx.x * TL;
+    chain_enter();
 
     // stage 1
     {
