@@ -88,41 +88,100 @@ int sm_count() {
 int max_abs2(const float2* z, int64_t rows, int64_t cols, int64_t pitch, double* out,
              double* partials, cudaStream_t st);
 
-// Twiddle table W_L^m = exp(-2 pi i m / L), m < L, computed in double.
-static int make_twiddles(int L, float2** out) {
-    std::vector<float2> h(std::max(L, 1));
-    for (int m = 0; m < L; ++m) {
-        const double a = -2.0 * M_PI * (double)m / (double)L;
-        h[m] = make_float2((float)std::cos(a), (float)std::sin(a));
+int twiddle_table(int L, const float2** out) {
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, float2*> cache;
+    int dev = 0;
+    DK_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    float2*& t = cache[std::make_pair(dev, L)];
+    if (!t) {
+        std::vector<float2> h(std::max(L, 1));
+        for (int m = 0; m < L; ++m) {
+            const double a = -2.0 * M_PI * (double)m / (double)L;
+            h[m] = make_float2((float)std::cos(a), (float)std::sin(a));
+        }
+        float2* d = nullptr;
+        DK_CUDA(cudaMalloc(&d, h.size() * sizeof(float2)));
+        const int st = upload_blocking(d, h.data(), h.size() * sizeof(float2));
+        if (st != DECON_OK) {
+            cudaFree(d);
+            return st;
+        }
+        t = d;
     }
-    DK_CUDA(cudaMalloc(out, h.size() * sizeof(float2)));
-    DK_TRY(upload_blocking(*out, h.data(), h.size() * sizeof(float2)));
+    *out = t;
     return DECON_OK;
 }
 
-static void free_plan(ConvPlan* p) {
-    if (!p) return;
-    cudaFree(p->otft);
-    cudaFree(p->otf16);
-    cudaFree(p->otf_inv);
-    cudaFree(p->otf);
-    cudaFree(p->s1);
-    cudaFree(p->s2);
-    cudaFree(p->twx);
-    cudaFree(p->twy);
-    cudaFree(p->twz);
-    cudaFree(p->dscal);
-    cudaFree(p->partials);
+constexpr uint64_t kPoolKeep = uint64_t(2) << 30;
+
+int device_pool(cudaMemPool_t* out) {
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    int dev = 0;
+    DK_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = pools.find(dev);
+    if (it == pools.end()) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool;
+        DK_CUDA(cudaMemPoolCreate(&pool, &props));
+        uint64_t keep = kPoolKeep;
+        DK_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        it = pools.emplace(dev, pool).first;
+    }
+    *out = it->second;
+    return DECON_OK;
 }
 
-static int dev_alloc(void** p, size_t bytes, const char* what) {
-    cudaError_t e = cudaMalloc(p, bytes);
+int pool_alloc(void** p, size_t bytes, const char* what) {
+    *p = nullptr;
+    cudaMemPool_t pool;
+    DK_TRY(device_pool(&pool));
+    const cudaStream_t s = setup_stream();
+    if (!s) return fail(DECON_ERR_CUDA, "set-up stream creation failed");
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaStreamSynchronize(s);
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         cudaGetLastError();
+        *p = nullptr;
         return fail(e == cudaErrorMemoryAllocation ? DECON_ERR_OOM : DECON_ERR_CUDA,
                     "cudaMalloc of %zu bytes for %s failed: %s", bytes, what, cudaGetErrorString(e));
     }
     return DECON_OK;
+}
+
+void pool_free(std::initializer_list<void*> ptrs) {
+    void* first = nullptr;
+    for (void* p : ptrs) first = first ? first : p;
+    if (!first) return;
+    // the pool and its stream belong to the device of the memory
+    int cur = 0;
+    cudaGetDevice(&cur);
+    cudaPointerAttributes at{};
+    const bool other = cudaPointerGetAttributes(&at, first) == cudaSuccess && at.device != cur;
+    if (other) cudaSetDevice(at.device);
+    cudaDeviceSynchronize();
+    const cudaStream_t s = setup_stream();
+    for (void* p : ptrs)
+        if (p) cudaFreeAsync(p, s);
+    if (other) cudaSetDevice(cur);
+    cudaGetLastError();
+}
+
+static void free_plan(ConvPlan* p) {
+    if (!p) return;
+    pool_free({p->otft, p->otf16, p->otf_inv, p->otf, p->s1, p->s2, p->dscal, p->partials});
 }
 
 // Elementwise helpers used by the RL set-up.
@@ -227,21 +286,16 @@ int decon_fast_padded_shape(int ndim, const int64_t* signal, const int64_t* kern
 
 // Kernel sum (FP64, linops_mlx.py:408-409) and OTF = rfftn(kernel canvas):
 // X pass over all Fz*Fy rows straight into the OTF buffer, then in-place Y
-// and Z forward passes (unpruned); operator_norm_sq = max |OTF|^2.  Reads
-// the two FP64 scalars back (synchronises the stream).
+// and Z forward passes (unpruned); operator_norm_sq = max |OTF|^2, read back
+// (synchronises the stream).
 static int build_otf(decon_conv* p, const float* kernel, int normalize, cudaStream_t s) {
     int st;
     const int64_t Fz = p->F[0], Fy = p->F[1];
-    p->kdiv = 1.f;
     const int64_t nk = p->K[0] * p->K[1] * p->K[2];
-    if (normalize) {
+    // the sum stays on the device: the X pass divides by it as it loads
+    if (normalize)
         DK_TRY(reduce_f32(kernel, nullptr, nk, DECON_RED_SUM, p->dscal, p->partials, p->npartials, s));
-        double ksum = 0;
-        cudaError_t e = cudaMemcpyAsync(&ksum, p->dscal, sizeof(double), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return fail(DECON_ERR_CUDA, "kernel sum failed: %s", cudaGetErrorString(e));
-        p->kdiv = (float)ksum;
-    }
+    p->ksum = normalize ? p->dscal : nullptr;
     Win3 none{0, 0, 0, 0, 0, 0};
     if ((st = launch_xr2c(*p, PRO_KERNEL, kernel, none, 0.f, 0.f, Fz, p->otf, s)) ||
         (st = transform_otf(*p, 1, s)) || (st = transform_otf(*p, 0, s)) ||
@@ -310,8 +364,8 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
     int st;
     const cudaStream_t s = as_stream(stream);
     const int64_t nz = p->N[0], ny = p->N[1];
-    if ((st = make_twiddles((int)Fx, &p->twx)) || (st = make_twiddles((int)Fy, &p->twy)) ||
-        (st = make_twiddles((int)Fz, &p->twz))) {
+    if ((st = twiddle_table((int)Fx, &p->twx)) || (st = twiddle_table((int)Fy, &p->twy)) ||
+        (st = twiddle_table((int)Fz, &p->twz))) {
         free_plan(p);
         delete p;
         return st;
@@ -323,11 +377,11 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
     p->ax_z.tw = p->twz;
     p->ax_z.tws = 1;
     p->npartials = std::max<int64_t>(reduce_partials_needed(), cdiv(nz * ny, std::min(p->T_x, 4)) + 1);
-    if ((st = dev_alloc((void**)&p->otf, (size_t)Fz * Fy * p->P * sizeof(float2), "OTF")) ||
-        (st = dev_alloc((void**)&p->s1, (size_t)nz * ny * p->P * sizeof(float2), "spectrum S1")) ||
-        (st = dev_alloc((void**)&p->s2, (size_t)nz * Fy * p->P * sizeof(float2), "spectrum S2")) ||
-        (st = dev_alloc((void**)&p->dscal, 16 * sizeof(double), "scalars")) ||
-        (st = dev_alloc((void**)&p->partials, p->npartials * sizeof(double), "partials"))) {
+    if ((st = pool_alloc((void**)&p->otf, (size_t)Fz * Fy * p->P * sizeof(float2), "OTF")) ||
+        (st = pool_alloc((void**)&p->s1, (size_t)nz * ny * p->P * sizeof(float2), "spectrum S1")) ||
+        (st = pool_alloc((void**)&p->s2, (size_t)nz * Fy * p->P * sizeof(float2), "spectrum S2")) ||
+        (st = pool_alloc((void**)&p->dscal, 16 * sizeof(double), "scalars")) ||
+        (st = pool_alloc((void**)&p->partials, p->npartials * sizeof(double), "partials"))) {
         free_plan(p);
         delete p;
         return st;
@@ -336,7 +390,7 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
     // otherwise decon_conv_set_schedule allocates it on request
     if (!circular && yz_supported(p->N, p->F) && getenv("DECON_YZ") != nullptr &&
         getenv("DECON_NO_YZ") == nullptr &&
-        (st = dev_alloc((void**)&p->otft, (size_t)p->Hx * Fy * Fz * sizeof(float2), "kx-major OTF"))) {
+        (st = pool_alloc((void**)&p->otft, (size_t)p->Hx * Fy * Fz * sizeof(float2), "kx-major OTF"))) {
         free_plan(p);
         delete p;
         return st;
@@ -388,8 +442,8 @@ int decon_conv_set_precision(decon_conv* p, int precision, void* stream) {
                     (long long)p->F[0], (long long)p->N[0]);
     const int64_t n = p->F[0] * p->F[1] * p->P;
     int st;
-    if (!p->otf16 && (st = dev_alloc((void**)&p->otf16, (size_t)n * sizeof(__half2), "FP16 OTF"))) return st;
-    if (!p->otf_inv && (st = dev_alloc((void**)&p->otf_inv, (size_t)p->F[0] * sizeof(float), "OTF scales")))
+    if (!p->otf16 && (st = pool_alloc((void**)&p->otf16, (size_t)n * sizeof(__half2), "FP16 OTF"))) return st;
+    if (!p->otf_inv && (st = pool_alloc((void**)&p->otf_inv, (size_t)p->F[0] * sizeof(float), "OTF scales")))
         return st;
     DK_TRY(quantize_otf(*p, as_stream(stream)));
     if (!p->z_otf16.ok) make_z_otf16(*p);
@@ -428,7 +482,7 @@ int decon_conv_set_schedule(decon_conv* p, int sched) {
     }
     if ((sched & DECON_SCHED_FUSED) && !p->otft && yz_supported(p->N, p->F) && p->F[0] != p->N[0]) {
         // the fused pass needs the kx-major OTF copy: allocate and fill it
-        DK_TRY(dev_alloc((void**)&p->otft, (size_t)p->Hx * p->F[1] * p->F[0] * sizeof(float2),
+        DK_TRY(pool_alloc((void**)&p->otft, (size_t)p->Hx * p->F[1] * p->F[0] * sizeof(float2),
                          "kx-major OTF"));
         cudaStream_t s = nullptr;
         DK_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));

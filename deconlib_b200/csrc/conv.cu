@@ -294,7 +294,7 @@ int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cva
         a.in = in;
         a.cval = cval;
         a.bg = bg;
-        a.kdiv = p.kdiv;
+        a.ksum = p.ksum;
         a.Nz = nz_rows;
         a.Kz = p.K[0];
         a.Ky = p.K[1];
@@ -321,7 +321,7 @@ int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cva
     a.pz = (p.K[0] + 1) / 2;
     a.py = (p.K[1] + 1) / 2;
     a.px = (p.K[2] + 1) / 2;
-    a.kdiv = p.kdiv;
+    a.ksum = p.ksum;
     a.out = out;
     a.P = p.P;
     a.Hx = (int)p.Hx;

@@ -58,7 +58,8 @@ __device__ __forceinline__ bool kernel_src(int64_t c, int64_t F, int64_t m, int6
 
 struct XR2CArgs {
     const float* in;
-    float cval, bg, kdiv;
+    float cval, bg;
+    const double* ksum;  // kernel sum the values are divided by (nullptr: not normalised)
     int64_t Nz, Ny, Nx;  // rows = Nz * Ny, row length Nx (zero-padded to Fx)
     Win3 win;
     int64_t Kz, Ky, Kx, pz, py, px;  // kernel embedding (PRO_KERNEL)
@@ -126,7 +127,8 @@ ColRegKernel colreg_group_e(int L, int mode);
 struct XRegArgs {
     int pro;               // Prologue (array, constant or RL start in the array kernel)
     const float* in;       // R2C input
-    float cval, bg, kdiv;
+    float cval, bg;
+    const double* ksum;  // kernel sum the values are divided by (nullptr: not normalised)
     int64_t Nz, Ny, Nx;
     int64_t Kz, Ky, Kx, pz, py, px;  // kernel embedding (PRO_KERNEL)
     float2* out;           // R2C output spectrum
@@ -181,11 +183,11 @@ struct ConvPlan {
     Axis ax_x, ax_y, ax_z;
     int T_x, T_y, T_z;
     float2 *otf, *s1, *s2;
-    float2 *twx, *twy, *twz;
+    const float2 *twx, *twy, *twz;
     double* dscal;        // device scalars (kernel sum, reductions)
     double* partials;     // per-CTA FP64 partial sums of fused reductions
     int64_t npartials;
-    float kdiv;
+    const double* ksum;   // device scalar the kernel is divided by, or nullptr
     double norm_sq;
     int device;
     // Register column passes (ok when the axis length has one): Y forward

@@ -426,8 +426,7 @@ struct decon_nlcg {
 
 static int nl_free(decon_nlcg* h) {
     if (!h) return DECON_OK;
-    cudaFree(h->dev);
-    cudaFree(h->part);
+    pool_free({h->dev, h->part});
     cudaFreeHost(h->host);
     delete h;
     return DECON_OK;
@@ -439,8 +438,8 @@ int decon_nlcg_create(decon_nlcg** out) {
     if (!out) return fail(DECON_ERR_NULL, "null pointer");
     *out = nullptr;
     decon_nlcg* h = new decon_nlcg();
-    if (cudaMalloc(&h->dev, sizeof(NlcgDev)) != cudaSuccess ||
-        cudaMalloc(&h->part, sizeof(double) * kNlSlots * kNlMaxBlocks) != cudaSuccess ||
+    if (pool_alloc((void**)&h->dev, sizeof(NlcgDev), "the NLCG state") != DECON_OK ||
+        pool_alloc((void**)&h->part, sizeof(double) * kNlSlots * kNlMaxBlocks, "the NLCG sums") != DECON_OK ||
         cudaMallocHost(&h->host, sizeof(NlcgDev)) != cudaSuccess) {
         cudaGetLastError();
         nl_free(h);

@@ -67,12 +67,7 @@ namespace dk {
 static int pr_alloc(decon_pdhg_solver* s, void** p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
-    const cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(DECON_ERR_OOM, "decon_pdhg_solver: cudaMalloc of %zu bytes failed: %s", bytes,
-                    cudaGetErrorString(e));
-    }
+    DK_TRY(pool_alloc(p, bytes, "decon_pdhg_solver"));
     s->allocs.push_back(*p);
     return DECON_OK;
 }
@@ -327,7 +322,7 @@ int decon_pdhg_solver_state(decon_pdhg_solver* s, decon_pdhg** state, int* queue
 int decon_pdhg_solver_destroy(decon_pdhg_solver* s) {
     if (!s) return DECON_OK;
     if (s->state) decon_pdhg_destroy(s->state);
-    for (void* p : s->allocs) cudaFree(p);
+    for (void* p : s->allocs) dk::pool_free({p});
     delete s;
     return DECON_OK;
 }

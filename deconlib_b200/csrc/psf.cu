@@ -112,59 +112,6 @@ __global__ void __launch_bounds__(1024) k_psf_scan(const int* __restrict__ flags
     }
 }
 
-// Twiddle tables W_L^m = exp(-2 pi i m / L) per (device, L), kept for the
-// life of the process (the first call for a length uploads it and waits for
-// the copy, so every stream may read the table).
-static int psf_twiddles(int L, const float2** out) {
-    static std::mutex mu;
-    static std::map<std::pair<int, int>, float2*> cache;
-    int dev = 0;
-    DK_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    float2*& t = cache[std::make_pair(dev, L)];
-    if (!t) {
-        std::vector<float2> h(L);
-        for (int m = 0; m < L; ++m) {
-            const double ang = -2.0 * M_PI * (double)m / (double)L;
-            h[m] = make_float2((float)std::cos(ang), (float)std::sin(ang));
-        }
-        float2* d = nullptr;
-        DK_CUDA(cudaMalloc(&d, h.size() * sizeof(float2)));
-        if (upload_blocking(d, h.data(), h.size() * sizeof(float2)) != DECON_OK) {
-            cudaFree(d);
-            return fail(DECON_ERR_CUDA, "decon_pupil_to_psf: twiddle upload failed");
-        }
-        t = d;
-    }
-    *out = t;
-    return DECON_OK;
-}
-
-// Stream-ordered scratch from a per-device pool that keeps up to 1 GB
-// reserved between calls (no re-mapping of the chunk buffer on every call).
-static int psf_pool(cudaMemPool_t* out) {
-    static std::mutex mu;
-    static std::map<int, cudaMemPool_t> pools;
-    int dev = 0;
-    DK_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = pools.find(dev);
-    if (it == pools.end()) {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool;
-        DK_CUDA(cudaMemPoolCreate(&pool, &props));
-        uint64_t keep = uint64_t(1) << 30;
-        DK_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-        it = pools.emplace(dev, pool).first;
-    }
-    *out = it->second;
-    return DECON_OK;
-}
-
-
 static PsfKernel pick(const Axis& ax, bool cols) {
     for (auto group : {psf_group_a, psf_group_b, psf_group_c, psf_group_d, psf_group_e}) {
         const PsfKernel k = group(ax.L, cols);
@@ -202,13 +149,13 @@ extern "C" int decon_pupil_to_psf(const float* pupil, const double* kz, const do
     const int64_t nyx = ny * nx;
     const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(nz, kPsfChunkVoxels / nyx));
     const float2 *twx = nullptr, *twy = nullptr;
-    DK_TRY(psf_twiddles((int)nx, &twx));
-    DK_TRY(psf_twiddles((int)ny, &twy));
+    DK_TRY(twiddle_table((int)nx, &twx));
+    DK_TRY(twiddle_table((int)ny, &twy));
     axx.tw = twx;
     axy.tw = twy;
     axx.tws = axy.tws = 1;
     cudaMemPool_t pool;
-    DK_TRY(psf_pool(&pool));
+    DK_TRY(device_pool(&pool));
     // scratch: complex chunk, then energy, partials, and the column lists
     const int nparts = (int)cdiv(nx, 32);
     const size_t chunk_bytes = (size_t)round_up(chunk * nyx * (int64_t)sizeof(float2), 256);

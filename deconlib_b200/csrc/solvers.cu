@@ -614,20 +614,19 @@ int decon_pdhg_create(int num_iter, double step_scale, double delta, double eta,
     const int nh = std::max(num_iter, 1);
     h->capacity = nh;
     const size_t bytes = sizeof(PdhgDev) + (size_t)(4 * nh + kPdhgSlots * kPdhgGrid) * sizeof(double);
-    cudaError_t e = cudaMalloc(&h->mem, bytes);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
+    int st = pool_alloc(&h->mem, bytes, "the PDHG state");
+    if (st != DECON_OK) {
         delete h;
-        return fail(DECON_ERR_OOM, "cudaMalloc of PDHG state failed: %s", cudaGetErrorString(e));
+        return st;
     }
     double* base = reinterpret_cast<double*>(reinterpret_cast<char*>(h->mem) + sizeof(PdhgDev));
     const PdhgDev d = pdhg_initial(num_iter, step_scale, delta, eta, tol, min_iter, patience, base, nh);
     h->dev = reinterpret_cast<PdhgDev*>(h->mem);
     // complete before the call returns: the solve may run on any stream
-    int st = upload_blocking(h->dev, &d, sizeof(d));
+    st = upload_blocking(h->dev, &d, sizeof(d));
     if (st == DECON_OK) st = memset_blocking(base, 0, (size_t)(4 * nh + kPdhgSlots * kPdhgGrid) * sizeof(double));
     if (st != DECON_OK) {
-        cudaFree(h->mem);
+        pool_free({h->mem});
         delete h;
         return st;
     }
@@ -655,7 +654,7 @@ int decon_pdhg_reset(decon_pdhg* h, int num_iter, double step_scale, double delt
 
 int decon_pdhg_destroy(decon_pdhg* h) {
     if (!h) return DECON_OK;
-    cudaFree(h->mem);
+    pool_free({h->mem});
     delete h;
     return DECON_OK;
 }

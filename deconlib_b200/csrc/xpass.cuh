@@ -47,7 +47,7 @@ __device__ __forceinline__ float fetch_x(const XR2CArgs& a, const RowSrc& r, int
     if constexpr (PRO == PRO_KERNEL) {
         int64_t kx;
         if (!kernel_src(x, a.Nx, a.Kx, a.px, kx)) return 0.f;
-        return __ldg(r.p + kx) / a.kdiv;
+        return __ldg(r.p + kx) / (a.ksum ? (float)__ldg(a.ksum) : 1.f);
     } else {
         const int64_t ix = x - a.win.ox;
         if (ix < 0 || ix >= a.win.wx) return 0.f;

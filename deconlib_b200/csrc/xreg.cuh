@@ -62,10 +62,10 @@ __device__ __forceinline__ const float* embedded_row(const XRegArgs& a, int64_t 
     if (!kernel_src(z, a.Nz, a.Kz, a.pz, kz) || !kernel_src(y, a.Ny, a.Ky, a.py, ky)) return nullptr;
     return a.in + (kz * a.Ky + ky) * a.Kx;
 }
-__device__ __forceinline__ float embedded(const XRegArgs& a, const float* p, int x) {
+__device__ __forceinline__ float embedded(const XRegArgs& a, const float* p, int x, float sum) {
     int64_t kx;
     if (p == nullptr || x >= a.Nx || !kernel_src(x, a.Nx, a.Kx, a.px, kx)) return 0.f;
-    return __ldg(p + kx) / a.kdiv;
+    return __ldg(p + kx) / sum;
 }
 
 // The solver's prologue on an array value: as it is, or max(y - b, 1e-6)
@@ -102,10 +102,11 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
                 for (int k = tid; k < a.Hx; k += NT) a.out[(row0 + i) * a.P + k] = make_float2(0.f, 0.f);
             return;
         }
+        const float sum = a.ksum ? (float)__ldg(a.ksum) : 1.f;
         for (int q = tid; q < TL * L; q += NT) {
             const int l = q / L, n = q - l * L;
-            stg[q] = ODD ? make_float2(embedded(a, rows[2 * l], n), embedded(a, rows[2 * l + 1], n))
-                         : make_float2(embedded(a, rows[l], 2 * n), embedded(a, rows[l], 2 * n + 1));
+            stg[q] = ODD ? make_float2(embedded(a, rows[2 * l], n, sum), embedded(a, rows[2 * l + 1], n, sum))
+                         : make_float2(embedded(a, rows[l], 2 * n, sum), embedded(a, rows[l], 2 * n + 1, sum));
         }
         __syncthreads();
     }
