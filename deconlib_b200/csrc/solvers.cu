@@ -16,6 +16,7 @@
 #include "solvers.cuh"
 #include "stencil.cuh"
 #include "pdhg_tiled.cuh"
+#include "hess_wide.cuh"
 
 namespace dk {
 
@@ -573,6 +574,44 @@ static int smem_prepare(const void* fn, size_t bytes, int* per_sm) {
     return DECON_OK;
 }
 
+// The wide stencil walk for these rows, or grid 0: rows must be 16-byte aligned
+// and fill at least 60 % of their 128-voxel pieces (below that the one-voxel
+// walk keeps more lanes busy).
+struct WidePlan {
+    WideGeo g{};
+    int grid = 0;
+};
+static WidePlan wide_plan(const Dims& d, std::initializer_list<const void*> ptrs) {
+    WidePlan p;
+    const int64_t lim = INT32_MAX / 2;
+    if (d.nx % 4 != 0 || 10 * d.nx < 6 * kWideX * cdiv(d.nx, kWideX) || d.nx > lim || d.ny > lim || d.nz > lim)
+        return p;
+    for (const void* q : ptrs)
+        if (reinterpret_cast<uintptr_t>(q) & 15) return p;
+    WideGeo& g = p.g;
+    g.nz = (int)d.nz;
+    g.ny = (int)d.ny;
+    g.nx = (int)d.nx;
+    g.n = d.nz * d.ny * d.nx;
+    g.ntx = (int)cdiv(d.nx, kWideX);
+    g.nty = (int)cdiv(d.ny, kWideRows);
+    // planes per tile: whole waves of two CTAs per SM against the planes that
+    // each tile reads beyond its own
+    const int64_t slots = std::min<int64_t>((int64_t)sm_count() * 2, kPdhgGrid);
+    double best = 0.0;
+    for (int64_t ntz = 1; ntz <= std::max<int64_t>(1, d.nz / 4); ++ntz) {
+        const int64_t zc = cdiv(d.nz, ntz), tiles = (int64_t)g.ntx * g.nty * cdiv(d.nz, zc);
+        const double cost = (double)cdiv(tiles, slots) * ((double)zc + 2.5);
+        if (ntz == 1 || cost < best * 0.999) {
+            best = cost;
+            g.zc = (int)zc;
+        }
+    }
+    g.ntiles = (int64_t)g.ntx * g.nty * cdiv(d.nz, g.zc);
+    p.grid = (int)std::min<int64_t>(g.ntiles, slots);
+    return p;
+}
+
 static int g1(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 256), (int64_t)sm_count() * 16));
 }
@@ -751,8 +790,16 @@ int decon_pdhg_hess_dual(decon_pdhg* h, float* y2, const float* xc, const float*
     W6 w;
     hessian_weights(r, w.w);
     const Dims d{shape[0], shape[1], shape[2]};
-    const int64_t n = d.nz * d.ny * d.nx;
-    (void)n;
+    const WidePlan wp = wide_plan(d, {xc, xp, y2});
+    if (wp.grid) {
+        // n % 4 == 0, so the six components are aligned as their base is
+        if (norm == 0)
+            DK_TRY(chain(k_wide_dual<0>, wp.grid, kWideThreads, 0, as_stream(stream), h->dev, y2, xc, xp, wp.g, w, alpha));
+        else
+            DK_TRY(chain(k_wide_dual<1>, wp.grid, kWideThreads, 0, as_stream(stream), h->dev, y2, xc, xp, wp.g, w, alpha));
+        DK_LAUNCHED();
+        return DECON_OK;
+    }
     const TileGeo tg(d);
     int per_sm = 1;
     const void* fn = norm == 0 ? (const void*)k_hess_dual_p<0> : (const void*)k_hess_dual_p<1>;
@@ -812,6 +859,13 @@ int decon_pdhg_hess_dk(decon_pdhg* h, const float* ax_new, const float* ax_cur, 
     hessian_weights(r, w.w);
     int per_sm = 1;
     const Dims d{shape[0], shape[1], shape[2]};
+    const WidePlan wp = wide_plan(d, {xn, xc});
+    if (wp.grid) {
+        DK_TRY(chain(k_wide_dk, wp.grid, kWideThreads, 0, as_stream(stream), h->dev, ax_new, ax_cur, ax_new ? m : 0, xn, xc,
+                     wp.g, w, ax_new ? kSlotDA2 : kPdhgSlots - 1, kSlotDL2));
+        DK_LAUNCHED();
+        return DECON_OK;
+    }
     const bool u32 = offsets_fit_u32(d);
     DK_TRY(smem_prepare(u32 ? (const void*)k_hess_dk_r<uint32_t> : (const void*)k_hess_dk_r<int64_t>, 0, &per_sm));
     const int grid = (int)std::min<int64_t>(kPdhgGrid, std::max<int64_t>(TileGeo(d).ntiles, 1));
