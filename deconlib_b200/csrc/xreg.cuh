@@ -68,12 +68,6 @@ __device__ __forceinline__ float embedded(const XRegArgs& a, const float* p, int
     return __ldg(p + kx) / sum;
 }
 
-// The solver's prologue on an array value: as it is, or max(y - b, 1e-6)
-// (rl_mlx.py:123-125).
-__device__ __forceinline__ float array_value(const XRegArgs& a, float v) {
-    return a.pro == PRO_RLINIT ? fmaxf(v - a.bg, 1e-6f) : v;
-}
-
 template <int L, bool ODD, int SRC>
 __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::blocks_for(4 * XRegShape<L, ODD>::S + 44))
     k_xreg_r2c(const XRegArgs a) {
@@ -139,33 +133,40 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
                 const int n = j + r * S;
                 v[r] = C1{n < lim || (half && n == lim) ? a.cval : 0.f, n < lim && two ? a.cval : 0.f};
             }
-        } else if constexpr (ODD) {
-            const float* p = a.in + (int64_t)line * 2 * a.Nx;
-            const int lim = 2 * line < a.nrows ? a.nin : 0, lim2 = 2 * line + 1 < a.nrows ? a.nin : 0;
-#pragma unroll
-            for (int r = 0; r < B; ++r) {
-                const int n = j + r * S;
-                v[r] = C1{n < lim ? array_value(a, __ldg(p + n)) : 0.f,
-                          n < lim2 ? array_value(a, __ldg(p + a.Nx + n)) : 0.f};
-            }
-        } else if (a.vec) {
-            const float2* p = reinterpret_cast<const float2*>(a.in + (int64_t)line * a.Nx);
-            const int lim = line < a.nrows ? a.nin : 0;
-#pragma unroll
-            for (int r = 0; r < B; ++r) v[r] = j + r * S < lim ? as_c1(__ldg(p + j + r * S)) : C1{0.f, 0.f};
-            if (a.pro == PRO_RLINIT) {
-#pragma unroll
-                for (int r = 0; r < B; ++r)
-                    if (j + r * S < lim) v[r] = C1{array_value(a, v[r].re), array_value(a, v[r].im)};
-            }
         } else {
-            const float* p = a.in + (int64_t)line * a.Nx;
-            const int lim = line < a.nrows ? (int)a.Nx : 0;
+            int lim, lim2;  // points with a value in the real and the imaginary part
+            if constexpr (ODD) {
+                const float* p = a.in + (int64_t)line * 2 * a.Nx;
+                lim = 2 * line < a.nrows ? a.nin : 0;
+                lim2 = 2 * line + 1 < a.nrows ? a.nin : 0;
 #pragma unroll
-            for (int r = 0; r < B; ++r) {
-                const int x = 2 * (j + r * S);
-                v[r] = C1{x < lim ? array_value(a, __ldg(p + x)) : 0.f,
-                          x + 1 < lim ? array_value(a, __ldg(p + x + 1)) : 0.f};
+                for (int r = 0; r < B; ++r) {
+                    const int n = j + r * S;
+                    v[r] = C1{n < lim ? __ldg(p + n) : 0.f, n < lim2 ? __ldg(p + a.Nx + n) : 0.f};
+                }
+            } else if (a.vec) {
+                const float2* p = reinterpret_cast<const float2*>(a.in + (int64_t)line * a.Nx);
+                lim = lim2 = line < a.nrows ? a.nin : 0;
+#pragma unroll
+                for (int r = 0; r < B; ++r) v[r] = j + r * S < lim ? as_c1(__ldg(p + j + r * S)) : C1{0.f, 0.f};
+            } else {
+                const float* p = a.in + (int64_t)line * a.Nx;
+                lim = line < a.nrows ? a.nin : 0;
+                lim2 = line < a.nrows ? (int)(a.Nx >> 1) : 0;
+#pragma unroll
+                for (int r = 0; r < B; ++r) {
+                    const int n = j + r * S;
+                    v[r] = C1{n < lim ? __ldg(p + 2 * n) : 0.f, n < lim2 ? __ldg(p + 2 * n + 1) : 0.f};
+                }
+            }
+            if (a.pro == PRO_RLINIT) {
+                // max(y - b, 1e-6) (rl_mlx.py:123-125), after all loads are out
+#pragma unroll
+                for (int r = 0; r < B; ++r) {
+                    const int n = j + r * S;
+                    v[r] = C1{n < lim ? fmaxf(v[r].re - a.bg, 1e-6f) : 0.f,
+                              n < lim2 ? fmaxf(v[r].im - a.bg, 1e-6f) : 0.f};
+                }
             }
         }
         dftn<B, -1>(v);
