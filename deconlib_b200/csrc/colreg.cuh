@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
         mbar_expect_tx(&obar, (uint32_t)(a.onbox * a.obox * row));
         for (int i = 0; i < a.onbox; ++i) {
             const int r0 = i * a.obox;
-            tma_load_3d(ot + r0 * row, &a.otfmap, c0 * cs, o, r0, &obar);
+            if (a.jdim == 1) tma_load_3d(ot + r0 * row, &a.otfmap, c0 * cs, r0, o, &obar);
+            else tma_load_3d(ot + r0 * row, &a.otfmap, c0 * cs, o, r0, &obar);
         }
     };
     if (tid == 0 && (int)blockIdx.x < a.nmain) {

@@ -191,8 +191,9 @@ struct ConvPlan {
     double norm_sq;
     int device;
     // Register column passes (ok when the axis length has one): Y forward
-    // S1 -> S2, axial in S2 (FP32 and FP16 OTF), Y inverse S2 -> S1
-    ColPass y_fwd, z_otf, z_otf16, y_inv;
+    // S1 -> S2, axial in S2 (FP32 and FP16 OTF), Y inverse S2 -> S1; one plane
+    // (Fz = 1, images): Y forward, product and Y inverse in one pass over S1
+    ColPass y_fwd, z_otf, z_otf16, y_inv, y_otf;
     bool reg_ok = false;
     // Mixed precision (decon_conv_set_precision): the OTF also stored as FP16
     // complex, scaled per kz plane by a power of two (OTF = otf16 * otf_inv[kz]),
