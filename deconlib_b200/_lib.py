@@ -130,6 +130,9 @@ _SIGS = {
                                   C.POINTER(C.c_int), C.POINTER(C.c_int), _dp, _dp, _dp, _dp,
                                   _dp, _p]),
     "decon_pdhg_set_stop": (C.c_int, [_p, C.c_int, _p]),
+    "decon_pdhg_first_dual": (C.c_int, [_p, C.c_int, _p, _p, _p, _i64p, C.c_float, C.c_float, C.c_int, _p]),
+    "decon_pdhg_first_primal": (C.c_int, [_p, C.c_int, _p, _p, _p, _p, _i64p, C.c_float, _p]),
+    "decon_pdhg_first_dk": (C.c_int, [_p, C.c_int, _p, _p, _i64, _p, _p, _i64p, C.c_float, _p]),
     "decon_pdhg_hess_dual": (C.c_int, [_p, _p, _p, _p, _i64p, C.c_float, C.c_float, C.c_int, _p]),
     "decon_pdhg_hess_primal": (C.c_int, [_p, _p, _p, _p, _p, _i64p, C.c_float, _p]),
     "decon_pdhg_hess_dual_primal": (C.c_int, [_p, _p, _p, _p, _p, _p, _p, _i64p, C.c_float,

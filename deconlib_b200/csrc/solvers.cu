@@ -17,6 +17,7 @@
 #include "stencil.cuh"
 #include "pdhg_tiled.cuh"
 #include "hess_wide.cuh"
+#include "pdhg_first.cuh"
 
 namespace dk {
 
@@ -612,6 +613,30 @@ static WidePlan wide_plan(const Dims& d, std::initializer_list<const void*> ptrs
     return p;
 }
 
+static bool first_geo(const int64_t shape[3], FirstGeo* g, int* grid) {
+    const int64_t lim = INT32_MAX / 2;
+    if (shape[0] < 1 || shape[1] < 1 || shape[2] < 1 || shape[0] > lim || shape[1] > lim || shape[2] > lim) return false;
+    g->nz = (int)shape[0];
+    g->ny = (int)shape[1];
+    g->nx = (int)shape[2];
+    g->n = shape[0] * shape[1] * shape[2];
+    g->ntx = (int)cdiv(g->nx, kFirstX);
+    g->nty = (int)cdiv(g->ny, kFirstY);
+    // planes per march: whole waves of the fixed grid (four CTAs of 512 threads
+    // per SM), a march costing about one plane to start
+    int64_t best = 0;
+    for (int64_t zc = 1; zc <= 16 && zc <= g->nz; ++zc) {
+        const int64_t tiles = (int64_t)g->ntx * g->nty * cdiv(g->nz, zc), cost = cdiv(tiles, kPdhgGrid) * (zc + 1);
+        if (zc == 1 || cost < best) {
+            best = cost;
+            g->zc = (int)zc;
+        }
+    }
+    g->ntiles = (int64_t)g->ntx * g->nty * cdiv(g->nz, g->zc);
+    *grid = (int)std::min<int64_t>(g->ntiles, kPdhgGrid);
+    return true;
+}
+
 static int g1(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 256), (int64_t)sm_count() * 16));
 }
@@ -780,6 +805,51 @@ int decon_pdhg_loss(decon_pdhg* h, const float* ax, const float* data, float bac
     else DK_TRY(chain(k_loss_reg<1>, kPdhgGrid, 256, 0, s, h->dev, lx, ncomp, n, k));
     DK_LAUNCHED();
     DK_TRY(chain(k_record_loss, 1, 256, 0, s, h->dev, alpha, k));
+    DK_LAUNCHED();
+    return DECON_OK;
+}
+
+int decon_pdhg_first_dual(decon_pdhg* h, int kind, float* y2, const float* xc, const float* xp,
+                          const int64_t shape[3], float r, float alpha, int norm, void* stream) {
+    if (!h || !y2 || !xc || !xp || !shape) return fail(DECON_ERR_NULL, "null pointer");
+    FirstGeo g;
+    int grid;
+    if (!first_geo(shape, &g, &grid)) return fail(DECON_ERR_VALUE, "decon_pdhg_first_dual: bad shape");
+    const cudaStream_t s = as_stream(stream);
+    if (kind == 0 && norm == 0) DK_TRY(chain(k_first_dual<0, 0>, grid, kFirstThreads, 0, s, h->dev, y2, xc, xp, g, r, alpha));
+    else if (kind == 0) DK_TRY(chain(k_first_dual<0, 1>, grid, kFirstThreads, 0, s, h->dev, y2, xc, xp, g, r, alpha));
+    else if (norm == 0) DK_TRY(chain(k_first_dual<1, 0>, grid, kFirstThreads, 0, s, h->dev, y2, xc, xp, g, r, alpha));
+    else DK_TRY(chain(k_first_dual<1, 1>, grid, kFirstThreads, 0, s, h->dev, y2, xc, xp, g, r, alpha));
+    DK_LAUNCHED();
+    return DECON_OK;
+}
+
+int decon_pdhg_first_primal(decon_pdhg* h, int kind, const float* xc, const float* aty, const float* y2, float* xn,
+                            const int64_t shape[3], float r, void* stream) {
+    if (!h || !xc || !aty || !y2 || !xn || !shape) return fail(DECON_ERR_NULL, "null pointer");
+    FirstGeo g;
+    int grid;
+    if (!first_geo(shape, &g, &grid)) return fail(DECON_ERR_VALUE, "decon_pdhg_first_primal: bad shape");
+    const cudaStream_t s = as_stream(stream);
+    if (kind == 0)
+        DK_TRY(chain(k_first_primal<0>, grid, kFirstThreads, 0, s, h->dev, xc, aty, y2, xn, g, r, kSlotDx2, kSlotXc2, kSlotXn2));
+    else
+        DK_TRY(chain(k_first_primal<1>, grid, kFirstThreads, 0, s, h->dev, xc, aty, y2, xn, g, r, kSlotDx2, kSlotXc2, kSlotXn2));
+    DK_LAUNCHED();
+    return DECON_OK;
+}
+
+int decon_pdhg_first_dk(decon_pdhg* h, int kind, const float* ax_new, const float* ax_cur, int64_t m, const float* xn,
+                        const float* xc, const int64_t shape[3], float r, void* stream) {
+    if (!h || !ax_new || !ax_cur || !xn || !xc || !shape) return fail(DECON_ERR_NULL, "null pointer");
+    FirstGeo g;
+    int grid;
+    if (!first_geo(shape, &g, &grid)) return fail(DECON_ERR_VALUE, "decon_pdhg_first_dk: bad shape");
+    const cudaStream_t s = as_stream(stream);
+    if (kind == 0)
+        DK_TRY(chain(k_first_dk<0>, grid, kFirstThreads, 0, s, h->dev, ax_new, ax_cur, m, xn, xc, g, r, kSlotDA2, kSlotDL2));
+    else
+        DK_TRY(chain(k_first_dk<1>, grid, kFirstThreads, 0, s, h->dev, ax_new, ax_cur, m, xn, xc, g, r, kSlotDA2, kSlotDL2));
     DK_LAUNCHED();
     return DECON_OK;
 }

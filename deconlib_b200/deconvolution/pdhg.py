@@ -27,7 +27,7 @@ import numpy as np
 import torch
 
 from .. import _lib
-from ._device import empty, fill, stream, to_device, zeros
+from ._device import empty, fill, shape3, stream, to_device, zeros
 from .base import MLXDeconvolutionResult
 from .composition import LinearOperator, compose
 from .core_operators import FractionalAreaDownsample
@@ -383,6 +383,16 @@ class PDHGRunner:
         # fused Hessian3D kernels (fused=False keeps the operator-by-operator path)
         self.fused = (fused and isinstance(reg, HessianRegularizer) and reg.ndim == 3
                       and x0.dim() == 3)
+        # identity and 3-D gradient: L evaluated on the fly (fused=False: through
+        # the operators)
+        self.first = None
+        if fused and type(reg) is IdentityRegularizer and x0.dim() <= 3:
+            self.first, self.r = 0, 1.0
+        elif fused and type(reg) is GradientRegularizer and reg.ndim == 3 and x0.dim() == 3:
+            self.first, self.r = 1, float(reg.r)
+        if self.first is not None:
+            self.shp = _lib.i64arr(shape3(x0.shape))
+            self.xbar = self.dxb = None
         self.side = None
         if self.fused:
             self.shp = _lib.i64arr(tuple(x0.shape))
@@ -463,6 +473,22 @@ class PDHGRunner:
                 _lib.call("decon_pdhg_hess_loss", h, _lib.ptr(axn), _lib.ptr(self.data),
                           C.c_float(self.bg), self.lcode, m, _lib.ptr(xn), shp, r, self.ncode,
                           C.c_double(self.alpha), k, s)
+        elif self.first is not None:
+            kind, shp, r = self.first, self.shp, C.c_float(self.r)
+            _lib.call("decon_pdhg_first_dual", h, kind, _lib.ptr(self.y2), _lib.ptr(xc), _lib.ptr(xp), shp, r,
+                      C.c_float(self.alpha), self.ncode, s)
+            _lib.call("decon_pdhg_first_primal", h, kind, _lib.ptr(xc), _lib.ptr(aty), _lib.ptr(self.y2),
+                      _lib.ptr(xo), shp, r, s)
+            xn = xo
+            axn = to_device(A.forward(xn))
+            _lib.call("decon_pdhg_first_dk", h, kind, _lib.ptr(axn), _lib.ptr(axc), m, _lib.ptr(xn), _lib.ptr(xc),
+                      shp, r, s)
+            _lib.call("decon_pdhg_step", h, s)
+            if do_loss:
+                lx = to_device(reg.forward(xn))
+                _lib.call("decon_pdhg_loss", h, _lib.ptr(axn), _lib.ptr(self.data),
+                          C.c_float(self.bg), self.lcode, m, _lib.ptr(lx), self.ncode, self.ncomp,
+                          n, C.c_double(self.alpha), k, s)
         else:
             _lib.call("decon_pdhg_xbar", h, _lib.ptr(xc), _lib.ptr(xp), _lib.ptr(self.xbar), n, s)
             lxb = to_device(reg.forward(self.xbar))

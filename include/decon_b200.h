@@ -375,6 +375,18 @@ int decon_pdhg_step(decon_pdhg* h, void* stream);
 int decon_pdhg_loss(decon_pdhg* h, const float* ax, const float* data, float background,
                     int loss_type, int64_t m, const float* lx, int norm, int ncomp, int64_t n,
                     double alpha, int k, void* stream);
+/* The regulariser half with L = identity (kind 0, y2 (1, n)) or the 3-D
+ * gradient (kind 1, y2 (3, z, y, x); pdhg_mlx.py:241-377), L evaluated on the
+ * fly: first_dual as decon_pdhg_dual_reg on L x_bar, first_primal as
+ * decon_pdhg_primal with L^T y2, first_dk as decon_pdhg_dk with L (x_new - x). */
+int decon_pdhg_first_dual(decon_pdhg* h, int kind, float* y2, const float* xc, const float* xp,
+                          const int64_t shape[3], float r, float alpha, int norm, void* stream);
+int decon_pdhg_first_primal(decon_pdhg* h, int kind, const float* xc, const float* aty,
+                            const float* y2, float* xn, const int64_t shape[3], float r,
+                            void* stream);
+int decon_pdhg_first_dk(decon_pdhg* h, int kind, const float* ax_new, const float* ax_cur, int64_t m,
+                        const float* xn, const float* xc, const int64_t shape[3], float r,
+                        void* stream);
 /* Fused Hessian3D forms of the regulariser half (L = Hessian3D(r), shape
  * (z, y, x)); the Hessian is evaluated on the fly, never stored:
  *   hess_dual:   y2 = proj(y2 + sigma H x_bar), x_bar = x + theta (x - x_prev)
