@@ -54,6 +54,8 @@ _SIGS = {
     "decon_conv_get_otf": (C.c_int, [_p, _p, _p]),
     "decon_conv_forward": (C.c_int, [_p, _p, _p, _p]),
     "decon_conv_adjoint": (C.c_int, [_p, _p, _p, _p]),
+    "decon_conv_forward_crop": (C.c_int, [_p, _p, _p, _i64p, _i64p, _p]),
+    "decon_conv_adjoint_crop": (C.c_int, [_p, _p, _p, _i64p, _i64p, _p]),
     "decon_conv_forward_down2": (C.c_int, [_p, _p, _p, _p]),
     "decon_conv_adjoint_up2": (C.c_int, [_p, _p, _p, _p]),
     "decon_rl_setup": (C.c_int, [_p, _p, C.c_float, _p, _p, _p, _p]),

@@ -570,6 +570,39 @@ int decon_conv_adjoint_up2(decon_conv* p, const float* y, float* x, void* stream
     return DECON_OK;
 }
 
+// compose(Crop, LinearFFTConvolver): the crop is a window of the X passes, so the
+// cropped-away rows are neither transformed back nor written, and the adjoint's
+// zero rows are not read.
+static int crop_window(const decon_conv* p, const int64_t start[3], const int64_t ext[3], Win3* w) {
+    for (int i = 0; i < 3; ++i)
+        if (start[i] < 0 || ext[i] < 1 || start[i] + ext[i] > p->N[i])
+            return fail(DECON_ERR_VALUE, "crop window outside the signal on axis %d", i);
+    *w = Win3{ext[0], ext[1], ext[2], start[0], start[1], start[2]};
+    return DECON_OK;
+}
+
+int decon_conv_forward_crop(decon_conv* p, const float* x, float* y, const int64_t start[3],
+                            const int64_t ext[3], void* stream) {
+    if (!p || !x || !y || !start || !ext) return fail(DECON_ERR_NULL, "null pointer");
+    Win3 w;
+    DK_TRY(crop_window(p, start, ext, &w));
+    const cudaStream_t s = as_stream(stream);
+    DK_TRY(spectrum_forward(*p, PRO_ARRAY, x, full_window(p->N), 0.f, 0.f, s));
+    DK_TRY(spectrum_filter_back(*p, false, s));
+    return launch_xc2r(*p, EPI_STORE, p->s1, w, y, nullptr, nullptr, 0.f, nullptr, nullptr, s);
+}
+
+int decon_conv_adjoint_crop(decon_conv* p, const float* y, float* x, const int64_t start[3],
+                            const int64_t ext[3], void* stream) {
+    if (!p || !x || !y || !start || !ext) return fail(DECON_ERR_NULL, "null pointer");
+    Win3 w;
+    DK_TRY(crop_window(p, start, ext, &w));
+    const cudaStream_t s = as_stream(stream);
+    DK_TRY(spectrum_forward(*p, PRO_ARRAY, y, w, 0.f, 0.f, s));
+    DK_TRY(spectrum_filter_back(*p, true, s));
+    return launch_xc2r(*p, EPI_STORE, p->s1, full_window(p->N), x, nullptr, nullptr, 0.f, nullptr, nullptr, s);
+}
+
 int decon_conv_adjoint(decon_conv* p, const float* y, float* x, void* stream) {
     if (!p || !x || !y) return fail(DECON_ERR_NULL, "null pointer");
     const cudaStream_t s = as_stream(stream);

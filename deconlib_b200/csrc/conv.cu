@@ -265,8 +265,15 @@ static bool is_full_window(const ConvPlan& p, const Win3& w) {
 static bool pair_aligned(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0; }
 
 // The fields both register X passes share.
-static XRegArgs xreg_args(const ConvPlan& p, int64_t nrows, int64_t Ny, int64_t Nx) {
+static XRegArgs xreg_args(const ConvPlan& p, int64_t nrows, int64_t Ny, int64_t Nx, const Win3& w, bool full) {
     XRegArgs a{};
+    a.win = full ? 0 : 1;
+    a.z0 = full ? 0 : (int)w.oz;
+    a.y0 = full ? 0 : (int)w.oy;
+    a.x0 = full ? 0 : (int)w.ox;
+    a.wz = full ? (int)(nrows / Ny) : (int)w.wz;
+    a.wy = full ? (int)Ny : (int)w.wy;
+    a.wx = full ? (int)Nx : (int)w.wx;
     const int L = p.ax_x.L;
     a.Ny = Ny;
     a.Nx = Nx;
@@ -284,12 +291,12 @@ static XRegArgs xreg_args(const ConvPlan& p, int64_t nrows, int64_t Ny, int64_t 
 int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cval, float bg,
                 int64_t nz_rows, float2* out, cudaStream_t st, int64_t kstride) {
     const int src = pro == PRO_KERNEL ? 2 : pro == PRO_UP2 ? 1 : 0;
-    const XRegKernel k = p.reg_ok && kstride == 0 && (pro == PRO_KERNEL || pro == PRO_UP2 || is_full_window(p, win))
-                             ? pick_xreg_r2c(p.ax_x.L, p.odd, src)
-                             : XRegKernel{};
+    const bool full = pro == PRO_KERNEL || pro == PRO_UP2 || is_full_window(p, win);
+    const XRegKernel k = p.reg_ok && kstride == 0 && (full || pro == PRO_ARRAY) ? pick_xreg_r2c(p.ax_x.L, p.odd, src)
+                                                                                : XRegKernel{};
     if (k.fn) {
         const int64_t Ny = pro == PRO_KERNEL ? p.F[1] : p.N[1], Nx = pro == PRO_KERNEL ? p.F[2] : p.N[2];
-        XRegArgs a = xreg_args(p, nz_rows * Ny, Ny, Nx);
+        XRegArgs a = xreg_args(p, nz_rows * Ny, Ny, Nx, win, full);
         a.pro = pro;
         a.in = in;
         a.cval = cval;
@@ -303,7 +310,7 @@ int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cva
         a.py = (p.K[1] + 1) / 2;
         a.px = (p.K[2] + 1) / 2;
         a.out = out;
-        a.vec = Nx % 2 == 0 && pair_aligned(in);
+        a.vec = a.wx % 2 == 0 && a.x0 % 2 == 0 && pair_aligned(in);
         return launch(k.fn, cdiv(a.nlines, k.TL), k.nt, k.smem, st, &a, PROF_XR2C);
     }
     XR2CArgs a{};
@@ -382,13 +389,16 @@ int launch_col(const ConvPlan& p, const Axis& ax, int T, int mode, const float2*
 int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* out,
                 const float* aux0, const float* aux1, float bg, double* partials, int* nblk_out,
                 cudaStream_t st) {
-    const XRegKernel k = p.reg_ok && !use_yz(p) && is_full_window(p, win)
-                             ? pick_xreg_c2r(p.ax_x.L, p.odd, epi)
-                             : XRegKernel{};
+    const bool full = is_full_window(p, win);
+    const XRegKernel k = p.reg_ok && !use_yz(p) && (full || epi == EPI_STORE) ? pick_xreg_c2r(p.ax_x.L, p.odd, epi)
+                                                                              : XRegKernel{};
     if (k.fn) {
         if (epi == EPI_DOWN2 && (p.odd || (p.N[0] | p.N[1] | p.N[2]) & 1))
             return fail(DECON_ERR_UNSUPPORTED, "2x area-sum epilogue: extents must be even");
-        XRegArgs a = xreg_args(p, p.N[0] * p.N[1], p.N[1], p.N[2]);
+        // odd Fx: rows are transformed in the pairs of the whole field, so that a
+        // window has its bits; pairs outside are skipped
+        const int64_t rows = full || p.odd ? p.N[0] * p.N[1] : win.wz * win.wy;
+        XRegArgs a = xreg_args(p, rows, p.N[1], p.N[2], win, full);
         a.spec = in;
         a.out_real = out;
         a.aux0 = aux0;
@@ -397,7 +407,7 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
         a.pred = epi == EPI_PRED;
         a.partials = partials;
         a.scale = (float)(1.0 / ((double)p.F[0] * (double)p.F[1] * (double)p.F[2]));
-        a.vec = p.N[2] % 2 == 0 && pair_aligned(out) && pair_aligned(aux0) && pair_aligned(aux1);
+        a.vec = a.wx % 2 == 0 && a.x0 % 2 == 0 && pair_aligned(out) && pair_aligned(aux0) && pair_aligned(aux1);
         const int64_t nblk = cdiv(a.nlines, k.TL);
         if (nblk_out) *nblk_out = (int)nblk;
         return launch(k.fn, nblk, k.nt, k.smem, st, &a, PROF_XC2R);

@@ -139,7 +139,10 @@ struct XRegArgs {
     int pred;              // EPI_RL_RATIO kernel: store the model, not the ratio
     float scale;
     int64_t P;
-    uint32_t nrows, nlines;  // rows of the volume; lines (rows, or pairs of rows for odd Fx)
+    // the real array is the box (wz, wy, wx) at (z0, y0, x0) of the volume; win: a
+    // box smaller than the volume (R2C: zero outside; C2R: nothing else is kept)
+    int win, z0, y0, x0, wz, wy, wx;
+    uint32_t nrows, nlines;  // rows of the volume (C2R: of the box); lines (rows, or pairs for odd Fx)
     int nin, nout;           // points of a line that can be non-zero / are kept
     int Hx;                  // spectrum points of a row
     int vec;                 // rows are 8-byte aligned pairs

@@ -68,6 +68,26 @@ __device__ __forceinline__ float embedded(const XRegArgs& a, const float* p, int
     return __ldg(p + kx) / sum;
 }
 
+// Spectrum rows row0 .. row0 + ROWS of zero lines.
+template <int ROWS, int NT>
+__device__ __forceinline__ void zero_rows(const XRegArgs& a, int64_t row0) {
+    const int n = (int)(row0 + ROWS < a.nrows ? ROWS : (int64_t)a.nrows - row0);
+    for (int i = 0; i < n; ++i)
+        for (int k = threadIdx.x; k < a.Hx; k += NT) a.out[(row0 + i) * a.P + k] = make_float2(0.f, 0.f);
+}
+
+// Offset of x = 0 of a row in the real array (its window of the volume: elements
+// x0 .. x0 + wx of the row exist), or kNoRow outside of it.
+constexpr int64_t kNoRow = INT64_MIN;
+__device__ __forceinline__ int64_t array_row(const XRegArgs& a, uint32_t row) {
+    if (row >= a.nrows) return kNoRow;
+    if (!a.win) return (int64_t)row * a.Nx;
+    const uint32_t z = row / (uint32_t)a.Ny, y = row - z * (uint32_t)a.Ny;
+    const uint32_t iz = z - (uint32_t)a.z0, iy = y - (uint32_t)a.y0;
+    if (iz >= (uint32_t)a.wz || iy >= (uint32_t)a.wy) return kNoRow;
+    return (int64_t)(iz * (uint32_t)a.wy + iy) * a.wx - a.x0;
+}
+
 template <int L, bool ODD, int SRC>
 __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::blocks_for(4 * XRegShape<L, ODD>::S + 44))
     k_xreg_r2c(const XRegArgs a) {
@@ -90,10 +110,7 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
         if (!__syncthreads_or(any)) {
             // the kernel covers a part of the canvas: whole CTAs of zero rows
             // (three quarters of them for a kernel of half the canvas)
-            const int64_t row0 = (int64_t)W * line0;
-            const int n = (int)(row0 + W * TL < a.nrows ? W * TL : (int64_t)a.nrows - row0);
-            for (int i = 0; i < n; ++i)
-                for (int k = tid; k < a.Hx; k += NT) a.out[(row0 + i) * a.P + k] = make_float2(0.f, 0.f);
+            zero_rows<W * TL, NT>(a, (int64_t)W * line0);
             return;
         }
         const float sum = a.ksum ? (float)__ldg(a.ksum) : 1.f;
@@ -103,6 +120,18 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
                          : make_float2(embedded(a, rows[l], 2 * n, sum), embedded(a, rows[l], 2 * n + 1, sum));
         }
         __syncthreads();
+    }
+
+    if constexpr (SRC == XS_ARRAY) {
+        if (a.win) {
+            constexpr int W = ODD ? 2 : 1;
+            bool any = false;
+            for (int i = tid; i < W * TL; i += NT) any = any || array_row(a, W * line0 + i) != kNoRow;
+            if (!__syncthreads_or(any)) {
+                zero_rows<W * TL, NT>(a, (int64_t)W * line0);
+                return;
+            }
+        }
     }
 
     // stage 1
@@ -134,38 +163,38 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
                 v[r] = C1{n < lim || (half && n == lim) ? a.cval : 0.f, n < lim && two ? a.cval : 0.f};
             }
         } else {
-            int lim, lim2;  // points with a value in the real and the imaginary part
+            // real part: row pa (odd Fx: the first row of the pair), imaginary part: pb
+            const int64_t oa = array_row(a, ODD ? 2 * line : line);
+            const int64_t ob = ODD ? array_row(a, 2 * line + 1) : oa;
+            const float *pa = a.in + (oa == kNoRow ? 0 : oa), *pb = a.in + (ob == kNoRow ? 0 : ob);
+            const uint32_t wa = oa == kNoRow ? 0 : a.wx, wb = ob == kNoRow ? 0 : a.wx;
+            auto has = [&](uint32_t w, int x) { return (uint32_t)(x - a.x0) < w; };
             if constexpr (ODD) {
-                const float* p = a.in + (int64_t)line * 2 * a.Nx;
-                lim = 2 * line < a.nrows ? a.nin : 0;
-                lim2 = 2 * line + 1 < a.nrows ? a.nin : 0;
 #pragma unroll
                 for (int r = 0; r < B; ++r) {
                     const int n = j + r * S;
-                    v[r] = C1{n < lim ? __ldg(p + n) : 0.f, n < lim2 ? __ldg(p + a.Nx + n) : 0.f};
+                    v[r] = C1{has(wa, n) ? __ldg(pa + n) : 0.f, has(wb, n) ? __ldg(pb + n) : 0.f};
                 }
             } else if (a.vec) {
-                const float2* p = reinterpret_cast<const float2*>(a.in + (int64_t)line * a.Nx);
-                lim = lim2 = line < a.nrows ? a.nin : 0;
-#pragma unroll
-                for (int r = 0; r < B; ++r) v[r] = j + r * S < lim ? as_c1(__ldg(p + j + r * S)) : C1{0.f, 0.f};
-            } else {
-                const float* p = a.in + (int64_t)line * a.Nx;
-                lim = line < a.nrows ? a.nin : 0;
-                lim2 = line < a.nrows ? (int)(a.Nx >> 1) : 0;
 #pragma unroll
                 for (int r = 0; r < B; ++r) {
-                    const int n = j + r * S;
-                    v[r] = C1{n < lim ? __ldg(p + 2 * n) : 0.f, n < lim2 ? __ldg(p + 2 * n + 1) : 0.f};
+                    const int x = 2 * (j + r * S);
+                    v[r] = has(wa, x) ? as_c1(__ldg(reinterpret_cast<const float2*>(pa + x))) : C1{0.f, 0.f};
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < B; ++r) {
+                    const int x = 2 * (j + r * S);
+                    v[r] = C1{has(wa, x) ? __ldg(pa + x) : 0.f, has(wa, x + 1) ? __ldg(pa + x + 1) : 0.f};
                 }
             }
             if (a.pro == PRO_RLINIT) {
                 // max(y - b, 1e-6) (rl_mlx.py:123-125), after all loads are out
 #pragma unroll
                 for (int r = 0; r < B; ++r) {
-                    const int n = j + r * S;
-                    v[r] = C1{n < lim ? fmaxf(v[r].re - a.bg, 1e-6f) : 0.f,
-                              n < lim2 ? fmaxf(v[r].im - a.bg, 1e-6f) : 0.f};
+                    const int x = ODD ? j + r * S : 2 * (j + r * S);
+                    v[r] = C1{has(wa, x) ? fmaxf(v[r].re - a.bg, 1e-6f) : 0.f,
+                              has(wb, ODD ? x : x + 1) ? fmaxf(v[r].im - a.bg, 1e-6f) : 0.f};
                 }
             }
         }
@@ -303,16 +332,21 @@ __device__ __forceinline__ void x_store(const XRegArgs& a, int64_t i, int step, 
     }
 }
 
-// Spectrum row of line l: consecutive rows, or, for the 2x area sum, the four
-// rows of one 2 x 2 (z, y) block in lines 4q .. 4q + 3.
+// Spectrum row of output row `row`: the same, a row of the output's window, or,
+// for the 2x area sum, the four rows of one 2 x 2 (z, y) block in lines 4q ..
+// 4q + 3.
 template <int EPI>
-__device__ __forceinline__ uint32_t c2r_line(const XRegArgs& a, uint32_t line) {
+__device__ __forceinline__ uint32_t c2r_row(const XRegArgs& a, uint32_t row) {
     if constexpr (EPI == EPI_DOWN2) {
-        const uint32_t q = line >> 2, my = (uint32_t)a.Ny >> 1;
+        const uint32_t q = row >> 2, my = (uint32_t)a.Ny >> 1;
         const uint32_t k = q / my, y = q - k * my;
-        return (2 * k + (line & 1)) * (uint32_t)a.Ny + 2 * y + ((line >> 1) & 1);
+        return (2 * k + (row & 1)) * (uint32_t)a.Ny + 2 * y + ((row >> 1) & 1);
+    } else if constexpr (EPI == EPI_STORE) {
+        if (!a.win) return row;
+        const uint32_t z = row / (uint32_t)a.wy, y = row - z * (uint32_t)a.wy;
+        return (z + (uint32_t)a.z0) * (uint32_t)a.Ny + y + (uint32_t)a.y0;
     } else {
-        return line;
+        return row;
     }
 }
 
@@ -330,6 +364,14 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
     const uint32_t line0 = blockIdx.x * TL;
     chain_enter();
 
+    if constexpr (ODD && EPI == EPI_STORE) {
+        if (a.win) {  // pairs of rows outside the window
+            bool any = false;
+            for (int i = tid; i < 2 * TL; i += NT) any = any || array_row(a, 2 * line0 + i) != kNoRow;
+            if (!__syncthreads_or(any)) return;
+        }
+    }
+
     // stage 1
     {
         const int l = tid / TPL, u = tid - l * TPL;
@@ -339,7 +381,7 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
             if constexpr (!ODD) {
                 // Z[k] = e + i d W^-k, Z[M-k] = conj(e) + i conj(d W^-k) with e = X[k] +
                 // conj X[M-k], d = X[k] - conj X[M-k]; irfft ignores Im of DC and Nyquist
-                const float2* in = a.spec + (int64_t)c2r_line<EPI>(a, line) * a.P;
+                const float2* in = a.spec + (int64_t)c2r_row<EPI>(a, line) * a.P;
 #pragma unroll
                 for (int r = 0; r < S; ++r) {
                     va[r] = as_c1(__ldg(in + u + r * B));
@@ -454,23 +496,22 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
             if (line >= a.nlines) continue;
             C1 v[B];
             transform(l, j, v);
-            const int nout = a.nout;
+            // elements x0 .. x0 + wx of a row are kept (all of them but for a window)
+            auto kept = [&](int x) { return (uint32_t)(x - a.x0) < (uint32_t)a.wx; };
             if constexpr (ODD) {
-                const int64_t i = (int64_t)line * 2 * a.Nx + j;
-                auto in_row = [&](int r) { return j + r * S < nout; };
-                x_store<EPI, float, B>(a, i, S, acc, in_row, [&](int r) { return v[r].re * s; });
-                if (2 * line + 1 < a.nrows)
-                    x_store<EPI, float, B>(a, i + a.Nx, S, acc, in_row, [&](int r) { return v[r].im * s; });
+                const int64_t o0 = array_row(a, 2 * line), o1 = array_row(a, 2 * line + 1);
+                auto in_row = [&](int r) { return kept(j + r * S); };
+                if (o0 != kNoRow) x_store<EPI, float, B>(a, o0 + j, S, acc, in_row, [&](int r) { return v[r].re * s; });
+                if (o1 != kNoRow) x_store<EPI, float, B>(a, o1 + j, S, acc, in_row, [&](int r) { return v[r].im * s; });
             } else if (a.vec) {
-                x_store<EPI, float2, B>(a, (int64_t)line * a.Nx + 2 * j, 2 * S, acc,
-                                        [&](int r) { return j + r * S < nout; },
+                x_store<EPI, float2, B>(a, (int64_t)line * a.wx - a.x0 + 2 * j, 2 * S, acc,
+                                        [&](int r) { return kept(2 * (j + r * S)); },
                                         [&](int r) { return make_float2(v[r].re * s, v[r].im * s); });
             } else {
-                const int64_t i = (int64_t)line * a.Nx + 2 * j;
-                const int nx = (int)a.Nx;
-                x_store<EPI, float, B>(a, i, 2 * S, acc, [&](int r) { return 2 * (j + r * S) < nx; },
+                const int64_t i = (int64_t)line * a.wx - a.x0 + 2 * j;
+                x_store<EPI, float, B>(a, i, 2 * S, acc, [&](int r) { return kept(2 * (j + r * S)); },
                                        [&](int r) { return v[r].re * s; });
-                x_store<EPI, float, B>(a, i + 1, 2 * S, acc, [&](int r) { return 2 * (j + r * S) + 1 < nx; },
+                x_store<EPI, float, B>(a, i + 1, 2 * S, acc, [&](int r) { return kept(2 * (j + r * S) + 1); },
                                        [&](int r) { return v[r].im * s; });
             }
         }

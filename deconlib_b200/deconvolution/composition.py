@@ -62,7 +62,11 @@ class Compose:
         # for measurement)
         self._down2 = None if os.environ.get("DECON_NO_DOWN2") == "1" else _down2_plan(outer, inner)
 
+        self._crop = _crop_plan(outer, inner)
+
     def forward(self, x):
+        if self._crop is not None:
+            return self._cropped("decon_conv_forward_crop", x, self.inner.in_shape, self.outer.out_shape)
         if self._down2 is not None:
             y = self._fused("decon_conv_forward_down2", x, self._down2[1], self._down2[2])
             if y is not None:
@@ -70,11 +74,31 @@ class Compose:
         return self.outer.forward(self.inner.forward(x))
 
     def adjoint(self, y):
+        if self._crop is not None:
+            return self._cropped("decon_conv_adjoint_crop", y, self.outer.out_shape, self.inner.in_shape)
         if self._down2 is not None:
             x = self._fused("decon_conv_adjoint_up2", y, self._down2[2], self._down2[1])
             if x is not None:
                 return x
         return self.inner.adjoint(self.outer.adjoint(y))
+
+    def _cropped(self, name, x, in_shape, out_shape):
+        """Crop o LinearFFTConvolver with the crop as a window of the
+        convolution's first or last FFT pass: the values of the two operators
+        in turn, without the copy of the padded grid."""
+        from .. import _lib
+        from ._device import empty, stream, to_device
+
+        x = to_device(x)
+        if tuple(x.shape) != tuple(in_shape):
+            # the operators' own checks and messages
+            if name.endswith("forward_crop"):
+                return self.outer.forward(self.inner.forward(x))
+            return self.inner.adjoint(self.outer.adjoint(x))
+        out = empty(out_shape)
+        start, ext = self._crop
+        _lib.call(name, self.inner.plan, _lib.ptr(x), _lib.ptr(out), start, ext, stream())
+        return out
 
     def _fused(self, name, x, in_shape, out_shape):
         """The recognised composition FractionalAreaDownsample(2) o
@@ -98,6 +122,22 @@ class Compose:
 
     def __call__(self, x):
         return self.forward(x)
+
+
+def _crop_plan(outer, inner):
+    """(start, extents) of a Crop of a LinearFFTConvolver's whole output as
+    3-D int64 arrays, else None."""
+    from .. import _lib
+    from ._device import shape3
+    from .core_operators import Crop
+    from .linops import LinearFFTConvolver
+
+    if type(outer) is not Crop or type(inner) is not LinearFFTConvolver:
+        return None
+    if tuple(outer.in_shape) != tuple(inner.out_shape) or 0 in outer.out_shape:
+        return None
+    start = (0,) * (3 - len(outer.start)) + tuple(outer.start)
+    return _lib.i64arr(start), _lib.i64arr(shape3(outer.out_shape))
 
 
 def _down2_plan(outer, inner):

@@ -141,6 +141,13 @@ int decon_conv_forward(decon_conv* plan, const float* x, float* y, void* stream)
 /* LinearFFTConvolver.adjoint: correlation with conj(OTF)
  * (linops_mlx.py:526-530). */
 int decon_conv_adjoint(decon_conv* plan, const float* y, float* x, void* stream);
+/* compose(Crop, LinearFFTConvolver) and its adjoint (core_operators.py:62-137):
+ * the box of extents ext at start of the convolved signal, and the correlation of
+ * an array of that box that is zero outside it. */
+int decon_conv_forward_crop(decon_conv* plan, const float* x, float* y_box, const int64_t start[3],
+                            const int64_t ext[3], void* stream);
+int decon_conv_adjoint_crop(decon_conv* plan, const float* y_box, float* x, const int64_t start[3],
+                            const int64_t ext[3], void* stream);
 /* compose(FractionalAreaDownsample(2), LinearFFTConvolver) (composition.py:92-106
  * over core_operators.py:222-352 and linops_mlx.py:520-530) when the
  * downsample halves every axis exactly (n_large = 2 n_small): forward writes

@@ -142,3 +142,24 @@ def test_psf_lengths_and_support(shape):
         a = torch.stack([torch.fft.ifft2(pupil * torch.exp(2j * np.pi * kz * v)) for v in z])
         ref = a.real ** 2 + a.imag ** 2
         assert rel(p, ref / ref.sum()) < TOL
+
+
+@pytest.mark.parametrize("fft,ext", [((32, 64, 64), None), ((32, 64, 64), (3, 7, 10)), ((48, 375, 90), (11, 100, 31)),
+                                     ((20, 27, 405), (5, 3, 101)), ((64, 60, 225), (1, 1, 1)), ((15, 27, 28), (4, 9, 8)),
+                                     ((90, 128), (20, 33)), ((96,), (17,)), ((21, 36, 49), (6, 11, 13))])
+def test_crop_of_a_convolution_equals_the_operators_in_turn(D, fft, ext):
+    shape = tuple(half(f) for f in fft)
+    ext = ext or shape
+    g = torch.Generator(device="cuda").manual_seed(len(fft))
+    c = D.LinearFFTConvolver(torch.rand(tuple(f - n + 1 for n, f in zip(shape, fft)), generator=g, device="cuda"),
+                             shape, fft_shape=fft)
+    x = torch.rand(shape, generator=g, device="cuda")
+    y = torch.rand(ext, generator=g, device="cuda")
+    for starts in (None, tuple(0 for _ in ext), tuple(n - e for n, e in zip(shape, ext)),
+                   tuple(min(1, n - e) for n, e in zip(shape, ext))):
+        crop = D.Crop(shape, ext, start=starts)
+        A = D.compose(crop, c)
+        assert torch.equal(A.forward(x), crop.forward(c.forward(x)))
+        assert torch.equal(A.adjoint(y), c.adjoint(crop.adjoint(y)))
+    with pytest.raises(ValueError):
+        A.forward(y if ext != shape else x[..., :-1])
