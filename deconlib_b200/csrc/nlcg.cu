@@ -28,6 +28,7 @@
 #include <initializer_list>
 
 #include "conv_impl.cuh"
+#include "elementwise.cuh"
 #include "zwalk.cuh"
 
 namespace dk {
@@ -49,20 +50,31 @@ struct NlcgDev {
     unsigned ticket;
 };
 
-__device__ __forceinline__ int64_t gstride() { return (int64_t)gridDim.x * blockDim.x; }
-__device__ __forceinline__ int64_t gtid() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
-
 // Block sums of v[0..NS) into partials; the last CTA folds them (block order,
 // FP64) into out[0..NS) and re-arms the ticket.  Returns true in the last CTA.
 template <int NS>
 __device__ bool fold_last(double (&v)[NS], double* __restrict__ part, unsigned* ticket,
                           double* out) {
     __shared__ bool last;
+    // the block sums together: one barrier, then one warp per sum
+    __shared__ double red[NS][kNlThreads / 32];
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-        const double t = block_sum(v[s]);
-        if (threadIdx.x == 0) part[s * gridDim.x + blockIdx.x] = t;
+        double t = v[s];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if ((threadIdx.x & 31) == 0) red[s][threadIdx.x >> 5] = t;
     }
+    __syncthreads();
+    for (int s = threadIdx.x >> 5; s < NS; s += blockDim.x >> 5) {
+        const int lane = threadIdx.x & 31;
+        double t = lane < (int)(blockDim.x >> 5) ? red[s][lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) {
+            part[s * gridDim.x + blockIdx.x] = t;
+            __threadfence();
+        }
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
@@ -91,44 +103,6 @@ __device__ bool fold_last(double (&v)[NS], double* __restrict__ part, unsigned* 
     __syncthreads();
     if (threadIdx.x == 0) *ticket = 0;
     return true;
-}
-
-// Element-wise loop over n values of NI inputs and NO outputs: groups of four
-// with float4 loads and stores when `vec` (every pointer 16-byte aligned),
-// then the remainder one by one.  f(in[NI], out[NO]) handles one element;
-// a null input reads 0, a null output is not stored.
-template <int NI, int NO, class F>
-__device__ __forceinline__ void ew4(int64_t n, const float* const (&in)[NI], float* const (&out)[NO],
-                                    bool vec, F&& f) {
-    const int64_t ng = vec ? n / 4 : 0;
-    for (int64_t gi = gtid(); gi < ng; gi += gstride()) {
-        float4 a[NI];
-#pragma unroll
-        for (int k = 0; k < NI; ++k)
-            a[k] = in[k] ? __ldg(reinterpret_cast<const float4*>(in[k]) + gi) : make_float4(0.f, 0.f, 0.f, 0.f);
-        float o[NO][4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            float x[NI], y[NO];
-#pragma unroll
-            for (int k = 0; k < NI; ++k) x[k] = e == 0 ? a[k].x : e == 1 ? a[k].y : e == 2 ? a[k].z : a[k].w;
-            f(x, y);
-#pragma unroll
-            for (int k = 0; k < NO; ++k) o[k][e] = y[k];
-        }
-#pragma unroll
-        for (int k = 0; k < NO; ++k)
-            if (out[k]) reinterpret_cast<float4*>(out[k])[gi] = make_float4(o[k][0], o[k][1], o[k][2], o[k][3]);
-    }
-    for (int64_t i = 4 * ng + gtid(); i < n; i += gstride()) {
-        float x[NI], y[NO];
-#pragma unroll
-        for (int k = 0; k < NI; ++k) x[k] = in[k] ? in[k][i] : 0.f;
-        f(x, y);
-#pragma unroll
-        for (int k = 0; k < NO; ++k)
-            if (out[k]) out[k][i] = y[k];
-    }
 }
 
 // f0 = max(x, 1e-6), s = sqrt(f0), f = s s; or (from_s) f = s s alone.
@@ -405,13 +379,6 @@ __global__ void k_nlcg_quad(const float* __restrict__ g, const float* __restrict
 
 static int nl_blocks(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(kNlMaxBlocks, cdiv(n, (int64_t)kNlThreads * 4)));
-}
-
-// 1 when every non-null pointer is 16-byte aligned (float4 path of ew4).
-static int al16(std::initializer_list<const void*> ps) {
-    for (const void* p : ps)
-        if (p && (reinterpret_cast<uintptr_t>(p) & 15) != 0) return 0;
-    return 1;
 }
 
 }  // namespace dk

@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "conv_impl.cuh"
+#include "elementwise.cuh"
 #include "solvers.cuh"
 #include "stencil.cuh"
 #include "pdhg_tiled.cuh"
@@ -38,21 +39,18 @@ __device__ __forceinline__ void put_partial(PdhgDev* s, int slot, double v) {
 // ---- data-term dual: y1 = prox(y1 + sigma * A xbar) (pdhg_mlx.py:723-728) ----
 // A xbar = (1 + theta) A x_cur - theta A x_prev (linearity of A).
 template <int LOSS>
-__global__ void __launch_bounds__(256) k_dual_data(PdhgDev* s, float* __restrict__ y1,
-                                                   const float* __restrict__ axc,
+__global__ void __launch_bounds__(256) k_dual_data(PdhgDev* s, float* y1, const float* __restrict__ axc,
                                                    const float* __restrict__ axp,
-                                                   const float* __restrict__ data, float bg,
-                                                   int64_t m) {
+                                                   const float* __restrict__ data, float bg, int64_t m, int vec) {
     chain_enter();
     if (s->stop) return;
     const float sg = (float)s->sigma, th = (float)s->theta;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float a = axc[i];
-        const float axbar = xbar_of(a, axp[i], th);
-        const float arg = dual_arg(y1[i], sg, axbar);
-        const float d = data[i];
-        float out;
+    const float* in[4] = {y1, axc, axp, data};
+    float* out[1] = {y1};
+    ew4(m, in, out, vec, [&](const float* x, float* o) {
+        const float axbar = xbar_of(x[1], x[2], th);
+        const float arg = dual_arg(x[0], sg, axbar);
+        const float d = x[3];
         if constexpr (LOSS == 0) {
             // prox_poisson_dual (pdhg_mlx.py:145-166)
             const float c = 1.f - arg - sg * bg;
@@ -61,13 +59,12 @@ __global__ void __launch_bounds__(256) k_dual_data(PdhgDev* s, float* __restrict
             float z = (2.f * sg * ds) / (sqrtf(disc) - c + 1e-12f);
             z = ds < 1e-6f ? fmaxf(c, 1e-6f) : z;
             z = fmaxf(z, 1e-6f);
-            out = 1.f - z;
+            o[0] = 1.f - z;
         } else {
             // prox_gaussian_dual (pdhg_mlx.py:189)
-            out = (arg - sg * (d - bg)) / (1.f + sg);
+            o[0] = (arg - sg * (d - bg)) / (1.f + sg);
         }
-        y1[i] = out;
-    }
+    });
 }
 
 // ---- regulariser dual: y2 = proj(y2 + sigma * L xbar) (pdhg_mlx.py:732-734) ----
@@ -143,16 +140,16 @@ __global__ void __launch_bounds__(256) k_primal(PdhgDev* s, const float* __restr
 
 // sum (a - b)^2 into a slot (||A x_new - A x||^2, pdhg_mlx.py:756-759)
 __global__ void __launch_bounds__(256) k_diffsq_slot(PdhgDev* s, const float* __restrict__ a,
-                                                     const float* __restrict__ b, int64_t n,
-                                                     int slot) {
+                                                     const float* __restrict__ b, int64_t n, int slot, int vec) {
     chain_enter();
     if (s->stop) return;
     double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const double d = (double)a[i] - (b ? (double)b[i] : 0.0);
+    const float* in[2] = {a, b};
+    float* out[1] = {nullptr};
+    ew4(n, in, out, vec, [&](const float* x, float*) {
+        const double d = (double)x[0] - (double)x[1];  // a missing b reads 0
         acc += d * d;
-    }
+    });
     put_partial(s, slot, acc);
 }
 
@@ -460,35 +457,36 @@ __global__ void __launch_bounds__(256) k_hess_regloss(PdhgDev* s, const float* _
 
 // ---- RL element-wise steps for composed operators (rl_mlx.py:146-150) -------
 
-__global__ void k_rl_ratio(const float* __restrict__ model, const float* __restrict__ y, float bg,
-                           float* __restrict__ ratio, int64_t n, double* __restrict__ partials) {
+__global__ void __launch_bounds__(256) k_rl_ratio(const float* __restrict__ model, const float* __restrict__ y,
+                                                  float bg, float* __restrict__ ratio, int64_t n,
+                                                  double* __restrict__ partials, int vec) {
     chain_enter();
     double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float m = model[i] + bg;
-        const float yv = y[i];
-        if (ratio) ratio[i] = yv / fmaxf(m, 1e-10f);
+    const float* in[2] = {model, y};
+    float* out[1] = {ratio};
+    ew4(n, in, out, vec, [&](const float* x, float* o) {
+        const float m = x[0] + bg, yv = x[1];
+        o[0] = yv / fmaxf(m, 1e-10f);
         if (partials) {
             const float ys = fmaxf(yv, 1e-6f), ms = fmaxf(m, 1e-6f);
             acc += (double)(yv * logf(ys / ms) - (yv - ms));
         }
-    }
+    });
     if (partials) {
         const double b = block_sum(acc);
         if (threadIdx.x == 0) partials[blockIdx.x] = b;
     }
 }
 
-__global__ void k_rl_update(float* __restrict__ x, const float* __restrict__ corr,
-                            const float* __restrict__ sens, int64_t n) {
+__global__ void __launch_bounds__(256) k_rl_update(float* x, const float* __restrict__ corr,
+                                                   const float* __restrict__ sens, int64_t n, int vec) {
     chain_enter();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float s = sens[i];
-        const float c = s > 0.f ? corr[i] / s : 0.f;
-        x[i] = fmaxf(x[i] * c, 1e-10f);
-    }
+    const float* in[3] = {x, corr, sens};
+    float* out[1] = {x};
+    ew4(n, in, out, vec, [&](const float* v, float* o) {
+        const float c = v[2] > 0.f ? v[1] / v[2] : 0.f;
+        o[0] = fmaxf(v[0] * c, 1e-10f);
+    });
 }
 
 __global__ void k_sub_floor(const float* __restrict__ y, float bg, float* __restrict__ out, int64_t n) {
@@ -637,6 +635,11 @@ static bool first_geo(const int64_t shape[3], FirstGeo* g, int* grid) {
     return true;
 }
 
+// CTAs of the passes that move four values per thread.
+static int g4(int64_t n) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 4 * 256), (int64_t)sm_count() * 8));
+}
+
 static int g1(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 256), (int64_t)sm_count() * 16));
 }
@@ -729,9 +732,11 @@ int decon_pdhg_dual_data(decon_pdhg* h, float* y1, const float* ax_cur, const fl
     if (!h || !y1 || !ax_cur || !ax_prev || !data) return fail(DECON_ERR_NULL, "null pointer");
     const cudaStream_t s = as_stream(stream);
     if (loss_type == 0)
-        DK_TRY(chain(k_dual_data<0>, g1(m), 256, 0, s, h->dev, y1, ax_cur, ax_prev, data, background, m));
+        DK_TRY(chain(k_dual_data<0>, g4(m), 256, 0, s, h->dev, y1, ax_cur, ax_prev, data, background, m,
+                     al16({y1, ax_cur, ax_prev, data})));
     else
-        DK_TRY(chain(k_dual_data<1>, g1(m), 256, 0, s, h->dev, y1, ax_cur, ax_prev, data, background, m));
+        DK_TRY(chain(k_dual_data<1>, g4(m), 256, 0, s, h->dev, y1, ax_cur, ax_prev, data, background, m,
+                     al16({y1, ax_cur, ax_prev, data})));
     DK_LAUNCHED();
     return DECON_OK;
 }
@@ -776,10 +781,11 @@ int decon_pdhg_dk(decon_pdhg* h, const float* ax_new, const float* ax_cur, int64
                   const float* l_dx, int64_t nl, void* stream) {
     if (!h || !ax_new || !ax_cur) return fail(DECON_ERR_NULL, "null pointer");
     const cudaStream_t s = as_stream(stream);
-    DK_TRY(chain(k_diffsq_slot, kPdhgGrid, 256, 0, s, h->dev, ax_new, ax_cur, m, kSlotDA2));
+    DK_TRY(chain(k_diffsq_slot, kPdhgGrid, 256, 0, s, h->dev, ax_new, ax_cur, m, kSlotDA2,
+                 al16({ax_new, ax_cur})));
     DK_LAUNCHED();
     if (l_dx) {
-        DK_TRY(chain(k_diffsq_slot, kPdhgGrid, 256, 0, s, h->dev, l_dx, nullptr, nl, kSlotDL2));
+        DK_TRY(chain(k_diffsq_slot, kPdhgGrid, 256, 0, s, h->dev, l_dx, nullptr, nl, kSlotDL2, al16({l_dx})));
         DK_LAUNCHED();
     }
     return DECON_OK;
@@ -1029,7 +1035,8 @@ int decon_rl_ratio(const float* model, const float* observed, float background, 
     const cudaStream_t s = as_stream(stream);
     const int g = std::min<int>(g1(n), (int)reduce_partials_needed());
     double* part = loss_sum ? static_cast<double*>(workspace) : nullptr;
-    DK_TRY(chain(k_rl_ratio, g, 256, 0, s, model, observed, background, ratio, n, part));
+    DK_TRY(chain(k_rl_ratio, g, 256, 0, s, model, observed, background, ratio, n, part,
+                 al16({model, observed, ratio})));
     DK_LAUNCHED();
     if (loss_sum) DK_TRY(finish_partials(part, g, loss_sum, s));
     return DECON_OK;
@@ -1037,7 +1044,8 @@ int decon_rl_ratio(const float* model, const float* observed, float background, 
 
 int decon_rl_update(float* x, const float* corr, const float* sens_masked, int64_t n, void* stream) {
     if (!x || !corr || !sens_masked) return fail(DECON_ERR_NULL, "null pointer");
-    DK_TRY(chain(k_rl_update, g1(n), 256, 0, as_stream(stream), x, corr, sens_masked, n));
+    DK_TRY(chain(k_rl_update, g4(n), 256, 0, as_stream(stream), x, corr, sens_masked, n,
+                 al16({x, corr, sens_masked})));
     DK_LAUNCHED();
     return DECON_OK;
 }
