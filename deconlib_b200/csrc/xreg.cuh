@@ -68,6 +68,21 @@ __device__ __forceinline__ float embedded(const XRegArgs& a, const float* p, int
     return __ldg(p + kx) / sum;
 }
 
+// Bytes lo .. hi of an array of `size` bytes into L2, by one thread.  The rows a
+// CTA reads are one piece of memory; its threads ask for them 8 bytes at a time
+// and in two or more rounds, and the operands of an epilogue only after the
+// transform.  One bulk request ahead of all that (150x600x700, X length 400):
+// R2C 138 -> 117 us, update epilogue 274 -> 242, ratio 259 -> 242.  Requesting
+// rows of later CTAs instead, or the spectrum rows of the C2R pass, which are
+// all asked for at once anyway, gained no more (34.1 vs 35.2 us at 256).
+__device__ __forceinline__ void prefetch_l2(const void* p, int64_t lo, int64_t hi, int64_t size) {
+    if (hi > size) hi = size;
+    const uintptr_t b = (reinterpret_cast<uintptr_t>(p) + lo + 15) & ~(uintptr_t)15;
+    const uintptr_t e = (reinterpret_cast<uintptr_t>(p) + hi) & ~(uintptr_t)15;
+    if (lo < hi && b < e)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((uint32_t)(e - b)) : "memory");
+}
+
 // Spectrum rows row0 .. row0 + ROWS of zero lines.
 template <int ROWS, int NT>
 __device__ __forceinline__ void zero_rows(const XRegArgs& a, int64_t row0) {
@@ -123,6 +138,11 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
     }
 
     if constexpr (SRC == XS_ARRAY) {
+        if (tid == 0 && !a.win && a.pro != PRO_CONST) {
+            constexpr int W = ODD ? 2 : 1;
+            const int64_t row = W * (int64_t)line0;
+            prefetch_l2(a.in, row * a.Nx * 4, (row + W * TL) * a.Nx * 4, a.nrows * a.Nx * 4);
+        }
         if (a.win) {
             constexpr int W = ODD ? 2 : 1;
             bool any = false;
@@ -298,8 +318,10 @@ __device__ __forceinline__ float x_value(const XRegArgs& a, float v, float x, fl
         // rl_mlx.py:149-150  x = max(x * where(active, A^T ratio / sens, 0), 1e-10)
         const float c = y > 0.f ? v / y : 0.f;
         return fmaxf(x * c, 1e-10f);
-    } else {
+    } else if constexpr (EPI == EPI_RL_RATIO) {
         // rl_mlx.py:147-148  model = A x + b ; ratio = y / max(model, 1e-10)
+        return y / fmaxf(v + a.bg, 1e-10f);
+    } else {
         const float m = v + a.bg;
         if (a.partials) {
             // rl_mlx.py:75-79: y log(max(y,eps)/max(m,eps)) - (y - max(m,eps))
@@ -329,6 +351,29 @@ __device__ __forceinline__ void x_store(const XRegArgs& a, int64_t i, int step, 
             if (r0 + e < B && keep(r0 + e))
                 *reinterpret_cast<V*>(a.out_real + i + (int64_t)(r0 + e) * step) =
                     x_value<EPI>(a, value(r0 + e), o[e].x, o[e].y, acc);
+    }
+}
+
+// A thread's B points of one line of the real array.
+template <int EPI, bool ODD, int B, int S>
+__device__ __forceinline__ void c2r_store(const XRegArgs& a, uint32_t line, int j, float s, const C1* v, double& acc) {
+    // elements x0 .. x0 + wx of a row are kept (all of them but for a window)
+    auto kept = [&](int x) { return (uint32_t)(x - a.x0) < (uint32_t)a.wx; };
+    if constexpr (ODD) {
+        const int64_t o0 = array_row(a, 2 * line), o1 = array_row(a, 2 * line + 1);
+        auto in_row = [&](int r) { return kept(j + r * S); };
+        if (o0 != kNoRow) x_store<EPI, float, B>(a, o0 + j, S, acc, in_row, [&](int r) { return v[r].re * s; });
+        if (o1 != kNoRow) x_store<EPI, float, B>(a, o1 + j, S, acc, in_row, [&](int r) { return v[r].im * s; });
+    } else if (a.vec) {
+        x_store<EPI, float2, B>(a, (int64_t)line * a.wx - a.x0 + 2 * j, 2 * S, acc,
+                                [&](int r) { return kept(2 * (j + r * S)); },
+                                [&](int r) { return make_float2(v[r].re * s, v[r].im * s); });
+    } else {
+        const int64_t i = (int64_t)line * a.wx - a.x0 + 2 * j;
+        x_store<EPI, float, B>(a, i, 2 * S, acc, [&](int r) { return kept(2 * (j + r * S)); },
+                               [&](int r) { return v[r].re * s; });
+        x_store<EPI, float, B>(a, i + 1, 2 * S, acc, [&](int r) { return kept(2 * (j + r * S) + 1); },
+                               [&](int r) { return v[r].im * s; });
     }
 }
 
@@ -364,6 +409,14 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
     const uint32_t line0 = blockIdx.x * TL;
     chain_enter();
 
+    if constexpr (EPI == EPI_RL_RATIO || EPI == EPI_RL_UPDATE) {
+        if (tid == 0) {
+            constexpr int W = ODD ? 2 : 1;
+            const int64_t lo = W * (int64_t)line0 * a.Nx * 4, hi = lo + W * TL * a.Nx * 4, size = a.nrows * a.Nx * 4;
+            prefetch_l2(a.aux0, lo, hi, size);
+            if (EPI == EPI_RL_UPDATE) prefetch_l2(a.aux1, lo, hi, size);
+        }
+    }
     if constexpr (ODD && EPI == EPI_STORE) {
         if (a.win) {  // pairs of rows outside the window
             bool any = false;
@@ -496,23 +549,14 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
             if (line >= a.nlines) continue;
             C1 v[B];
             transform(l, j, v);
-            // elements x0 .. x0 + wx of a row are kept (all of them but for a window)
-            auto kept = [&](int x) { return (uint32_t)(x - a.x0) < (uint32_t)a.wx; };
-            if constexpr (ODD) {
-                const int64_t o0 = array_row(a, 2 * line), o1 = array_row(a, 2 * line + 1);
-                auto in_row = [&](int r) { return kept(j + r * S); };
-                if (o0 != kNoRow) x_store<EPI, float, B>(a, o0 + j, S, acc, in_row, [&](int r) { return v[r].re * s; });
-                if (o1 != kNoRow) x_store<EPI, float, B>(a, o1 + j, S, acc, in_row, [&](int r) { return v[r].im * s; });
-            } else if (a.vec) {
-                x_store<EPI, float2, B>(a, (int64_t)line * a.wx - a.x0 + 2 * j, 2 * S, acc,
-                                        [&](int r) { return kept(2 * (j + r * S)); },
-                                        [&](int r) { return make_float2(v[r].re * s, v[r].im * s); });
+            if constexpr (EPI == EPI_RL_RATIO) {
+                // the loss and the model in code of their own: in the same loop
+                // every iteration jumped over a logarithm per voxel (284 -> 259 us
+                // at 150x600x700)
+                if (a.partials || a.pred) c2r_store<EPI_PRED, ODD, B, S>(a, line, j, s, v, acc);
+                else c2r_store<EPI, ODD, B, S>(a, line, j, s, v, acc);
             } else {
-                const int64_t i = (int64_t)line * a.wx - a.x0 + 2 * j;
-                x_store<EPI, float, B>(a, i, 2 * S, acc, [&](int r) { return kept(2 * (j + r * S)); },
-                                       [&](int r) { return v[r].re * s; });
-                x_store<EPI, float, B>(a, i + 1, 2 * S, acc, [&](int r) { return kept(2 * (j + r * S) + 1); },
-                                       [&](int r) { return v[r].im * s; });
+                c2r_store<EPI, ODD, B, S>(a, line, j, s, v, acc);
             }
         }
     }
