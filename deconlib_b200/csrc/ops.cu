@@ -319,8 +319,11 @@ int decon_banded_axis(const float* in, float* out, int64_t outer, int64_t n_in, 
             // enough CTAs to fill the GPU, each walking many rows; short rows side
             // by side in a block (one row per block left two thirds of it idle at 88)
             const int64_t tx = std::min<int64_t>(256, round_up(n_out, 32)), ty = 256 / tx, gx = cdiv(n_out, tx);
-            const int64_t gy =
-                std::max<int64_t>(1, std::min<int64_t>(cdiv(outer, ty), cdiv((int64_t)sm_count() * 16, gx)));
+            // eight rows per thread once that fills the GPU: its taps and weights are
+            // read once for all of them
+            const int64_t full = cdiv((int64_t)sm_count() * 16, gx), few = cdiv((int64_t)sm_count() * 2, gx);
+            const int64_t gy = std::min<int64_t>(
+                std::max(std::min(cdiv(outer, ty), few), std::min(cdiv(outer, ty * 8), full)), 65535);
             dim3 g((unsigned)gx, (unsigned)gy);
             DK_TRY(chain(k_banded_last_rows, g, dim3((unsigned)tx, (unsigned)ty), 0, st, in, out, outer, n_in, n_out, idx, w, width));
         } else {
