@@ -1,11 +1,11 @@
-// Register DFTs of composite length on one or two columns at once, and the
-// split of an axis length into two of them.
+// Register DFTs of composite length, and the split of an axis length into two
+// of them.
 //
 // dftn<N, DIR>(v) transforms N complex values held by one thread, natural
-// order in and out, unnormalised.  The real type F is float (one column) or
-// Two (two columns: every addition and multiply-add is one packed f32x2
-// instruction, which halves the issue slots of the arithmetic; the FP32 pipe
-// itself has the same rate for both).  N is a product of the primitive
+// order in and out, unnormalised.  Two columns per thread in packed f32x2
+// instructions halve the issue slots of the arithmetic but not its pipe time,
+// and double the registers: no gain (axial pass at 256 points 115 us against
+// 118 in the layout that suits them best).  N is a product of the primitive
 // codelets 2, 3, 4, 5, 8, 16: co-prime factors combine without twiddles
 // (prime-factor indexing, Good 1958), the others by one Cooley-Tukey step
 // with twiddles that are compile-time constants.
@@ -18,23 +18,10 @@
 
 namespace dk {
 
-// ---- one or two reals -------------------------------------------------------
-
-struct Two {
-    float2 v;
-};
 __device__ __forceinline__ float add(float a, float b) { return a + b; }
 __device__ __forceinline__ float sub(float a, float b) { return a - b; }
 __device__ __forceinline__ float mul(float a, float b) { return a * b; }
 __device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ Two both(float s) { return Two{make_float2(s, s)}; }
-__device__ __forceinline__ Two add(Two a, Two b) { return Two{__fadd2_rn(a.v, b.v)}; }
-// a - b as one packed operation: the product with -1 is exact
-__device__ __forceinline__ Two sub(Two a, Two b) { return Two{__ffma2_rn(b.v, make_float2(-1.f, -1.f), a.v)}; }
-__device__ __forceinline__ Two mul(Two a, float b) { return Two{__fmul2_rn(a.v, make_float2(b, b))}; }
-__device__ __forceinline__ Two mad(Two a, float b, Two c) { return Two{__ffma2_rn(a.v, make_float2(b, b), c.v)}; }
-__device__ __forceinline__ Two mul(Two a, Two b) { return Two{__fmul2_rn(a.v, b.v)}; }
-__device__ __forceinline__ Two mad(Two a, Two b, Two c) { return Two{__ffma2_rn(a.v, b.v, c.v)}; }
 
 template <class F>
 struct Cx {

@@ -302,159 +302,6 @@ __global__ void k_record_loss(PdhgDev* s, double alpha, int kk) {
     if (threadIdx.x == 0) s->loss_hist[kk] = dl + alpha * rl;
 }
 
-// ---- fused Hessian3D PDHG kernels --------------------------------------------
-// The regulariser half of the iteration without materialising L x_bar, L^T y2
-// or L (x_new - x): the Hessian is evaluated on the fly from the fields below
-// (values identical to the stand-alone operator, the same float32 ops).
-
-struct XbarField {  // x_bar = x + theta (x - x_prev)
-    const float* xc;
-    const float* xp;
-    float th;
-    int64_t ny, nx;
-    __device__ __forceinline__ float operator()(int64_t z, int64_t y, int64_t x) const {
-        const int64_t i = (z * ny + y) * nx + x;
-        const float a = __ldg(xc + i);
-        return xbar_of(a, __ldg(xp + i), th);
-    }
-};
-
-struct DiffField {  // x_new - x
-    const float* a;
-    const float* b;
-    int64_t ny, nx;
-    __device__ __forceinline__ float operator()(int64_t z, int64_t y, int64_t x) const {
-        const int64_t i = (z * ny + y) * nx + x;
-        return __ldg(a + i) - __ldg(b + i);
-    }
-};
-
-struct PlainField {
-    const float* p;
-    int64_t ny, nx;
-    __device__ __forceinline__ float operator()(int64_t z, int64_t y, int64_t x) const {
-        return __ldg(p + (z * ny + y) * nx + x);
-    }
-};
-
-// y2 = proj(y2 + sigma H x_bar) (pdhg_mlx.py:732-734 with x_bar of :841).
-template <int NORM>
-__global__ void __launch_bounds__(256) k_hess_dual(PdhgDev* s, float* __restrict__ y2,
-                                                   const float* __restrict__ xc,
-                                                   const float* __restrict__ xp, Dims d, W6 w,
-                                                   float alpha) {
-    chain_enter();
-    if (s->stop) return;
-    const float sg = (float)s->sigma;
-    const XbarField f{xc, xp, (float)s->theta, d.ny, d.nx};
-    const int64_t n = d.nz * d.ny * d.nx;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t x = i % d.nx, t = i / d.nx, y = t % d.ny, z = t / d.ny;
-        float h[6];
-        hess6(f, z, y, x, d, w.w, h);
-        if constexpr (NORM == 0) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                const int64_t j = c * n + i;
-                y2[j] = fminf(fmaxf(dual_arg(y2[j], sg, h[c]), -alpha), alpha);
-            }
-        } else {
-            float v[6];
-            float ss = 0.f;
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                v[c] = dual_arg(y2[c * n + i], sg, h[c]);
-                ss += v[c] * v[c];
-            }
-            const float sc = fmaxf(sqrtf(ss + 1e-12f) / alpha, 1.f);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) y2[c * n + i] = v[c] / sc;
-        }
-    }
-}
-
-// x_new = max(0, x - tau (A^T y1 + H^T y2)) with the FP64 sums of k_primal.
-__global__ void __launch_bounds__(256) k_hess_primal(PdhgDev* s, const float* __restrict__ xc,
-                                                     const float* __restrict__ aty,
-                                                     const float* __restrict__ y2,
-                                                     float* __restrict__ xn, Dims d, W6 w) {
-    chain_enter();
-    if (s->stop) return;
-    const float tau = (float)s->tau;
-    const int64_t n = d.nz * d.ny * d.nx;
-    double dx2 = 0.0, xc2 = 0.0, xn2 = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t x = i % d.nx, t = i / d.nx, y = t % d.ny, z = t / d.ny;
-        const float a = xc[i];
-        const float g = __fadd_rn(aty[i], hess_adj_at(y2, z, y, x, d, w.w));
-        const float v = primal_of(a, tau, g);
-        xn[i] = v;
-        const float dd = v - a;
-        dx2 += (double)dd * dd;
-        xc2 += (double)a * a;
-        xn2 += (double)v * v;
-    }
-    put_partial(s, kSlotDx2, dx2);
-    put_partial(s, kSlotXc2, xc2);
-    put_partial(s, kSlotXn2, xn2);
-}
-
-// ||A x_new - A x||^2 (slot DA2) and ||H (x_new - x)||^2 (slot DL2).
-__global__ void __launch_bounds__(256) k_hess_dk(PdhgDev* s, const float* __restrict__ axn,
-                                                 const float* __restrict__ axc, int64_t m,
-                                                 const float* __restrict__ xn,
-                                                 const float* __restrict__ xc, Dims d, W6 w) {
-    chain_enter();
-    if (s->stop) return;
-    double a2 = 0.0, l2 = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const double dd = (double)axn[i] - (double)axc[i];
-        a2 += dd * dd;
-    }
-    const DiffField f{xn, xc, d.ny, d.nx};
-    const int64_t n = d.nz * d.ny * d.nx;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t x = i % d.nx, t = i / d.nx, y = t % d.ny, z = t / d.ny;
-        float h[6];
-        hess6(f, z, y, x, d, w.w, h);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) l2 += (double)h[c] * (double)h[c];
-    }
-    put_partial(s, kSlotDA2, a2);
-    put_partial(s, kSlotDL2, l2);
-}
-
-// Regulariser part of the objective on H x (pdhg_mlx.py:873-879).
-template <int NORM>
-__global__ void __launch_bounds__(256) k_hess_regloss(PdhgDev* s, const float* __restrict__ x,
-                                                      Dims d, W6 w, int kk) {
-    chain_enter();
-    if (!loss_active(s, kk)) return;
-    const PlainField f{x, d.ny, d.nx};
-    const int64_t n = d.nz * d.ny * d.nx;
-    double acc = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t xx = i % d.nx, t = i / d.nx, y = t % d.ny, z = t / d.ny;
-        float h[6];
-        hess6(f, z, y, xx, d, w.w, h);
-        if constexpr (NORM == 0) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) acc += fabs((double)h[c]);
-        } else {
-            float ss = 0.f;
-#pragma unroll
-            for (int c = 0; c < 6; ++c) ss += h[c] * h[c];
-            acc += (double)sqrtf(ss + 1e-12f);
-        }
-    }
-    put_partial(s, kSlotReg, acc);
-}
-
 // ---- RL element-wise steps for composed operators (rl_mlx.py:146-150) -------
 
 __global__ void __launch_bounds__(256) k_rl_ratio(const float* __restrict__ model, const float* __restrict__ y,

@@ -156,21 +156,6 @@ __device__ __forceinline__ float hess_adj_gen(const G& g, int64_t z, int64_t y, 
     return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(azz, ayy), axx), ayz), axz), axy);
 }
 
-// Accessor of the six components stored as hw[c * n + i].
-struct Hess6Global {
-    const float* hw;
-    int64_t n, ny, nx;
-    __device__ __forceinline__ float operator()(int c, int64_t z, int64_t y, int64_t x) const {
-        return __ldg(hw + c * n + (z * ny + y) * nx + x);
-    }
-};
-
-__device__ __forceinline__ float hess_adj_at(const float* hw, int64_t z, int64_t y, int64_t x,
-                                             const Dims& d, const float w[6]) {
-    const Hess6Global g{hw, d.nz * d.ny * d.nx, d.ny, d.nx};
-    return hess_adj_gen(g, z, y, x, d, w);
-}
-
 // Component weights [r^2, 1, 1, sqrt2 r, sqrt2 r, sqrt2] (linops_mlx.py:237-239;
 // SQRT2 is a float32 device scalar there).
 inline void hessian_weights(float r, float w[6]) {
