@@ -245,7 +245,7 @@ def run_serving(D, n_jobs):
            "note": "latency = arrival to restored volume on the host; plain = the same jobs "
                    "one at a time through richardson_lucy_with_operator / solve_pdhg_mlx on the "
                    "reference's canvases (fast_padded_shape); the server puts each job on "
-                   "static_fft_shape (compile-time FFT lengths)"}
+                   "static_fft_shape (lengths 2^a x {1, 3, 5, 15})"}
     return out
 
 
@@ -915,7 +915,7 @@ def run_ours(args, ws, rank, local):
             "bound": "hbm",
             "kernel": ("k_yz<512,256> fused Y FFT / axial FFT x OTF x IFFT / Y IFFT, one 8-CTA "
                        "cluster per kx column" if fused else
-                       "k_col_pipe<16,1,OTF> axial FFT x OTF x IFFT (lean, 2 CTAs/SM)"),
+                       "k_colreg<256,OTF> axial FFT x OTF x IFFT (register DFTs, 2 CTAs/SM)"),
             "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
             "peak_source": src, "traffic": traffic, "algorithmic_bytes_per_launch": z_bytes,
             "launch_ms": z_ms, "launches": nz_launch.value,

@@ -6,8 +6,8 @@ own PSFs join the same batch.  Every problem gets its own convolution plan,
 with an FFT canvas and a pass schedule chosen by ``autotune_schedule`` (each
 candidate canvas is a different radix factorisation of the axes, each
 schedule a different family of equivalent FFT kernels: fused or separate
-Y / axial passes, pipelined / one-tile / plain-load column kernels, one- or
-two-CTA axial kernel, radix order, lines per CTA; the fastest measured
+Y / axial passes, register or runtime-radix kernels, radix order, lines per
+CTA; the fastest measured
 forward + adjoint convolution wins, cached per shape in memory and in a JSON
 file), and K iterations of
 all problems are recorded into one CUDA graph by the native batch runtime
@@ -121,10 +121,9 @@ def _next_23(n: int) -> int:
 
 def fft_shape_candidates(signal_shape, kernel_shape, max_growth: float = 1.35) -> List[tuple]:
     """Canvases to try: the reference's 5-smooth minimum on every axis, and
-    variants with 2^a 3^b or power-of-two lengths (other radix sequences;
-    power-of-two y / z lengths <= 512 also select the TMA-pipelined column
-    kernels) where they grow an axis by <= max_growth, and the lengths of
-    ``static_fft_shape`` (compile-time radix sequences).  Sorted by volume."""
+    variants with 2^a 3^b or power-of-two lengths (other radix pairs) where
+    they grow an axis by <= max_growth, and the lengths of
+    ``static_fft_shape``.  Sorted by volume."""
     m = [int(n) + int(k) - 1 for n, k in zip(signal_shape, kernel_shape)]
     s5 = [_next_smooth_number(v) for v in m]
     st = static_fft_shape(signal_shape, kernel_shape)
@@ -226,9 +225,8 @@ def autotune_schedule(signal_shape, psf, candidates: Optional[List[tuple]] = Non
     """Fastest (canvas, schedule) for a LinearFFTConvolver of ``psf`` on
     ``signal_shape``: every candidate canvas (a different radix factorisation)
     is timed under every applicable schedule (fused or separate Y / axial
-    passes, pipelined / one-tile / plain-load column kernels, one- or two-CTA
-    axial kernel, radix order, lines per CTA), forward + adjoint with CUDA
-    events after a warm-up.  The winner is cached per (device, signal shape,
+    passes, register or runtime-radix kernels, radix order, lines per CTA),
+    forward + adjoint with CUDA events after a warm-up.  The winner is cached per (device, signal shape,
     kernel shape) in memory and in the JSON file of ``tune_cache_path()``;
     shapes with the same candidate canvases share one timing."""
     _load_cache()
@@ -240,7 +238,7 @@ def autotune_schedule(signal_shape, psf, candidates: Optional[List[tuple]] = Non
         return _TUNED[key][0], _TUNED[key][1]
     cands = list((candidates or fft_shape_candidates(sig, kshape))[:max_candidates])
     if candidates is None:
-        # always time the canvas of compile-time FFT lengths
+        # always time the canvas of static_fft_shape
         st = tuple(static_fft_shape(sig, kshape))
         if st not in cands:
             cands[-1:] = [st]

@@ -15,7 +15,11 @@
 // is formed, so no thread waits for HBM while the SM has arithmetic to do.
 // Loading straight into registers instead left the warps on the loads for
 // ~45 % of the issue slots (axial pass at 256 points, canvas 256x512x512:
-// 150 us; with the TMA buffers 118 us, 539 MB = 4.57 TB/s).  Shared-memory
+// 150 us; with the TMA buffers 118 us on spectra of its own, 128 us between the
+// other passes: 539 MB, 4.2 TB/s; 141 us for the shared-memory FFT before).
+// Bound by latency at 0.65 instructions per cycle and scheduler; neither more
+// warps (64 registers), nor half the threads for R2 = 2 R1, which idle in that
+// stage, nor two columns per thread was faster over the lengths.  Shared-memory
 // rows are 128 bytes (T = 16) or 64 (T = 8), read by half-warps in whole rows,
 // so no swizzle is needed; the exchange buffer is separate from the input
 // buffer, which is what frees the latter early.

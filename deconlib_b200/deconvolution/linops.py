@@ -59,26 +59,22 @@ def fast_padded_shape(signal_shape, kernel_shape, min_pad=None) -> Tuple[int, ..
     return tuple(out)
 
 
-# FFT lengths with a compile-time radix sequence in the library (2^a x {1, 3,
-# 5, 15}, 64 to 1024): the strided passes of these lengths run straight-line
-# stages; other 7-smooth lengths take the runtime-radix path, which measured
-# ~4x slower per canvas voxel on the B200.
+# Lengths 2^a x {1, 3, 5, 15}, 64 to 1024.  Few enough that jobs of similar
+# sizes share a canvas; every 5-smooth length up to 1024 has kernels of its own
+# and runs about as fast per canvas voxel.
 STATIC_FFT_LENGTHS = (64, 80, 96, 128, 160, 192, 240, 256, 320, 384, 480, 512, 640, 768, 960, 1024)
 
 
 def static_fft_shape(signal_shape, kernel_shape) -> Tuple[int, ...]:
-    """Wrap-free canvas on the compile-time FFT lengths (not in the reference).
+    """Wrap-free canvas on few FFT lengths (not in the reference).
 
     Per axis the smallest length >= N + M - 1 in ``STATIC_FFT_LENGTHS`` (the
     last axis, transformed as packed complex pairs, twice such a length), when
     that grows the axis by at most 1/3 over ``fast_padded_shape``'s 5-smooth
     length; otherwise the 5-smooth length.  The axial (first) axis of a 3-D
     canvas takes 64, 128 or 256 instead when that is at most twice the
-    length chosen so: those lengths run the TMA-pipelined axial kernels,
-    which measured faster per iteration on the B200 even on the larger canvas
-    (RL at 76x362x244: 1.43 ms on 256x768x512 vs 2.29 ms on 160x768x512).
-    A convolution's result does not depend on the canvas beyond FP32
-    rounding."""
+    length chosen so: the lengths that have an FP16 OTF.  A convolution's
+    result does not depend on the canvas beyond FP32 rounding."""
     ref = fast_padded_shape(signal_shape, kernel_shape)
     nd = len(ref)
     out = []
@@ -267,7 +263,7 @@ class LinearFFTConvolver:
         """"fp32" or "mixed" (not in the reference): "mixed" stores the OTF as
         FP16 complex with a power-of-two scale per kz plane for the axial FFT
         pass; transforms and products stay FP32, reductions FP64.  Raises
-        RuntimeError when this canvas has no pipelined axial pass."""
+        RuntimeError when this canvas has no FP16 axial pass."""
         codes = {"fp32": 0, "mixed": 1}
         if precision not in codes:
             raise ValueError(f"precision must be 'fp32' or 'mixed', got {precision!r}")
@@ -277,7 +273,7 @@ class LinearFFTConvolver:
 
     def set_kernel(self, kernel) -> "LinearFFTConvolver":
         """Replace the kernel by another of the same shape, rebuilding the OTF
-        in this plan's device buffers (no allocation, no cudaFree).  Not in
+        in this plan's device buffers (no allocation).  Not in
         the reference; a serving loop uses it to hand a pooled plan to the next
         job of the same shape.  Synchronises the current stream."""
         k = to_device(kernel)

@@ -16,13 +16,12 @@ time.  The server
     kernel and signal shapes, which rebuilds the OTF in place
     (``LinearFFTConvolver.set_kernel``), and its PDHG state to the next PDHG
     job (``decon_pdhg_reset``).  Nothing is freed while jobs run, because
-    ``cudaFree`` synchronises the whole device and would drain every stream;
-  * puts every job's convolution on a canvas of compile-time FFT lengths
-    (``canvas="static"``: ``static_fft_shape``, each axis at most 1/3 longer
-    than the reference's 5-smooth canvas), because the runtime-radix FFT path
-    that most 5-smooth lengths take measured ~4x slower per canvas voxel;
-    ``canvas="reference"`` keeps ``fast_padded_shape``.  The canvas changes a
-    result by FP32 rounding only.
+    releasing a plan waits for the whole device and would drain every stream;
+  * puts every job's convolution on the canvas of ``static_fft_shape``
+    (``canvas="static"``: lengths 2^a x {1, 3, 5, 15}, so that more jobs share
+    a pooled plan) or, with ``canvas="reference"``, of ``fast_padded_shape``
+    (5-smooth, usually smaller).  The canvas changes a result by FP32 rounding
+    only.
 
 Latency is arrival -> restored volume on the host.  The reference has no
 serving layer; each job computes exactly what ``richardson_lucy_with_operator``
@@ -379,7 +378,7 @@ class DeconServer:
     ``budget_bytes``: device bytes admitted jobs (plus idle pooled plans) may
     hold; ``max_active``: concurrent jobs (one stream each); ``chunk``:
     iterations queued per job per scheduling round; ``canvas``: "static"
-    (compile-time FFT lengths) or "reference" (the reference's canvases)."""
+    (lengths 2^a x {1, 3, 5, 15}) or "reference" (the reference's canvases)."""
 
     def __init__(self, budget_bytes: int = 150 * 10**9, max_active: int = 8, chunk: int = 8,
                  prioritise: bool = True, canvas: str = "static"):

@@ -111,11 +111,12 @@ int decon_conv_norm_sq(const decon_conv* plan, double* out);
  *   FUSED        the fused Y / axial cluster pass where the canvas allows it
  *                (allocates the kx-major OTF copy on first request; DECON_YZ=1
  *                selects it for every plan)
- *   NO_PIPE      one-tile TMA column kernels instead of the persistent pipelined ones
- *   NO_TMA       plain-load column kernels (no tensor maps)
- *   LEAN_OFF     one-CTA-per-SM axial kernel instead of the two-CTA (lean) one
- *   ODD_RADIX    radix plans with the 5 / 3 / 7 stages first (runtime-length axes)
- *   HALF_LINES   half the lines per CTA on runtime-length axes (more, smaller CTAs) */
+ *   NO_PIPE      the FP32 OTF for a plan set to mixed precision; no effect else
+ *   NO_TMA       runtime-radix kernels with plain loads instead of the register
+ *                kernels (no tensor maps)
+ *   LEAN_OFF     no effect (kept for saved schedules)
+ *   ODD_RADIX    radix plans with the 5 / 3 / 7 stages first (runtime-radix axes)
+ *   HALF_LINES   half the lines per CTA on runtime-radix axes (more, smaller CTAs) */
 #define DECON_SCHED_FUSED 1
 #define DECON_SCHED_NO_PIPE 2
 #define DECON_SCHED_NO_TMA 4
