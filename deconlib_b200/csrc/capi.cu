@@ -376,7 +376,9 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
     p->ax_y.tws = 1;
     p->ax_z.tw = p->twz;
     p->ax_z.tws = 1;
-    p->npartials = std::max<int64_t>(reduce_partials_needed(), cdiv(nz * ny, std::min(p->T_x, 4)) + 1);
+    // one partial per CTA of the fullest X pass: four rows per CTA in the register
+    // kernels, T_x, or half of it (DECON_SCHED_HALF_LINES), in the others
+    p->npartials = std::max<int64_t>(reduce_partials_needed(), cdiv(nz * ny, std::max(1, std::min(p->T_x / 2, 4))) + 1);
     if ((st = pool_alloc((void**)&p->otf, (size_t)Fz * Fy * p->P * sizeof(float2), "OTF")) ||
         (st = pool_alloc((void**)&p->s1, (size_t)nz * ny * p->P * sizeof(float2), "spectrum S1")) ||
         (st = pool_alloc((void**)&p->s2, (size_t)nz * Fy * p->P * sizeof(float2), "spectrum S2")) ||

@@ -386,6 +386,12 @@ int launch_col(const ConvPlan& p, const Axis& ax, int T, int mode, const float2*
                   (mode == COL_OTF || mode == COL_OTF_CONJ) ? PROF_ZOTF : PROF_COL);
 }
 
+// A pass that sums writes one partial per CTA.
+static int check_partials(const ConvPlan& p, const double* partials, int64_t nblk) {
+    if (partials && nblk > p.npartials) return fail(DECON_ERR_VALUE, "X pass: partials buffer too small");
+    return DECON_OK;
+}
+
 int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* out,
                 const float* aux0, const float* aux1, float bg, double* partials, int* nblk_out,
                 cudaStream_t st) {
@@ -409,6 +415,7 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
         a.scale = (float)(1.0 / ((double)p.F[0] * (double)p.F[1] * (double)p.F[2]));
         a.vec = a.wx % 2 == 0 && a.x0 % 2 == 0 && pair_aligned(out) && pair_aligned(aux0) && pair_aligned(aux1);
         const int64_t nblk = cdiv(a.nlines, k.TL);
+        DK_TRY(check_partials(p, partials, nblk));
         if (nblk_out) *nblk_out = (int)nblk;
         return launch(k.fn, nblk, k.nt, k.smem, st, &a, PROF_XC2R);
     }
@@ -454,6 +461,7 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
     }
     const int nthr = threads_for(a.T, a.ax);
     const int64_t nblk = cdiv(a.nrows, a.T);
+    DK_TRY(check_partials(p, partials, nblk));
     if (nblk_out) *nblk_out = (int)nblk;
     const size_t smem = (size_t)a.T * a.ax.L * sizeof(float2);
     void* fn = pick_xc2r_kernel(epi);

@@ -1,0 +1,43 @@
+"""Schedules of a convolution plan other than the default one.
+
+A schedule changes which kernels run and how many rows or columns a CTA takes,
+so per-row values keep their bits wherever the kernels are the same, and sums
+over a volume change by the order of their FP64 additions only.
+"""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+HALF_LINES = 32
+
+
+@pytest.fixture(scope="module")
+def D():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import deconlib_b200.deconvolution as d
+
+    return d
+
+
+# X lines of the runtime-radix pass with four, two and one row per CTA.  Half the
+# lines mean twice the CTAs (1200, 1600 and 1400), each with a loss partial of its
+# own: more than the 1184 that every plan holds.
+@pytest.mark.parametrize("sig,fft", [((8, 300, 1030), (8, 320, 2100)), ((4, 400, 2100), (4, 400, 4200)),
+                                     ((4, 350, 4200), (4, 350, 8400))])
+def test_loss_under_half_lines(D, sig, fft):
+    rng = np.random.default_rng(5)
+    psf = rng.random((1, 1, 5)).astype(np.float32)
+    obs = rng.poisson(20.0, sig).astype(np.float32)
+    runs = []
+    for sched in (0, HALF_LINES):
+        conv = D.LinearFFTConvolver(psf, sig, fft_shape=fft, schedule=sched)
+        runs.append(D.richardson_lucy_with_operator(obs, conv, num_iter=2, background=1.0, eval_interval=1))
+    a, b = runs
+    assert torch.equal(a.restored, b.restored)
+    # 6e6 terms of one sign in another order: below 6e6 eps64 of the sum
+    assert len(a.loss_history) == 2
+    np.testing.assert_allclose(a.loss_history, b.loss_history, rtol=1e-9)
