@@ -18,7 +18,7 @@ PKG = os.path.dirname(HERE)
 ROOT = os.path.dirname(PKG)
 OBJ = os.path.join(ROOT, "_build", "obj")
 LIB = os.path.join(PKG, "libdecon_b200.so")
-SOURCES = ["capi.cu", "conv.cu", "reduce.cu", "ops.cu", "solvers.cu", "noalloc.cu", "batch.cu", "psf.cu", "nlcg.cu", "pdhg_run.cu", "pupil.cu",
+SOURCES = ["capi.cu", "pool.cu", "conv.cu", "reduce.cu", "ops.cu", "solvers.cu", "noalloc.cu", "batch.cu", "psf.cu", "nlcg.cu", "pdhg_run.cu", "pupil.cu",
            "fftplain.cu",
            "colreg_a.cu", "colreg_b.cu", "colreg_c.cu", "colreg_d.cu", "colreg_e.cu",
            "psf_any.cu", "psf_a.cu", "psf_b.cu", "psf_c.cu", "psf_d.cu", "psf_e.cu",

@@ -39,23 +39,6 @@ int fail(int code, const char* fmt, ...) {
     return code;
 }
 
-static cudaStream_t setup_stream() {
-    static std::mutex mu;
-    static std::map<int, cudaStream_t> streams;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = streams.find(dev);
-    if (it != streams.end()) return it->second;
-    cudaStream_t s = nullptr;
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    streams[dev] = s;
-    return s;
-}
-
 int upload_blocking(void* dst, const void* src, size_t bytes) {
     const cudaStream_t s = setup_stream();
     if (!s) return fail(DECON_ERR_CUDA, "set-up stream creation failed");
@@ -112,71 +95,6 @@ int twiddle_table(int L, const float2** out) {
     }
     *out = t;
     return DECON_OK;
-}
-
-constexpr uint64_t kPoolKeep = uint64_t(2) << 30;
-
-int device_pool(cudaMemPool_t* out) {
-    static std::mutex mu;
-    static std::map<int, cudaMemPool_t> pools;
-    int dev = 0;
-    DK_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = pools.find(dev);
-    if (it == pools.end()) {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool;
-        DK_CUDA(cudaMemPoolCreate(&pool, &props));
-        uint64_t keep = kPoolKeep;
-        DK_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-        it = pools.emplace(dev, pool).first;
-    }
-    *out = it->second;
-    return DECON_OK;
-}
-
-int pool_alloc(void** p, size_t bytes, const char* what) {
-    *p = nullptr;
-    cudaMemPool_t pool;
-    DK_TRY(device_pool(&pool));
-    const cudaStream_t s = setup_stream();
-    if (!s) return fail(DECON_ERR_CUDA, "set-up stream creation failed");
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        cudaStreamSynchronize(s);
-        cudaMemPoolTrimTo(pool, 0);
-        e = cudaMallocFromPoolAsync(p, bytes, pool, s);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        *p = nullptr;
-        return fail(e == cudaErrorMemoryAllocation ? DECON_ERR_OOM : DECON_ERR_CUDA,
-                    "cudaMalloc of %zu bytes for %s failed: %s", bytes, what, cudaGetErrorString(e));
-    }
-    return DECON_OK;
-}
-
-void pool_free(std::initializer_list<void*> ptrs) {
-    void* first = nullptr;
-    for (void* p : ptrs) first = first ? first : p;
-    if (!first) return;
-    // the pool and its stream belong to the device of the memory
-    int cur = 0;
-    cudaGetDevice(&cur);
-    cudaPointerAttributes at{};
-    const bool other = cudaPointerGetAttributes(&at, first) == cudaSuccess && at.device != cur;
-    if (other) cudaSetDevice(at.device);
-    cudaDeviceSynchronize();
-    const cudaStream_t s = setup_stream();
-    for (void* p : ptrs)
-        if (p) cudaFreeAsync(p, s);
-    if (other) cudaSetDevice(cur);
-    cudaGetLastError();
 }
 
 static void free_plan(ConvPlan* p) {

@@ -12,6 +12,7 @@
 #include <utility>
 
 #include "../../include/decon_b200.h"
+#include "pool.cuh"
 
 namespace dk {
 
@@ -123,17 +124,6 @@ int chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t
     return DECON_OK;
 }
 #endif
-
-// Device memory of plans, solver states and scratch, from a pool per device that
-// keeps at most 2 GB between objects: a solve that builds its plan (500 MB at
-// 128x256x256) spent 1.2 ms in cudaMalloc and 1.4-4.6 ms in cudaFree.  Memory
-// above that goes back to the driver at the next synchronisation, all of it
-// when an allocation fails.  pool_alloc returns memory that every stream may
-// use at once; pool_free waits for the device's work, as cudaFree does, so
-// nothing still running can touch what the next object gets.
-int device_pool(cudaMemPool_t* out);
-int pool_alloc(void** p, size_t bytes, const char* what);
-void pool_free(std::initializer_list<void*> ptrs);
 
 // Table W_L^m = exp(-2 pi i m / L), m < L, computed in double; one per device
 // and length, kept for the life of the process, readable by every stream.

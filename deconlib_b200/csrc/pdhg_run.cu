@@ -322,7 +322,7 @@ int decon_pdhg_solver_state(decon_pdhg_solver* s, decon_pdhg** state, int* queue
 int decon_pdhg_solver_destroy(decon_pdhg_solver* s) {
     if (!s) return DECON_OK;
     if (s->state) decon_pdhg_destroy(s->state);
-    for (void* p : s->allocs) dk::pool_free({p});
+    dk::pool_free(s->allocs.data(), s->allocs.size());
     delete s;
     return DECON_OK;
 }

@@ -146,7 +146,7 @@ class _ConvPlan:
         if h is not None and h.value and _lib._lib is not None:
             try:
                 with torch.cuda.device(self.device):
-                    torch.cuda.synchronize()
+                    # waits for the device before it frees
                     _lib._lib.decon_conv_destroy(h)
             except Exception:
                 pass

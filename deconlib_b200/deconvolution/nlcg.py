@@ -75,7 +75,7 @@ class _Scalars:
         h = getattr(self, "h", None)
         if h is not None and h.value and _lib._lib is not None:
             try:
-                torch.cuda.synchronize()
+                # waits for the device before it frees
                 _lib._lib.decon_nlcg_destroy(h)
             except Exception:
                 pass

@@ -76,7 +76,7 @@ class _Scalars:
 
     def __del__(self):
         if getattr(self, "h", None) is not None and _lib._lib is not None:
-            torch.cuda.synchronize()
+            # waits for the device before it frees
             _lib._lib.decon_pdhg_destroy(self.h)
 
 
@@ -314,7 +314,7 @@ class _State:
     def __del__(self):
         if getattr(self, "h", None) is not None and _lib._lib is not None:
             try:
-                torch.cuda.synchronize()
+                # waits for the device before it frees
                 _lib._lib.decon_pdhg_destroy(self.h)
             except Exception:
                 pass

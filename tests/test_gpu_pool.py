@@ -1,0 +1,40 @@
+"""Plans that go away while a stream is being captured: the capture is not
+disturbed (the wait before memory is freed must not be one that ends it)."""
+
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed", "global"])
+@pytest.mark.parametrize("same_thread", [False, True])
+def test_plan_destroyed_during_a_capture(mode, same_thread):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import deconlib_b200.deconvolution as D
+
+    psf = np.random.default_rng(0).random((3, 5, 5)).astype(np.float32)
+    plans = [D.LinearFFTConvolver(psf, (16, 32, 32)) for _ in range(2)]
+    y = plans[0].forward(torch.ones((16, 32, 32), device="cuda"))
+    x = torch.zeros(64, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode=mode):
+        x += 1
+        if same_thread:
+            plans.clear()
+        else:
+            t = threading.Thread(target=plans.clear)
+            t.start()
+            t.join()
+        x += 2
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(x, torch.full_like(x, 3))
+    # a plan made from that memory
+    z = D.LinearFFTConvolver(psf, (16, 32, 32)).forward(torch.ones((16, 32, 32), device="cuda"))
+    assert torch.equal(y, z)
