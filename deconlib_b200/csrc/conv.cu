@@ -469,20 +469,18 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
     return launch(fn, nblk, nthr, smem, st, &a, PROF_XC2R);
 }
 
+// Found once, by the first thread that asks; the others wait for it.
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
+    static const PFN_cuTensorMapEncodeTiled_v12000 enc = [] {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            enc = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-        else
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-    }
+            fn = nullptr;
+        }
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    }();
     return enc;
 }
 

@@ -5,6 +5,10 @@ so per-row values keep their bits wherever the kernels are the same, and sums
 over a volume change by the order of their FP64 additions only.
 """
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -41,3 +45,34 @@ def test_loss_under_half_lines(D, sig, fft):
     # 6e6 terms of one sign in another order: below 6e6 eps64 of the sum
     assert len(a.loss_history) == 2
     np.testing.assert_allclose(a.loss_history, b.loss_history, rtol=1e-9)
+
+
+FIRST_PLANS = """
+import threading
+import numpy as np, torch
+import deconlib_b200.deconvolution as D
+
+psf = np.random.default_rng(0).random((5, 9, 9)).astype(np.float32)
+x = torch.rand((40, 100, 90), device="cuda")
+torch.cuda.synchronize()
+gate, plans = threading.Barrier(12), [None] * 12
+
+def make(i):
+    gate.wait()
+    plans[i] = D.LinearFFTConvolver(psf, (40, 100, 90))
+
+threads = [threading.Thread(target=make, args=(i,)) for i in range(12)]
+for t in threads:
+    t.start()
+for t in threads:
+    t.join()
+y = D.LinearFFTConvolver(psf, (40, 100, 90)).forward(x)
+assert all(torch.equal(p.forward(x), y) for p in plans)
+"""
+
+
+def test_first_plans_of_a_process_by_several_threads(D):
+    # every thread's plan gets the kernels of a plan made alone: the same bits
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for _ in range(3):
+        subprocess.run([sys.executable, "-c", FIRST_PLANS], check=True, timeout=120, cwd=root)
