@@ -138,8 +138,9 @@ int max_abs2(const float2* z, int64_t rows, int64_t cols, int64_t pitch, double*
 
 }  // namespace dk
 
+// The partials and one result (decon_rl_mask).
 extern "C" int64_t decon_reduce_workspace_bytes(void) {
-    return dk::reduce_partials_needed() * (int64_t)sizeof(double);
+    return (dk::reduce_partials_needed() + 1) * (int64_t)sizeof(double);
 }
 
 extern "C" int decon_reduce(const float* a, const float* b, int64_t n, int op, double* out,

@@ -909,7 +909,7 @@ int decon_rl_mask(float* x, float* sens, int64_t n, void* workspace, void* strea
     const cudaStream_t s = as_stream(stream);
     double* ws = static_cast<double*>(workspace);
     // the max lands in ws[0]; partials use the rest
-    DK_TRY(reduce_f32(sens, nullptr, n, DECON_RED_MAX, ws, ws + 1, reduce_partials_needed() - 1, s));
+    DK_TRY(reduce_f32(sens, nullptr, n, DECON_RED_MAX, ws, ws + 1, reduce_partials_needed(), s));
     DK_TRY(chain(k_rl_mask_generic, g1(n), 256, 0, s, x, sens, ws, n));
     DK_LAUNCHED();
     return DECON_OK;

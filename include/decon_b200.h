@@ -328,7 +328,8 @@ int decon_batch_destroy(decon_batch* b);
  *   decon_rl_update: x = max(x * (sens>0 ? corr/sens : 0), 1e-10) (:149-150)
  *   decon_rl_data_floor: out = max(y - b, 1e-6) (:123)
  *   decon_rl_mask:   floor = max(max(sens) 1e-6, 1e-10); sens = active ? sens
- *                    : 0; x = active ? max(x, 1e-6) : 0 (:125-133). */
+ *                    : 0; x = active ? max(x, 1e-6) : 0 (:125-133); needs a
+ *                    workspace of decon_reduce_workspace_bytes(). */
 int decon_rl_ratio(const float* model, const float* observed, float background, float* ratio,
                    int64_t n, double* loss_sum, void* workspace, void* stream);
 int decon_rl_update(float* x, const float* corr, const float* sens_masked, int64_t n, void* stream);
@@ -522,7 +523,8 @@ int decon_gradient3d_adjoint(const float* g, float* x, const int64_t shape[3], f
 #define DECON_RED_DIFFSQ 2   /* sum (a - b)^2                  */
 #define DECON_RED_MAX 3      /* max a                          */
 #define DECON_RED_DOT 4      /* sum a b                        */
-/* Bytes of device workspace decon_reduce needs (per concurrent call). */
+/* Bytes of device workspace decon_reduce, decon_rl_ratio and decon_rl_mask need
+ * (per concurrent call). */
 int64_t decon_reduce_workspace_bytes(void);
 /* out[0] (device double) = reduction over n elements of a (and b).  Two
  * fixed-shape passes, so the result is bitwise reproducible run to run.
