@@ -282,13 +282,15 @@ constexpr int small_radix(int L, int most = 40) {
 #define DK_PAIR_LENGTHS_E(X) \
     X(640) X(648) X(675) X(720) X(729) X(750) X(768) X(800) X(810) X(864) X(900) X(960) X(972) X(1000) X(1024)
 
-// X lines: even Fx = 2 L up to 1024, and the odd 5-smooth Fx.
+// X lines: even Fx = 2 L up to 2048, and the odd 5-smooth Fx.
 #define DK_XREG_LENGTHS_a(X) \
     X(16) X(18) X(20) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(45) X(48) X(50) X(54) X(60) X(64) X(72)
 #define DK_XREG_LENGTHS_b(X) X(75) X(80) X(81) X(90) X(96) X(100) X(108) X(120) X(125) X(128) X(135) X(144) X(150)
 #define DK_XREG_LENGTHS_c(X) X(160) X(162) X(180) X(192) X(200) X(216) X(225) X(240) X(243) X(250)
 #define DK_XREG_LENGTHS_d(X) X(256) X(270) X(288) X(300) X(320) X(324) X(360) X(375)
 #define DK_XREG_LENGTHS_e(X) X(384) X(400) X(405) X(432) X(450) X(480) X(486) X(500) X(512)
+#define DK_XREG_LENGTHS_f(X) X(540) X(576) X(600) X(625) X(640) X(648) X(675) X(720) X(729) X(750)
+#define DK_XREG_LENGTHS_g(X) X(768) X(800) X(810) X(864) X(900) X(960) X(972) X(1000) X(1024)
 #define DK_XREG_LENGTHS_odd(X) \
     X(25) X(27) X(45) X(75) X(81) X(125) X(135) X(225) X(243) X(375) X(405) X(625) X(675) X(729)
 

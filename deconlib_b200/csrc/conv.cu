@@ -248,7 +248,8 @@ namespace dk {
 #define DK_XREG_PICK(kind)                                        \
     static XRegKernel pick_xreg_##kind(int L, bool odd, int what) { \
         if (odd) return xreg_##kind##_odd(L, what);                 \
-        for (auto group : {xreg_##kind##_a, xreg_##kind##_b, xreg_##kind##_c, xreg_##kind##_d, xreg_##kind##_e}) { \
+        for (auto group : {xreg_##kind##_a, xreg_##kind##_b, xreg_##kind##_c, xreg_##kind##_d, xreg_##kind##_e, xreg_##kind##_f, \
+                           xreg_##kind##_g}) { \
             const XRegKernel k = group(L, what);                    \
             if (k.fn) return k;                                     \
         }                                                           \

@@ -23,10 +23,26 @@
 
 namespace dk {
 
+// The radix S of which a thread holds two butterflies: the most equal pair with S
+// at most 20 (odd lines: 27, one register set per pair of rows), and above 512
+// points at most 24, then 32, where 20 leaves no pair: the fewer registers, the
+// more lines per SM (800 points as 20 x 40 instead of 25 x 32: R2C of 32768 rows 118 ->
+// 88 us, C2R 135 -> 108; 960 as 24 x 40 instead of 30 x 32: 139 -> 108, 148 -> 131).
+// Against the runtime-radix passes: 640 points 279 -> 71 and 311 -> 89 us, 1024
+// points 381 -> 144 and 410 -> 164.
+constexpr int xreg_radix(int L, bool odd) {
+    if (odd) return small_radix(L, 27);
+    for (int most : {20, 24, 32}) {
+        const int s = small_radix(L, most);
+        if (s != 0 || L <= 512) return s;
+    }
+    return 0;
+}
+
 // Lines, threads and exchange layout of a CTA.
 template <int L, bool ODD>
 struct XRegShape {
-    static constexpr int S = small_radix(L, ODD ? 27 : 20), B = L / S;
+    static constexpr int S = xreg_radix(L, ODD), B = L / S;
     static constexpr int TPL = B / 2 + 1;  // threads per line in the paired stage
     static constexpr int TL = 32 * TPL <= 160 ? 32 : (16 * TPL <= 160 ? 16 : (8 * TPL <= 160 ? 8 : 4));
     static constexpr int NT = (TL * TPL + 31) / 32 * 32;
