@@ -315,9 +315,9 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
         delete p;
         return st;
     }
-    // DECON_NO_TMA=1: the plain-load column kernels
-    p->reg_ok = getenv("DECON_NO_TMA") == nullptr;
-    if (p->reg_ok) make_col_passes(*p);
+    // DECON_NO_TMA=1: column passes with plain loads
+    p->tma = getenv("DECON_NO_TMA") == nullptr;
+    make_col_passes(*p);
     if ((st = build_otf(p, kernel, normalize, s))) {
         free_plan(p);
         delete p;
@@ -411,7 +411,9 @@ int decon_conv_set_schedule(decon_conv* p, int sched) {
         cudaStreamDestroy(s);
         DK_TRY(e);
     }
+    const bool remake = ((p->sched ^ sched) & DECON_SCHED_NO_TMA) != 0;
     p->sched = sched;
+    if (remake) make_col_passes(*p);
     return DECON_OK;
 }
 

@@ -75,7 +75,10 @@ __device__ __forceinline__ void gather_rows(V* sm, const V* __restrict__ src, in
     }
 }
 
-template <int L, int MODE>
+// PLAIN: every tile by plain loads (a plan without tensor maps); nfull tiles of a
+// plane's rem columns.  A kernel of its own: as a run-time choice it cost the TMA
+// path 0.5-1.5 %.
+template <int L, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>::blocks)
     k_colreg(const __grid_constant__ ColRegArgs a) {
     using S = ColRegShape<L, MODE>;
@@ -118,20 +121,21 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
             else tma_load_3d(ot + r0 * row, &a.otfmap, c0 * cs, o, r0, &obar);
         }
     };
-    if (tid == 0 && (int)blockIdx.x < a.nmain) {
+    if (!PLAIN && tid == 0 && (int)blockIdx.x < a.nmain) {
         issue(blockIdx.x);
         if constexpr (OTF) issue_otf(blockIdx.x);
     }
 
     uint32_t ph = 0;
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, ph ^= 1) {
-        const bool main = tile < a.nmain;
-        const bool more = tile + (int)gridDim.x < a.nmain;
+        const bool main = !PLAIN && tile < a.nmain;
+        const bool more = !PLAIN && tile + (int)gridDim.x < a.nmain;
         int o, kx;
         bool ok = true;
-        if (main) {
+        if (main || PLAIN) {
             o = tile / a.nfull;
             kx = (tile - o * a.nfull) * T + t;
+            if constexpr (PLAIN) ok = kx < a.rem;
         } else {
             const int p = t / a.rem;
             o = (tile - a.nmain) * a.per + p;
@@ -235,19 +239,21 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
 }
 
 template <int L, int MODE>
-ColRegKernel colreg_one() {
+ColRegKernel colreg_one(bool plain) {
     using S = ColRegShape<L, MODE>;
-    return ColRegKernel{(void*)k_colreg<L, MODE>, S::T, S::NT, S::exch};
+    if constexpr (MODE != CR_OTF16)
+        if (plain) return ColRegKernel{(void*)k_colreg<L, MODE, true>, S::T, S::NT, S::exch};
+    return ColRegKernel{(void*)k_colreg<L, MODE, false>, S::T, S::NT, S::exch};
 }
 
 template <int L>
-ColRegKernel colreg_kernel(int mode) {
+ColRegKernel colreg_kernel(int mode, bool plain) {
     switch (mode) {
-        case CR_FWD: return colreg_one<L, CR_FWD>();
-        case CR_INV: return colreg_one<L, CR_INV>();
-        case CR_OTF: return colreg_one<L, CR_OTF>();
+        case CR_FWD: return colreg_one<L, CR_FWD>(plain);
+        case CR_INV: return colreg_one<L, CR_INV>(plain);
+        case CR_OTF: return colreg_one<L, CR_OTF>(plain);
         case CR_OTF16:
-            if constexpr (L == 64 || L == 128 || L == 256) return colreg_one<L, CR_OTF16>();
+            if constexpr (L == 64 || L == 128 || L == 256) return colreg_one<L, CR_OTF16>(false);
     }
     return ColRegKernel{};
 }

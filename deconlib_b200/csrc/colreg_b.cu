@@ -3,8 +3,8 @@
 
 namespace dk {
 
-ColRegKernel colreg_group_b(int L, int mode) {
-#define DK_CASE(n) if (L == n) return colreg_kernel<n>(mode);
+ColRegKernel colreg_group_b(int L, int mode, bool plain) {
+#define DK_CASE(n) if (L == n) return colreg_kernel<n>(mode, plain);
     DK_PAIR_LENGTHS_B(DK_CASE)
 #undef DK_CASE
     return ColRegKernel{};

@@ -293,8 +293,8 @@ int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cva
                 int64_t nz_rows, float2* out, cudaStream_t st, int64_t kstride) {
     const int src = pro == PRO_KERNEL ? 2 : pro == PRO_UP2 ? 1 : 0;
     const bool full = pro == PRO_KERNEL || pro == PRO_UP2 || is_full_window(p, win);
-    const XRegKernel k = p.reg_ok && kstride == 0 && (full || pro == PRO_ARRAY) ? pick_xreg_r2c(p.ax_x.L, p.odd, src)
-                                                                                : XRegKernel{};
+    const XRegKernel k = kstride == 0 && (full || pro == PRO_ARRAY) ? pick_xreg_r2c(p.ax_x.L, p.odd, src)
+                                                                    : XRegKernel{};
     if (k.fn) {
         const int64_t Ny = pro == PRO_KERNEL ? p.F[1] : p.N[1], Nx = pro == PRO_KERNEL ? p.F[2] : p.N[2];
         XRegArgs a = xreg_args(p, nz_rows * Ny, Ny, Nx, win, full);
@@ -397,8 +397,8 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
                 const float* aux0, const float* aux1, float bg, double* partials, int* nblk_out,
                 cudaStream_t st) {
     const bool full = is_full_window(p, win);
-    const XRegKernel k = p.reg_ok && !use_yz(p) && (full || epi == EPI_STORE) ? pick_xreg_c2r(p.ax_x.L, p.odd, epi)
-                                                                              : XRegKernel{};
+    const XRegKernel k = !use_yz(p) && (full || epi == EPI_STORE) ? pick_xreg_c2r(p.ax_x.L, p.odd, epi)
+                                                                  : XRegKernel{};
     if (k.fn) {
         if (epi == EPI_DOWN2 && (p.odd || (p.N[0] | p.N[1] | p.N[2]) & 1))
             return fail(DECON_ERR_UNSUPPORTED, "2x area-sum epilogue: extents must be even");
@@ -504,14 +504,17 @@ bool encode_tile_map(CUtensorMap* map, const void* base, int esize, int64_t pitc
 // register column passes (colreg.cuh)
 // ---------------------------------------------------------------------------
 
+// DECON_NO_TMA / DECON_SCHED_NO_TMA: plain loads (and the FP32 OTF for a mixed plan).
+static bool no_tma(const ConvPlan& p) { return !p.tma || (p.sched & DECON_SCHED_NO_TMA) != 0; }
+
 // DECON_NO_PIPE / DECON_SCHED_NO_PIPE: the FP32 OTF also for a mixed plan.
 static bool no_pipe(const ConvPlan& p) {
     return getenv("DECON_NO_PIPE") != nullptr || (p.sched & DECON_SCHED_NO_PIPE) != 0;
 }
 
-static ColRegKernel pick_colreg(int L, int mode) {
+static ColRegKernel pick_colreg(int L, int mode, bool plain) {
     for (auto group : {colreg_group_a, colreg_group_b, colreg_group_c, colreg_group_d, colreg_group_e}) {
-        const ColRegKernel k = group(L, mode);
+        const ColRegKernel k = group(L, mode, plain);
         if (k.fn) return k;
     }
     return ColRegKernel{};
@@ -530,8 +533,8 @@ static void split_rows(int n, int row_bytes, int* box, int* nbox) {
 static bool make_col_pass(const ConvPlan& p, ColPass& c, const Axis& ax, int mode, int jdim,
                           const float2* src, int64_t s1, int64_t s2, int nin, float2* dst, int64_t d1,
                           int nout, int64_t nouter) {
-    c.ok = false;
-    c.k = pick_colreg(ax.L, mode);
+    c.ok = c.maps = false;
+    c.k = pick_colreg(ax.L, mode, false);
     if (!c.k.fn) return false;
     ColRegArgs& a = c.a;
     memset(&a, 0, sizeof(a));
@@ -552,14 +555,10 @@ static bool make_col_pass(const ConvPlan& p, ColPass& c, const Axis& ax, int mod
     a.nfull = (int)(p.Hx / T);
     a.rem = (int)(p.Hx - (int64_t)a.nfull * T);
     a.per = a.rem ? T / a.rem : 1;
-    const int64_t nmain = nouter * a.nfull, ntiles = nmain + (a.rem ? cdiv(nouter, a.per) : 0);
-    if (ntiles > 0x7fffffffLL - 65536) return false;
-    a.nmain = (int)nmain;
-    a.ntiles = (int)ntiles;
     split_rows(nin, T * 8, &a.box, &a.nbox);
     a.in_bytes = a.nbox * a.box * T * 8;
-    if (!encode_tile_map(&a.srcmap, src, 8, p.P, s1, s2, T, jdim == 1 ? a.box : 1, jdim == 1 ? 1 : a.box))
-        return false;
+    bool maps = !no_tma(p) && encode_tile_map(&a.srcmap, src, 8, p.P, s1, s2, T, jdim == 1 ? a.box : 1,
+                                              jdim == 1 ? 1 : a.box);
     c.smem = c.k.exch + a.in_bytes;
     if (mode == 2 || mode == 3) {
         const int esize = mode == 3 ? 4 : 8;
@@ -569,11 +568,22 @@ static bool make_col_pass(const ConvPlan& p, ColPass& c, const Axis& ax, int mod
         a.otf_os = jdim == 1 ? p.F[1] * p.P : p.P;
         a.otf_js = jdim == 1 ? p.P : p.F[1] * p.P;
         split_rows(ax.L, T * esize, &a.obox, &a.onbox);
-        if (!encode_tile_map(&a.otfmap, mode == 3 ? (const void*)p.otf16 : (const void*)p.otf, esize, p.P,
-                             p.F[1], p.F[0], T, jdim == 1 ? a.obox : 1, jdim == 1 ? 1 : a.obox))
-            return false;
+        maps = maps && encode_tile_map(&a.otfmap, mode == 3 ? (const void*)p.otf16 : (const void*)p.otf, esize,
+                                       p.P, p.F[1], p.F[0], T, jdim == 1 ? a.obox : 1, jdim == 1 ? 1 : a.obox);
         c.smem += a.onbox * a.obox * T * esize;
     }
+    int64_t nmain = nouter * a.nfull, ntiles = nmain + (a.rem ? cdiv(nouter, a.per) : 0);
+    if (!maps) {
+        if (mode == 3) return false;
+        c.k = pick_colreg(ax.L, mode, true);
+        a.nfull = (int)cdiv(p.Hx, T);
+        a.rem = (int)p.Hx;
+        nmain = 0;
+        ntiles = nouter * a.nfull;
+    }
+    if (ntiles > 0x7fffffffLL - 65536) return false;
+    a.nmain = (int)nmain;
+    a.ntiles = (int)ntiles;
     void* flag = nullptr;
     int per_sm = 0;
     if (c.smem > 227 * 1024 || cudaGetSymbolAddress(&flag, g_wait_timeout) != cudaSuccess ||
@@ -583,6 +593,7 @@ static bool make_col_pass(const ConvPlan& p, ColPass& c, const Axis& ax, int mod
     }
     a.flag = static_cast<int*>(flag);
     c.grid = (int)std::min<int64_t>(ntiles, (int64_t)sm_count() * per_sm);
+    c.maps = maps;
     return c.ok = true;
 }
 
@@ -602,7 +613,7 @@ void make_z_otf16(ConvPlan& p) {
     make_col_pass(p, p.z_otf16, p.ax_z, 3, 2, p.s2, Fy, Nz, (int)Nz, p.s2, Fy, (int)Nz, Fy);
 }
 
-static int launch_col_pass(const ConvPlan&, const ColPass& c, bool conj, cudaStream_t st) {
+static int launch_col_pass(const ColPass& c, bool conj, cudaStream_t st) {
     ColRegArgs a = c.a;
     if (conj) a.conj = -1.f;
     return launch_chained(c.k.fn, dim3((unsigned)c.grid), c.k.nt, c.smem, true, st, &a, a.otf ? PROF_ZOTF : PROF_COL);
@@ -613,16 +624,15 @@ int transform_otf(const ConvPlan& p, int axis, cudaStream_t st) {
     const int n = (int)p.F[axis];
     const Axis& ax = axis == 1 ? p.ax_y : p.ax_z;
     ColPass c;
-    if (p.reg_ok && make_col_pass(p, c, ax, 0, axis == 1 ? 1 : 2, p.otf, Fy, Fz, n, p.otf, Fy, n,
-                                  axis == 1 ? Fz : Fy))
-        return launch_col_pass(p, c, false, st);
+    if (make_col_pass(p, c, ax, 0, axis == 1 ? 1 : 2, p.otf, Fy, Fz, n, p.otf, Fy, n, axis == 1 ? Fz : Fy))
+        return launch_col_pass(c, false, st);
     if (axis == 1)
         return launch_col(p, ax, p.T_y, COL_FWD, p.otf, Fy * P, P, n, p.otf, Fy * P, P, n, Fz, st);
     return launch_col(p, ax, p.T_z, COL_FWD, p.otf, P, Fy * P, n, p.otf, P, Fy * P, n, Fy, st);
 }
 
 bool zpass_pipelined(const ConvPlan& p) {
-    if (!p.z_otf.ok || no_pipe(p) || (p.sched & DECON_SCHED_NO_TMA)) return false;
+    if (!p.z_otf.maps || no_pipe(p)) return false;
     const int L = p.ax_z.L;
     return L == 64 || L == 256 || (L == 128 && p.N[0] <= 64);
 }
@@ -785,7 +795,7 @@ static int launch_yz(const ConvPlan& p, bool adjoint, cudaStream_t st) {
     return DECON_OK;
 }
 
-static bool one_plane(const ConvPlan& p) { return p.y_otf.ok && !(p.sched & DECON_SCHED_NO_TMA); }
+static bool one_plane(const ConvPlan& p) { return p.y_otf.ok; }
 
 // Forward spectrum: x (window in N-space) -> S2 (after the Y pass), or, with
 // the fused Y / axial pass, -> the kx-major S1 (X pass only).
@@ -795,8 +805,8 @@ int spectrum_forward(const ConvPlan& p, int pro, const float* in, Win3 win, floa
     if (use_yz(p)) return launch_xr2c(p, pro, in, win, cval, bg, Nz, p.s1, st, Nz * Ny);
     DK_TRY(launch_xr2c(p, pro, in, win, cval, bg, Nz, p.s1, st));
     if (one_plane(p)) return DECON_OK;  // the Y transforms run with the product (spectrum_filter_back)
-    if (p.y_fwd.ok && !(p.sched & DECON_SCHED_NO_TMA)) {
-        DK_TRY(launch_col_pass(p, p.y_fwd, false, st));
+    if (p.y_fwd.ok) {
+        DK_TRY(launch_col_pass(p.y_fwd, false, st));
     } else {
         DK_TRY(launch_col(p, p.ax_y, p.T_y, COL_FWD, p.s1, Ny * P, P, (int)Ny, p.s2, Fy * P, P,
                           (int)Fy, Nz, st));
@@ -807,19 +817,18 @@ int spectrum_forward(const ConvPlan& p, int pro, const float* in, Win3 win, floa
 // Z pass (x OTF or conj OTF) and the inverse Y pass: S2 -> S1.
 int spectrum_filter_back(const ConvPlan& p, bool adjoint, cudaStream_t st) {
     if (use_yz(p)) return launch_yz(p, adjoint, st);
-    if (one_plane(p)) return launch_col_pass(p, p.y_otf, adjoint, st);
+    if (one_plane(p)) return launch_col_pass(p.y_otf, adjoint, st);
     const int64_t Nz = p.N[0], Ny = p.N[1], Fy = p.F[1], P = p.P;
     const int mode = adjoint ? COL_OTF_CONJ : COL_OTF;
-    const bool reg = !(p.sched & DECON_SCHED_NO_TMA);
-    if (p.z_otf.ok && reg) {
-        const bool h16 = p.precision == 1 && p.z_otf16.ok && !no_pipe(p);
-        DK_TRY(launch_col_pass(p, h16 ? p.z_otf16 : p.z_otf, adjoint, st));
+    if (p.z_otf.ok) {
+        const bool h16 = p.precision == 1 && p.z_otf16.ok && p.z_otf.maps && !no_pipe(p);
+        DK_TRY(launch_col_pass(h16 ? p.z_otf16 : p.z_otf, adjoint, st));
     } else {
         DK_TRY(launch_col(p, p.ax_z, p.T_z, mode, p.s2, P, Fy * P, (int)Nz, p.s2, P, Fy * P,
                           (int)Nz, Fy, st));
     }
-    if (p.y_inv.ok && reg) {
-        DK_TRY(launch_col_pass(p, p.y_inv, false, st));
+    if (p.y_inv.ok) {
+        DK_TRY(launch_col_pass(p.y_inv, false, st));
     } else {
         DK_TRY(launch_col(p, p.ax_y, p.T_y, COL_INV, p.s2, Fy * P, P, (int)Fy, p.s1, Ny * P, P,
                           (int)Ny, Nz, st));

@@ -115,13 +115,13 @@ struct ColPass {
     ColRegKernel k;
     ColRegArgs a;
     int smem = 0, grid = 0;
-    bool ok = false;
+    bool ok = false, maps = false;  // maps: the rows come by TMA
 };
-ColRegKernel colreg_group_a(int L, int mode);
-ColRegKernel colreg_group_b(int L, int mode);
-ColRegKernel colreg_group_c(int L, int mode);
-ColRegKernel colreg_group_d(int L, int mode);
-ColRegKernel colreg_group_e(int L, int mode);
+ColRegKernel colreg_group_a(int L, int mode, bool plain);
+ColRegKernel colreg_group_b(int L, int mode, bool plain);
+ColRegKernel colreg_group_c(int L, int mode, bool plain);
+ColRegKernel colreg_group_d(int L, int mode, bool plain);
+ColRegKernel colreg_group_e(int L, int mode, bool plain);
 
 // Register X passes (xreg.cuh).
 struct XRegArgs {
@@ -197,7 +197,7 @@ struct ConvPlan {
     // S1 -> S2, axial in S2 (FP32 and FP16 OTF), Y inverse S2 -> S1; one plane
     // (Fz = 1, images): Y forward, product and Y inverse in one pass over S1
     ColPass y_fwd, z_otf, z_otf16, y_inv, y_otf;
-    bool reg_ok = false;
+    bool tma = true;  // tensor maps (DECON_NO_TMA was not set when the plan was made)
     // Mixed precision (decon_conv_set_precision): the OTF also stored as FP16
     // complex, scaled per kz plane by a power of two (OTF = otf16 * otf_inv[kz]),
     // read by the pipelined axial pass instead of the FP32 OTF.

@@ -112,8 +112,9 @@ int decon_conv_norm_sq(const decon_conv* plan, double* out);
  *                (allocates the kx-major OTF copy on first request; DECON_YZ=1
  *                selects it for every plan)
  *   NO_PIPE      the FP32 OTF for a plan set to mixed precision; no effect else
- *   NO_TMA       runtime-radix kernels with plain loads instead of the register
- *                kernels (no tensor maps)
+ *   NO_TMA       plain loads instead of TMA copies in the register column passes
+ *                (no tensor maps; the same bits), and the FP32 OTF for a plan set
+ *                to mixed precision
  *   LEAN_OFF     no effect (kept for saved schedules)
  *   ODD_RADIX    radix plans with the 5 / 3 / 7 stages first (runtime-radix axes)
  *   HALF_LINES   half the lines per CTA on runtime-radix axes (more, smaller CTAs) */

@@ -15,7 +15,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-HALF_LINES = 32
+NO_TMA, HALF_LINES = 4, 32
 
 
 @pytest.fixture(scope="module")
@@ -76,3 +76,22 @@ def test_first_plans_of_a_process_by_several_threads(D):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     for _ in range(3):
         subprocess.run([sys.executable, "-c", FIRST_PLANS], check=True, timeout=120, cwd=root)
+
+
+# tiles of 16 and 8 columns, whole and with planes side by side, one plane, short
+# and 1024-point axes, and a 7-smooth one (runtime radices on every schedule)
+@pytest.mark.parametrize("sig,fft", [((20, 40, 60), (40, 80, 120)), ((8, 9, 9), (16, 18, 18)), ((70, 180, 33), (135, 360, 64)),
+                                     ((1, 300, 100), (1, 600, 200)), ((5, 30, 500), (10, 60, 1000)),
+                                     ((3, 500, 30), (16, 1024, 48)), ((500, 9, 30), (1000, 18, 50)), ((10, 20, 30), (20, 42, 60))])
+def test_plain_loads_give_the_same_bits(D, monkeypatch, sig, fft):
+    rng = np.random.default_rng(1)
+    psf = rng.random(tuple(f - n + 1 for n, f in zip(sig, fft))).astype(np.float32)
+    x = torch.from_numpy(rng.random(sig).astype(np.float32)).cuda()
+    c = D.LinearFFTConvolver(psf, sig, fft_shape=fft)
+    y, z = c.forward(x), c.adjoint(x)
+    c.set_schedule(NO_TMA)
+    assert torch.equal(c.forward(x), y) and torch.equal(c.adjoint(x), z)
+    monkeypatch.setenv("DECON_NO_TMA", "1")
+    p = D.LinearFFTConvolver(psf, sig, fft_shape=fft)
+    assert torch.equal(p.otf, c.otf)
+    assert torch.equal(p.forward(x), y) and torch.equal(p.adjoint(x), z)
