@@ -22,7 +22,7 @@ SOURCES = ["capi.cu", "pool.cu", "conv.cu", "reduce.cu", "ops.cu", "solvers.cu",
            "fftplain.cu",
            "colreg_a.cu", "colreg_b.cu", "colreg_c.cu", "colreg_d.cu", "colreg_e.cu",
            "psf_any.cu", "psf_a.cu", "psf_b.cu", "psf_c.cu", "psf_d.cu", "psf_e.cu",
-           *(f"xreg_{d}_{g}.cu" for g in ("g", "f", "e", "d", "c", "b", "a", "odd") for d in ("c2r", "r2c"))]
+           *(f"xreg_{d}_{g}.cu" for g in ("g", "f", "e", "d", "c", "b", "a", "odd", "kx") for d in ("c2r", "r2c"))]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

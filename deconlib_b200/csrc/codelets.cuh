@@ -291,6 +291,10 @@ constexpr int small_radix(int L, int most = 40) {
 #define DK_XREG_LENGTHS_e(X) X(384) X(400) X(405) X(432) X(450) X(480) X(486) X(500) X(512)
 #define DK_XREG_LENGTHS_f(X) X(540) X(576) X(600) X(625) X(640) X(648) X(675) X(720) X(729) X(750)
 #define DK_XREG_LENGTHS_g(X) X(768) X(800) X(810) X(864) X(900) X(960) X(972) X(1000) X(1024)
+// kx-major spectrum (the fused Y / axial pass): 2^a x {1, 3, 5, 15}, the lengths
+// that had compile-time kernels for it; the others run on runtime radices.
+#define DK_XREG_LENGTHS_kx(X) \
+    X(64) X(80) X(96) X(128) X(160) X(192) X(240) X(256) X(320) X(384) X(480) X(512) X(640) X(768) X(960) X(1024)
 #define DK_XREG_LENGTHS_odd(X) \
     X(25) X(27) X(45) X(75) X(81) X(125) X(135) X(225) X(243) X(375) X(405) X(625) X(675) X(729)
 

@@ -245,15 +245,16 @@ extern "C" int decon_profile_stop(double* ms_total, int64_t* launches) {
 
 namespace dk {
 
-#define DK_XREG_PICK(kind)                                        \
-    static XRegKernel pick_xreg_##kind(int L, bool odd, int what) { \
-        if (odd) return xreg_##kind##_odd(L, what);                 \
-        for (auto group : {xreg_##kind##_a, xreg_##kind##_b, xreg_##kind##_c, xreg_##kind##_d, xreg_##kind##_e, xreg_##kind##_f, \
-                           xreg_##kind##_g}) { \
-            const XRegKernel k = group(L, what);                    \
-            if (k.fn) return k;                                     \
-        }                                                           \
-        return XRegKernel{};                                        \
+#define DK_XREG_PICK(kind) \
+    static XRegKernel pick_xreg_##kind(int L, bool odd, bool kx, int what) { \
+        if (kx) return odd ? XRegKernel{} : xreg_##kind##_kx(L, what); \
+        if (odd) return xreg_##kind##_odd(L, what); \
+        for (auto group : {xreg_##kind##_a, xreg_##kind##_b, xreg_##kind##_c, xreg_##kind##_d, xreg_##kind##_e, \
+                           xreg_##kind##_f, xreg_##kind##_g}) { \
+            const XRegKernel k = group(L, what); \
+            if (k.fn) return k; \
+        } \
+        return XRegKernel{}; \
     }
 DK_XREG_PICK(r2c)
 DK_XREG_PICK(c2r)
@@ -293,8 +294,7 @@ int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cva
                 int64_t nz_rows, float2* out, cudaStream_t st, int64_t kstride) {
     const int src = pro == PRO_KERNEL ? 2 : pro == PRO_UP2 ? 1 : 0;
     const bool full = pro == PRO_KERNEL || pro == PRO_UP2 || is_full_window(p, win);
-    const XRegKernel k = kstride == 0 && (full || pro == PRO_ARRAY) ? pick_xreg_r2c(p.ax_x.L, p.odd, src)
-                                                                    : XRegKernel{};
+    const XRegKernel k = full || pro == PRO_ARRAY ? pick_xreg_r2c(p.ax_x.L, p.odd, kstride != 0, src) : XRegKernel{};
     if (k.fn) {
         const int64_t Ny = pro == PRO_KERNEL ? p.F[1] : p.N[1], Nx = pro == PRO_KERNEL ? p.F[2] : p.N[2];
         XRegArgs a = xreg_args(p, nz_rows * Ny, Ny, Nx, win, full);
@@ -311,6 +311,7 @@ int launch_xr2c(const ConvPlan& p, int pro, const float* in, Win3 win, float cva
         a.py = (p.K[1] + 1) / 2;
         a.px = (p.K[2] + 1) / 2;
         a.out = out;
+        if (kstride) a.P = kstride;
         a.vec = a.wx % 2 == 0 && a.x0 % 2 == 0 && pair_aligned(in);
         return launch(k.fn, cdiv(a.nlines, k.TL), k.nt, k.smem, st, &a, PROF_XR2C);
     }
@@ -397,8 +398,8 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
                 const float* aux0, const float* aux1, float bg, double* partials, int* nblk_out,
                 cudaStream_t st) {
     const bool full = is_full_window(p, win);
-    const XRegKernel k = !use_yz(p) && (full || epi == EPI_STORE) ? pick_xreg_c2r(p.ax_x.L, p.odd, epi)
-                                                                  : XRegKernel{};
+    const int64_t kstride = use_yz(p) ? p.N[0] * p.N[1] : 0;
+    const XRegKernel k = full || epi == EPI_STORE ? pick_xreg_c2r(p.ax_x.L, p.odd, kstride != 0, epi) : XRegKernel{};
     if (k.fn) {
         if (epi == EPI_DOWN2 && (p.odd || (p.N[0] | p.N[1] | p.N[2]) & 1))
             return fail(DECON_ERR_UNSUPPORTED, "2x area-sum epilogue: extents must be even");
@@ -407,6 +408,7 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
         const int64_t rows = full || p.odd ? p.N[0] * p.N[1] : win.wz * win.wy;
         XRegArgs a = xreg_args(p, rows, p.N[1], p.N[2], win, full);
         a.spec = in;
+        if (kstride) a.P = kstride;
         a.out_real = out;
         a.aux0 = aux0;
         a.aux1 = aux1;
@@ -444,7 +446,7 @@ int launch_xc2r(const ConvPlan& p, int epi, const float2* in, Win3 win, float* o
     a.aux1 = aux1;
     a.bg = bg;
     a.partials = partials;
-    a.kstride = use_yz(p) ? p.N[0] * p.N[1] : 0;
+    a.kstride = kstride;
     {
         const int L = a.ax.L;
         a.fd_L = make_fastdiv(L);

@@ -154,7 +154,7 @@ struct XRegKernel {
     void* fn = nullptr;
     int TL = 0, nt = 0, smem = 0;
 };
-#define DK_XREG_GROUPS(X) X(a) X(b) X(c) X(d) X(e) X(f) X(g) X(odd)
+#define DK_XREG_GROUPS(X) X(a) X(b) X(c) X(d) X(e) X(f) X(g) X(odd) X(kx)
 #define DK_XREG_DECL(g)                       \
     XRegKernel xreg_r2c_##g(int L, int src);  \
     XRegKernel xreg_c2r_##g(int L, int epi);

@@ -14,6 +14,11 @@
 //   C2R  stage 1: X[k], X[L - k] -> radix S, butterflies u and B - u
 //        stage 2: radix B -> x, with the element-wise epilogues
 //
+// KX: the kx-major spectrum of the fused Y / axial pass, element (k, row) at
+// k P + row.  Adjacent threads then take adjacent rows in the spectrum stage, 64
+// bytes of a frequency (8 rows) in whole pieces.  A template: as a run-time stride
+// it would cost the row-major passes.
+//
 // The self-paired butterflies (u = 0, and B / 2 for even B) go through the same
 // code: their second half repeats the first and is not stored.
 #pragma once
@@ -100,11 +105,11 @@ __device__ __forceinline__ void prefetch_l2(const void* p, int64_t lo, int64_t h
 }
 
 // Spectrum rows row0 .. row0 + ROWS of zero lines.
-template <int ROWS, int NT>
+template <int ROWS, int NT, bool KX>
 __device__ __forceinline__ void zero_rows(const XRegArgs& a, int64_t row0) {
     const int n = (int)(row0 + ROWS < a.nrows ? ROWS : (int64_t)a.nrows - row0);
     for (int i = 0; i < n; ++i)
-        for (int k = threadIdx.x; k < a.Hx; k += NT) a.out[(row0 + i) * a.P + k] = make_float2(0.f, 0.f);
+        for (int k = threadIdx.x; k < a.Hx; k += NT) a.out[KX ? k * a.P + row0 + i : (row0 + i) * a.P + k] = make_float2(0.f, 0.f);
 }
 
 // Offset of x = 0 of a row in the real array (its window of the volume: elements
@@ -119,7 +124,7 @@ __device__ __forceinline__ int64_t array_row(const XRegArgs& a, uint32_t row) {
     return (int64_t)(iz * (uint32_t)a.wy + iy) * a.wx - a.x0;
 }
 
-template <int L, bool ODD, int SRC>
+template <int L, bool ODD, int SRC, bool KX>
 __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::blocks_for(4 * XRegShape<L, ODD>::S + 44))
     k_xreg_r2c(const XRegArgs a) {
     using H = XRegShape<L, ODD>;
@@ -141,7 +146,7 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
         if (!__syncthreads_or(any)) {
             // the kernel covers a part of the canvas: whole CTAs of zero rows
             // (three quarters of them for a kernel of half the canvas)
-            zero_rows<W * TL, NT>(a, (int64_t)W * line0);
+            zero_rows<W * TL, NT, KX>(a, (int64_t)W * line0);
             return;
         }
         const float sum = a.ksum ? (float)__ldg(a.ksum) : 1.f;
@@ -164,7 +169,7 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
             bool any = false;
             for (int i = tid; i < W * TL; i += NT) any = any || array_row(a, W * line0 + i) != kNoRow;
             if (!__syncthreads_or(any)) {
-                zero_rows<W * TL, NT>(a, (int64_t)W * line0);
+                zero_rows<W * TL, NT, KX>(a, (int64_t)W * line0);
                 return;
             }
         }
@@ -242,9 +247,9 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
     __syncthreads();
 
     // stage 2
-    const int l = tid / TPL, u = tid - l * TPL;
+    const int l = KX ? tid % TL : tid / TPL, u = KX ? tid / TL : tid - l * TPL;
     const uint32_t line = line0 + l;
-    if (l >= TL || line >= a.nlines) return;
+    if ((KX ? u >= TPL : l >= TL) || line >= a.nlines) return;
     C1 va[S], vb[S];
     {
         const float2* e = sm + l * E::pitch;
@@ -267,7 +272,8 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
     if constexpr (!ODD) {
         // X[k] = e + W^k o, X[M-k] = conj(e - W^k o) with e = (Z[k] + conj
         // Z[M-k]) / 2, o = -i (Z[k] - conj Z[M-k]) / 2
-        float2* out = a.out + (int64_t)line * a.P;
+        float2* out = a.out + (KX ? (int64_t)line : (int64_t)line * a.P);
+        const int64_t ks = KX ? a.P : 1;
         const bool second = u > 0 && 2 * u < B;
 #pragma unroll
         for (int r = 0; r < S; ++r) {
@@ -276,8 +282,8 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT, XRegShape<L, ODD>::bloc
             const C1 s = zk + zm, d = zk - zm;
             const C1 e{0.5f * s.re, 0.5f * s.im}, o{0.5f * d.im, -0.5f * d.re};
             const C1 t = twist<false>(o, __ldg(&a.twx[k]));
-            out[k] = as_f2(e + t);
-            if (second || (u == 0 && r == 0)) out[L - k] = as_f2(conj_of(e - t));
+            out[k * ks] = as_f2(e + t);
+            if (second || (u == 0 && r == 0)) out[(L - k) * ks] = as_f2(conj_of(e - t));
         }
     } else {
         // Xa = (Z[k] + conj Z[L-k]) / 2, Xb = -i (Z[k] - conj Z[L-k]) / 2
@@ -411,7 +417,7 @@ __device__ __forceinline__ uint32_t c2r_row(const XRegArgs& a, uint32_t row) {
     }
 }
 
-template <int L, bool ODD, int EPI>
+template <int L, bool ODD, int EPI, bool KX>
 __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
                                   XRegShape<L, ODD>::blocks_for(EPI == EPI_DOWN2 && XRegShape<L, ODD>::B > 12
                                                                     ? 4 * XRegShape<L, ODD>::B + 44
@@ -443,18 +449,19 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
 
     // stage 1
     {
-        const int l = tid / TPL, u = tid - l * TPL;
+        const int l = KX ? tid % TL : tid / TPL, u = KX ? tid / TL : tid - l * TPL;
         const uint32_t line = line0 + l;
-        if (l < TL && line < a.nlines) {
+        if ((KX ? u < TPL : l < TL) && line < a.nlines) {
             C1 va[S], vb[S];
             if constexpr (!ODD) {
                 // Z[k] = e + i d W^-k, Z[M-k] = conj(e) + i conj(d W^-k) with e = X[k] +
                 // conj X[M-k], d = X[k] - conj X[M-k]; irfft ignores Im of DC and Nyquist
-                const float2* in = a.spec + (int64_t)c2r_row<EPI>(a, line) * a.P;
+                const int64_t row = c2r_row<EPI>(a, line), ks = KX ? a.P : 1;
+                const float2* in = a.spec + (KX ? row : row * a.P);
 #pragma unroll
                 for (int r = 0; r < S; ++r) {
-                    va[r] = as_c1(__ldg(in + u + r * B));
-                    vb[r] = as_c1(__ldg(in + L - u - r * B));
+                    va[r] = as_c1(__ldg(in + (u + r * B) * ks));
+                    vb[r] = as_c1(__ldg(in + (L - u - r * B) * ks));
                 }
                 if (u == 0) va[0].im = vb[0].im = 0.f;
 #pragma unroll
@@ -584,33 +591,35 @@ __global__ void __launch_bounds__(XRegShape<L, ODD>::NT,
     }
 }
 
-template <int L, bool ODD>
+template <int L, bool ODD, bool KX = false>
 XRegKernel xreg_r2c_of(int src) {
     using H = XRegShape<L, ODD>;
     constexpr int smem = H::template Ex<H::B>::bytes;
     switch (src) {
-        case XS_ARRAY: return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_ARRAY>, H::TL, H::NT, smem};
+        case XS_ARRAY: return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_ARRAY, KX>, H::TL, H::NT, smem};
         case XS_UP2:
-            if constexpr (!ODD) return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_UP2>, H::TL, H::NT, smem};
+            if constexpr (!ODD) return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_UP2, KX>, H::TL, H::NT, smem};
             break;
         case XS_KERNEL:
-            return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_KERNEL>, H::TL, H::NT,
-                              smem + H::TL * L * (int)sizeof(float2)};
+            if constexpr (!KX)
+                return XRegKernel{(void*)k_xreg_r2c<L, ODD, XS_KERNEL, KX>, H::TL, H::NT,
+                                  smem + H::TL * L * (int)sizeof(float2)};
+            break;
     }
     return XRegKernel{};
 }
 
-template <int L, bool ODD>
+template <int L, bool ODD, bool KX = false>
 XRegKernel xreg_c2r_of(int epi) {
     using H = XRegShape<L, ODD>;
     constexpr int smem = H::template Ex<H::S>::bytes;
     switch (epi) {
-        case EPI_STORE: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_STORE>, H::TL, H::NT, smem};
+        case EPI_STORE: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_STORE, KX>, H::TL, H::NT, smem};
         case EPI_PRED:
-        case EPI_RL_RATIO: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_RL_RATIO>, H::TL, H::NT, smem};
-        case EPI_RL_UPDATE: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_RL_UPDATE>, H::TL, H::NT, smem};
+        case EPI_RL_RATIO: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_RL_RATIO, KX>, H::TL, H::NT, smem};
+        case EPI_RL_UPDATE: return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_RL_UPDATE, KX>, H::TL, H::NT, smem};
         case EPI_DOWN2:
-            if constexpr (!ODD) return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_DOWN2>, H::TL, H::NT, smem};
+            if constexpr (!ODD) return XRegKernel{(void*)k_xreg_c2r<L, ODD, EPI_DOWN2, KX>, H::TL, H::NT, smem};
             break;
     }
     return XRegKernel{};

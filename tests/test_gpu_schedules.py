@@ -15,7 +15,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-NO_TMA, HALF_LINES = 4, 32
+FUSED, NO_TMA, HALF_LINES = 1, 4, 32
 
 
 @pytest.fixture(scope="module")
@@ -95,3 +95,43 @@ def test_plain_loads_give_the_same_bits(D, monkeypatch, sig, fft):
     p = D.LinearFFTConvolver(psf, sig, fft_shape=fft)
     assert torch.equal(p.otf, c.otf)
     assert torch.equal(p.forward(x), y) and torch.equal(p.adjoint(x), z)
+
+
+# X lines with a kx-major kernel of their own, and others (runtime radices)
+@pytest.mark.parametrize("L", [64, 80, 96, 128, 160, 192, 240, 256, 320, 384, 480, 512, 640, 768, 960, 1024, 50, 63, 600])
+def test_fused_pass_at_every_x_length(D, L):
+    # FP32 transforms of the same canvas, factored differently: twice the 1e-6
+    # that the repository allows each of them against FP64
+    sig, fft = (5, 18, L // 2 * 2), (128, 256, 2 * L)
+    rng = np.random.default_rng(L)
+    psf = rng.random((9, 31, L // 2)).astype(np.float32) ** 4
+    x = torch.from_numpy(rng.random(sig).astype(np.float32)).cuda()
+    c0 = D.LinearFFTConvolver(psf, sig, fft_shape=fft)
+    c = D.LinearFFTConvolver(psf, sig, fft_shape=fft, schedule=FUSED)
+    assert c.fused_yz
+    rel = lambda a, b: float((a.double() - b.double()).norm() / b.double().norm())  # noqa: E731
+    assert rel(c.forward(x), c0.forward(x)) < 2e-6 and rel(c.adjoint(x), c0.adjoint(x)) < 2e-6
+    # the same plan's epilogues and windows are the operators in turn, bit for bit
+    crop = D.Crop(sig, (3, 7, L // 2 + 1), start=(1, 2, 3))
+    A = D.compose(crop, c)
+    z = crop.forward(x)
+    assert torch.equal(A.forward(x), crop.forward(c.forward(x)))
+    assert torch.equal(A.adjoint(z), c.adjoint(crop.adjoint(z)))
+    obs = torch.poisson(100 * x)
+    a = D.richardson_lucy_with_operator(obs, c, num_iter=3, background=2.0, eval_interval=1)
+    b = D.richardson_lucy_with_operator(obs, c0, num_iter=3, background=2.0, eval_interval=1)
+    assert rel(a.restored, b.restored) < 1e-5  # as test_gpu_yz.py allows RL
+    np.testing.assert_allclose(a.loss_history, b.loss_history, rtol=1e-6)
+
+
+@pytest.mark.parametrize("L", [64, 80, 240, 256, 640, 1024, 50])
+def test_fused_area_sum_at_x_lengths(D, L):
+    sig, fft = (6, 32, L // 2 * 2), (128, 256, 2 * L)
+    rng = np.random.default_rng(L)
+    c = D.LinearFFTConvolver(rng.random((9, 31, L // 2)).astype(np.float32), sig, fft_shape=fft, schedule=FUSED)
+    down = D.FractionalAreaDownsample(2.0)
+    A = D.compose(down, c)
+    x = torch.from_numpy(rng.random(sig).astype(np.float32)).cuda()
+    y = down.forward(x)
+    assert torch.equal(A.forward(x), down.forward(c.forward(x)))
+    assert torch.equal(A.adjoint(y), c.adjoint(down.adjoint(y)))
