@@ -49,6 +49,7 @@ _SIGS = {
     "decon_conv_norm_sq": (C.c_int, [_p, _dp]),
     "decon_conv_fused_yz": (C.c_int, [_p, C.POINTER(C.c_int)]),
     "decon_conv_set_schedule": (C.c_int, [_p, C.c_int]),
+    "decon_conv_schedule_bits": (C.c_int, [_p, C.POINTER(C.c_int)]),
     "decon_conv_get_schedule": (C.c_int, [_p, C.POINTER(C.c_int)]),
     "decon_conv_shape": (C.c_int, [_p, _i64p, _i64p]),
     "decon_conv_get_otf": (C.c_int, [_p, _p, _p]),

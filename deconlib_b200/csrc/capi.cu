@@ -423,6 +423,12 @@ int decon_conv_get_schedule(const decon_conv* p, int* sched) {
     return DECON_OK;
 }
 
+int decon_conv_schedule_bits(const decon_conv* p, int* bits) {
+    if (!p || !bits) return fail(DECON_ERR_NULL, "null pointer");
+    *bits = schedule_bits(*p);
+    return DECON_OK;
+}
+
 int decon_conv_fused_yz(const decon_conv* p, int* out) {
     if (!p || !out) return fail(DECON_ERR_NULL, "null pointer");
     *out = use_yz(*p) ? 1 : 0;

@@ -799,6 +799,20 @@ static int launch_yz(const ConvPlan& p, bool adjoint, cudaStream_t st) {
 
 static bool one_plane(const ConvPlan& p) { return p.y_otf.ok; }
 
+int schedule_bits(const ConvPlan& p) {
+    const bool yz = use_yz(p);
+    int bits = 0;
+    if (p.precision == 0 && getenv("DECON_NO_YZ") == nullptr && getenv("DECON_YZ") == nullptr &&
+        (p.otft != nullptr || (yz_supported(p.N, p.F) && p.F[0] != p.N[0])))
+        bits |= DECON_SCHED_FUSED;
+    const bool columns = one_plane(p) || (p.y_fwd.ok && p.y_inv.ok && p.z_otf.ok);  // register kernels
+    if (!yz && p.tma && (one_plane(p) || p.y_fwd.ok || p.y_inv.ok || p.z_otf.ok)) bits |= DECON_SCHED_NO_TMA;
+    if (!yz && p.precision == 1 && p.z_otf16.ok) bits |= DECON_SCHED_NO_PIPE;
+    const bool rows = pick_xreg_r2c(p.ax_x.L, p.odd, yz, 0).fn && pick_xreg_c2r(p.ax_x.L, p.odd, yz, EPI_STORE).fn;
+    if (!rows || (!yz && !columns)) bits |= DECON_SCHED_ODD_RADIX | DECON_SCHED_HALF_LINES;
+    return bits;
+}
+
 // Forward spectrum: x (window in N-space) -> S2 (after the Y pass), or, with
 // the fused Y / axial pass, -> the kx-major S1 (X pass only).
 int spectrum_forward(const ConvPlan& p, int pro, const float* in, Win3 win, float cval, float bg,

@@ -225,6 +225,8 @@ int build_otf_kmajor(const ConvPlan& p, cudaStream_t st);
 
 // Quantise p.otf into p.otf16 / p.otf_inv (capi.cu).
 int quantize_otf(const ConvPlan& p, cudaStream_t st);
+// The schedule bits that change a launch of this plan (conv.cu).
+int schedule_bits(const ConvPlan& p);
 // True when this plan's axial pass can take an FP16 OTF (conv.cu).
 bool zpass_pipelined(const ConvPlan& p);
 

@@ -253,6 +253,14 @@ class LinearFFTConvolver:
         return self
 
     @property
+    def schedule_bits(self) -> int:
+        """The schedule bits that change what this plan launches (under its
+        present fused setting and precision); the others have no effect."""
+        b = C.c_int()
+        _lib.check(_lib.load().decon_conv_schedule_bits(self._plan.handle, C.byref(b)))
+        return int(b.value)
+
+    @property
     def fused_yz(self) -> bool:
         """True when this plan runs the fused Y / axial cluster pass."""
         f = C.c_int()

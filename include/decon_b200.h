@@ -126,6 +126,9 @@ int decon_conv_norm_sq(const decon_conv* plan, double* out);
 #define DECON_SCHED_HALF_LINES 32
 int decon_conv_set_schedule(decon_conv* plan, int sched);
 int decon_conv_get_schedule(const decon_conv* plan, int* sched);
+/* The bits that change what this plan launches, beside its present FUSED bit
+ * and precision: schedules that differ in other bits only are the same. */
+int decon_conv_schedule_bits(const decon_conv* plan, int* bits);
 /* 1 when this plan's convolutions run the fused Y / axial pass (opt-in; one
  * thread-block cluster per kx column; canvases with Fy in {256, 512}, Fz in
  * {128, 256}, the signal in the first half of both axes, even Ny, FP32 OTF),

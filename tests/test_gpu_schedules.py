@@ -135,3 +135,18 @@ def test_fused_area_sum_at_x_lengths(D, L):
     y = down.forward(x)
     assert torch.equal(A.forward(x), down.forward(c.forward(x)))
     assert torch.equal(A.adjoint(y), c.adjoint(down.adjoint(y)))
+
+
+def test_schedule_bits_are_those_that_change_the_result_or_the_kernels(D, monkeypatch):
+    psf = np.ones((3, 5, 5), np.float32)
+    bits = lambda sig, fft, **kw: D.LinearFFTConvolver(psf, sig, fft_shape=fft, **kw).schedule_bits  # noqa: E731
+    assert bits((20, 40, 60), (40, 80, 120)) == NO_TMA
+    assert bits((40, 120, 100), (128, 256, 200)) == NO_TMA | FUSED
+    # the fused pass leaves the column kernels out; rows of 100 points run on runtime radices there
+    assert bits((40, 120, 100), (128, 256, 256), schedule=FUSED) == FUSED
+    assert bits((40, 120, 90), (128, 256, 200), schedule=FUSED) == FUSED | 16 | HALF_LINES
+    assert bits((20, 16, 30), (40, 21, 120)) == NO_TMA | 16 | HALF_LINES  # a 7-smooth axis
+    assert bits((3, 16, 30), (7, 21, 42)) == 16 | HALF_LINES
+    assert bits((30, 40, 60), (64, 80, 120), precision="mixed") == NO_TMA | 2
+    monkeypatch.setenv("DECON_NO_TMA", "1")
+    assert bits((20, 40, 60), (40, 80, 120)) == 0
