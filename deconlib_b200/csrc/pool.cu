@@ -92,6 +92,10 @@ static void release(int dev, std::vector<void*> ptrs) {
         held.insert(held.end(), ptrs.begin(), ptrs.end());
     } else {
         for (void* p : ptrs) cudaFreeAsync(p, s);
+        // what the pool does not keep goes back here, and only then do allocations
+        // outside of the pool find the rest: a cudaMalloc that would fail takes the
+        // unused memory of pools, but not what is still queued to be freed
+        cudaStreamSynchronize(s);
     }
     cudaThreadExchangeStreamCaptureMode(&mode);
     cudaGetLastError();
@@ -110,7 +114,6 @@ int pool_alloc(void** p, size_t bytes, const char* what) {
         int dev = 0;
         cudaGetDevice(&dev);
         release(dev, {});
-        cudaStreamSynchronize(s);
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(p, bytes, pool, s);
     }

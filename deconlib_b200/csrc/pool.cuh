@@ -1,8 +1,8 @@
 // Device memory of plans, solver states and scratch, from a pool per device that
 // keeps at most 2 GB between objects: a solve that builds its plan (500 MB at
 // 128x256x256) spent 1.2 ms in cudaMalloc and 1.4-4.6 ms in cudaFree.  Memory
-// above that goes back to the driver at the next synchronisation, all of it
-// when an allocation fails.  Host code only.
+// above that goes back to the driver as an object is freed, all of it when an
+// allocation fails, in the pool or (by the driver) outside of it.  Host code only.
 #pragma once
 
 #include <cuda_runtime_api.h>

@@ -376,7 +376,9 @@ class DeconServer:
     """Continuous-batching request loop (see the module docstring).
 
     ``budget_bytes``: device bytes admitted jobs (plus idle pooled plans) may
-    hold; ``max_active``: concurrent jobs (one stream each); ``chunk``:
+    hold, beside the up to 2 GB of freed memory that the library keeps for the
+    next plan (the driver takes them back for an allocation that would fail);
+    ``max_active``: concurrent jobs (one stream each); ``chunk``:
     iterations queued per job per scheduling round; ``canvas``: "static"
     (lengths 2^a x {1, 3, 5, 15}) or "reference" (the reference's canvases)."""
 

@@ -24,7 +24,7 @@ cudaError_t cudaSetDevice(int d) { device = d; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)(uintptr_t)(0x10 + device); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { note("given back"); return cudaSuccess; }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps* q) { *p = (cudaMemPool_t)(uintptr_t)(0x20 + q->location.id); return cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { note("trim"); out_of_memory = false; return cudaSuccess; }
@@ -65,22 +65,22 @@ int main() {
     pool_free({nullptr, nullptr});
     expect("nothing to free", {});
     pool_free({a, nullptr, b});
-    expect("one wait, then the buffers", {"wait 0", "free a00", "free b00"});
+    expect("one wait, then the buffers, then the pool's surplus", {"wait 0", "free a00", "free b00", "given back 0"});
     wait_ok = false;
     pool_free({a, b});
     expect("a refused wait frees nothing", {});
     wait_ok = true;
     pool_free({c});
-    expect("the held buffers go after the next wait", {"wait 0", "free c00", "free a00", "free b00"});
+    expect("the held buffers go after the next wait", {"wait 0", "free c00", "free a00", "free b00", "given back 0"});
     pool_free({c});
-    expect("and only once", {"wait 0", "free c00"});
+    expect("and only once", {"wait 0", "free c00", "given back 0"});
     wait_ok = false;
     pool_free({other});
     wait_ok = true;
     pool_free({a});
-    expect("another device's buffers stay held", {"wait 0", "free a00"});
+    expect("another device's buffers stay held", {"wait 0", "free a00", "given back 0"});
     pool_free({other});
-    expect("until that device is waited for", {"wait 0", "free 100a00", "free 100a00"});
+    expect("until that device is waited for", {"wait 0", "free 100a00", "free 100a00", "given back 0"});
     if (device != 0) ++bad, printf("device not restored\n");
     wait_ok = false;
     pool_free({a});
@@ -88,6 +88,6 @@ int main() {
     out_of_memory = true;
     void* p = nullptr;
     if (pool_alloc(&p, 64, "test") != DECON_OK || !p) ++bad, printf("allocation after a trim failed\n");
-    expect("out of memory: held buffers and the pool's own go back", {"wait 0", "free a00", "trim 0"});
+    expect("out of memory: held buffers and the pool's own go back", {"wait 0", "free a00", "given back 0", "trim 0", "given back 0"});
     return bad;
 }

@@ -38,3 +38,20 @@ def test_plan_destroyed_during_a_capture(mode, same_thread):
     # a plan made from that memory
     z = D.LinearFFTConvolver(psf, (16, 32, 32)).forward(torch.ones((16, 32, 32), device="cuda"))
     assert torch.equal(y, z)
+
+
+def test_memory_of_a_destroyed_plan_is_given_back():
+    # a plan of about 4 GB: all but the 2 GB that the pool keeps is free again
+    # when the plan is gone, without another synchronisation
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import deconlib_b200.deconvolution as D
+
+    psf = np.ones((3, 5, 5), np.float32)
+    D.LinearFFTConvolver(psf, (16, 32, 32))
+    before = torch.cuda.mem_get_info()[0]
+    plan = D.LinearFFTConvolver(psf, (380, 900, 900), fft_shape=(512, 1024, 1024))
+    held = torch.cuda.mem_get_info()[0]
+    assert before - held > 4 * 2**30
+    del plan
+    assert torch.cuda.mem_get_info()[0] > before - 2 * 2**30 - 2**28

@@ -1,6 +1,6 @@
 """The device memory pool against fakes of the CUDA calls (no GPU): memory is
-freed after the device's work is done, once per object, and is held while that
-wait is refused."""
+freed after the device's work is done, once per object, is held while that wait
+is refused, and what the pool does not keep is given back at once."""
 
 import os
 import shutil
