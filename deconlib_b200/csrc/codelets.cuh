@@ -18,41 +18,32 @@
 
 namespace dk {
 
-__device__ __forceinline__ float add(float a, float b) { return a + b; }
-__device__ __forceinline__ float sub(float a, float b) { return a - b; }
-__device__ __forceinline__ float mul(float a, float b) { return a * b; }
-__device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
-
-template <class F>
-struct Cx {
-    F re, im;
+struct C1 {
+    float re, im;
 };
-template <class F>
-__device__ __forceinline__ Cx<F> operator+(Cx<F> a, Cx<F> b) {
-    return Cx<F>{add(a.re, b.re), add(a.im, b.im)};
+__device__ __forceinline__ C1 operator+(C1 a, C1 b) {
+    return C1{a.re + b.re, a.im + b.im};
 }
-template <class F>
-__device__ __forceinline__ Cx<F> operator-(Cx<F> a, Cx<F> b) {
-    return Cx<F>{sub(a.re, b.re), sub(a.im, b.im)};
+__device__ __forceinline__ C1 operator-(C1 a, C1 b) {
+    return C1{a.re - b.re, a.im - b.im};
 }
 // a + DIR i b
-template <int DIR, class F>
-__device__ __forceinline__ Cx<F> add_i(Cx<F> a, Cx<F> b) {
-    return DIR > 0 ? Cx<F>{sub(a.re, b.im), add(a.im, b.re)} : Cx<F>{add(a.re, b.im), sub(a.im, b.re)};
+template <int DIR>
+__device__ __forceinline__ C1 add_i(C1 a, C1 b) {
+    return DIR > 0 ? C1{a.re - b.im, a.im + b.re} : C1{a.re + b.im, a.im - b.re};
 }
 // a * (c + DIR i s)
-template <int DIR, class F>
-__device__ __forceinline__ Cx<F> spin(Cx<F> a, float c, float s) {
+template <int DIR>
+__device__ __forceinline__ C1 spin(C1 a, float c, float s) {
     const float d = DIR > 0 ? s : -s;
-    return Cx<F>{mad(a.re, c, mul(a.im, -d)), mad(a.im, c, mul(a.re, d))};
+    return C1{fmaf(a.re, c, a.im * -d), fmaf(a.im, c, a.re * d)};
 }
 // a * w, or a * conj(w)
-template <bool CONJ, class F>
-__device__ __forceinline__ Cx<F> twist(Cx<F> a, float2 w) {
+template <bool CONJ>
+__device__ __forceinline__ C1 twist(C1 a, float2 w) {
     return spin<CONJ ? -1 : +1>(a, w.x, w.y);
 }
 
-typedef Cx<float> C1;
 __device__ __forceinline__ C1 as_c1(float2 v) { return C1{v.x, v.y}; }
 __device__ __forceinline__ float2 as_f2(C1 v) { return make_float2(v.re, v.im); }
 __device__ __forceinline__ C1 conj_of(C1 v) { return C1{v.re, -v.im}; }
@@ -87,8 +78,8 @@ constexpr double cos_turn(int m, int n) {
 constexpr double sin_turn(int m, int n) { return cos_turn(4 * m - n, 4 * n); }
 
 // v * exp(DIR 2 pi i M / N)
-template <int N, int M, int DIR, class F>
-__device__ __forceinline__ Cx<F> turn(Cx<F> v) {
+template <int N, int M, int DIR>
+__device__ __forceinline__ C1 turn(C1 v) {
     constexpr int m = ((M % N) + N) % N;
     if constexpr (m == 0) {
         return v;
@@ -100,66 +91,65 @@ __device__ __forceinline__ Cx<F> turn(Cx<F> v) {
 
 // ---- codelets -----------------------------------------------------------------
 
-template <class F>
-__device__ __forceinline__ void dft_2(Cx<F>& a, Cx<F>& b) {
-    const Cx<F> t = a;
+__device__ __forceinline__ void dft_2(C1& a, C1& b) {
+    const C1 t = a;
     a = t + b;
     b = t - b;
 }
-template <int DIR, class F>
-__device__ __forceinline__ void dft_4(Cx<F>& a, Cx<F>& b, Cx<F>& c, Cx<F>& d) {
-    const Cx<F> t0 = a + c, t1 = a - c, t2 = b + d, t3 = b - d;
+template <int DIR>
+__device__ __forceinline__ void dft_4(C1& a, C1& b, C1& c, C1& d) {
+    const C1 t0 = a + c, t1 = a - c, t2 = b + d, t3 = b - d;
     a = t0 + t2;
     c = t0 - t2;
     b = add_i<DIR>(t1, t3);
     d = add_i<-DIR>(t1, t3);
 }
-template <int DIR, class F>
-__device__ __forceinline__ void dft_3(Cx<F>* v) {
+template <int DIR>
+__device__ __forceinline__ void dft_3(C1* v) {
     constexpr float s3 = (float)sin_turn(1, 3);
-    const Cx<F> s = v[1] + v[2], d = v[1] - v[2];
-    const Cx<F> m{mad(s.re, -0.5f, v[0].re), mad(s.im, -0.5f, v[0].im)};
+    const C1 s = v[1] + v[2], d = v[1] - v[2];
+    const C1 m{fmaf(s.re, -0.5f, v[0].re), fmaf(s.im, -0.5f, v[0].im)};
     constexpr float k = DIR > 0 ? s3 : -s3;
     v[0] = v[0] + s;
-    v[1] = Cx<F>{mad(d.im, -k, m.re), mad(d.re, k, m.im)};
-    v[2] = Cx<F>{mad(d.im, k, m.re), mad(d.re, -k, m.im)};
+    v[1] = C1{fmaf(d.im, -k, m.re), fmaf(d.re, k, m.im)};
+    v[2] = C1{fmaf(d.im, k, m.re), fmaf(d.re, -k, m.im)};
 }
-template <int DIR, class F>
-__device__ __forceinline__ void dft_5(Cx<F>* v) {
+template <int DIR>
+__device__ __forceinline__ void dft_5(C1* v) {
     constexpr float c1 = (float)cos_turn(1, 5), c2 = (float)cos_turn(2, 5);
     constexpr float s1 = DIR > 0 ? (float)sin_turn(1, 5) : -(float)sin_turn(1, 5);
     constexpr float s2 = DIR > 0 ? (float)sin_turn(2, 5) : -(float)sin_turn(2, 5);
-    const Cx<F> b1 = v[1] + v[4], b2 = v[2] + v[3], d1 = v[1] - v[4], d2 = v[2] - v[3];
-    const Cx<F> t1{mad(b2.re, c2, mad(b1.re, c1, v[0].re)), mad(b2.im, c2, mad(b1.im, c1, v[0].im))};
-    const Cx<F> t2{mad(b2.re, c1, mad(b1.re, c2, v[0].re)), mad(b2.im, c1, mad(b1.im, c2, v[0].im))};
+    const C1 b1 = v[1] + v[4], b2 = v[2] + v[3], d1 = v[1] - v[4], d2 = v[2] - v[3];
+    const C1 t1{fmaf(b2.re, c2, fmaf(b1.re, c1, v[0].re)), fmaf(b2.im, c2, fmaf(b1.im, c1, v[0].im))};
+    const C1 t2{fmaf(b2.re, c1, fmaf(b1.re, c2, v[0].re)), fmaf(b2.im, c1, fmaf(b1.im, c2, v[0].im))};
     v[0] = v[0] + (b1 + b2);
     // i u, u = s1 d1 + s2 d2 and s2 d1 - s1 d2
-    const Cx<F> u1{mad(d2.re, s2, mul(d1.re, s1)), mad(d2.im, s2, mul(d1.im, s1))};
-    const Cx<F> u2{mad(d2.re, -s1, mul(d1.re, s2)), mad(d2.im, -s1, mul(d1.im, s2))};
+    const C1 u1{fmaf(d2.re, s2, d1.re * s1), fmaf(d2.im, s2, d1.im * s1)};
+    const C1 u2{fmaf(d2.re, -s1, d1.re * s2), fmaf(d2.im, -s1, d1.im * s2)};
     v[1] = add_i<+1>(t1, u1);
     v[4] = add_i<-1>(t1, u1);
     v[2] = add_i<+1>(t2, u2);
     v[3] = add_i<-1>(t2, u2);
 }
-template <int DIR, class F>
-__device__ __forceinline__ void dft_8(Cx<F>* v) {
+template <int DIR>
+__device__ __forceinline__ void dft_8(C1* v) {
     constexpr float h = (float)cos_turn(1, 8);
     dft_4<DIR>(v[0], v[2], v[4], v[6]);
     dft_4<DIR>(v[1], v[3], v[5], v[7]);
     // odd half: times W8^1 = h (1 + DIR i), W8^2 = DIR i, W8^3 = h (-1 + DIR i);
     // the factor h goes into the last additions
-    const Cx<F> e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
-    const Cx<F> o0 = v[1], o2 = v[5];
-    const Cx<F> p = add_i<DIR>(v[3], v[3]);   // (1 + DIR i) o1
-    const Cx<F> q = add_i<-DIR>(v[7], v[7]);  // (1 - DIR i) o3 = -(-1 + DIR i) o3
+    const C1 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
+    const C1 o0 = v[1], o2 = v[5];
+    const C1 p = add_i<DIR>(v[3], v[3]);   // (1 + DIR i) o1
+    const C1 q = add_i<-DIR>(v[7], v[7]);  // (1 - DIR i) o3 = -(-1 + DIR i) o3
     v[0] = e0 + o0;
     v[4] = e0 - o0;
     v[2] = add_i<DIR>(e2, o2);
     v[6] = add_i<-DIR>(e2, o2);
-    v[1] = Cx<F>{mad(p.re, h, e1.re), mad(p.im, h, e1.im)};
-    v[5] = Cx<F>{mad(p.re, -h, e1.re), mad(p.im, -h, e1.im)};
-    v[3] = Cx<F>{mad(q.re, -h, e3.re), mad(q.im, -h, e3.im)};
-    v[7] = Cx<F>{mad(q.re, h, e3.re), mad(q.im, h, e3.im)};
+    v[1] = C1{fmaf(p.re, h, e1.re), fmaf(p.im, h, e1.im)};
+    v[5] = C1{fmaf(p.re, -h, e1.re), fmaf(p.im, -h, e1.im)};
+    v[3] = C1{fmaf(q.re, -h, e3.re), fmaf(q.im, -h, e3.im)};
+    v[7] = C1{fmaf(q.re, h, e3.re), fmaf(q.im, h, e3.im)};
 }
 
 template <class Fn, int... I>
@@ -196,8 +186,8 @@ constexpr int codelet_split(int n) {
     }
 }
 
-template <int N, int DIR, class F>
-__device__ __forceinline__ void dftn(Cx<F>* v) {
+template <int N, int DIR>
+__device__ __forceinline__ void dftn(C1* v) {
     constexpr int A = codelet_split(N);
     if constexpr (N == 1) {
     } else if constexpr (N == 2) {
@@ -214,7 +204,7 @@ __device__ __forceinline__ void dftn(Cx<F>* v) {
         // n = (B n1 + A n2) mod N;  k = k1 mod A, k2 mod B
         constexpr int B = N / A;
         constexpr int EA = B * inverse_mod(B % A, A), EB = A * inverse_mod(A % B, B);
-        Cx<F> y[A][B];
+        C1 y[A][B];
 #pragma unroll
         for (int n1 = 0; n1 < A; ++n1) {
 #pragma unroll
@@ -223,7 +213,7 @@ __device__ __forceinline__ void dftn(Cx<F>* v) {
         }
 #pragma unroll
         for (int k2 = 0; k2 < B; ++k2) {
-            Cx<F> t[A];
+            C1 t[A];
 #pragma unroll
             for (int n1 = 0; n1 < A; ++n1) t[n1] = y[n1][k2];
             dftn<A, DIR>(t);
@@ -233,7 +223,7 @@ __device__ __forceinline__ void dftn(Cx<F>* v) {
     } else {
         // n = n1 + A n2;  k = k2 + B k1
         constexpr int B = N / A;
-        Cx<F> y[A][B];
+        C1 y[A][B];
         unrolled([&](auto i1) {
             constexpr int n1 = decltype(i1)::value;
 #pragma unroll
@@ -246,7 +236,7 @@ __device__ __forceinline__ void dftn(Cx<F>* v) {
         }, std::make_integer_sequence<int, A>{});
 #pragma unroll
         for (int k2 = 0; k2 < B; ++k2) {
-            Cx<F> t[A];
+            C1 t[A];
 #pragma unroll
             for (int n1 = 0; n1 < A; ++n1) t[n1] = y[n1][k2];
             dftn<A, DIR>(t);

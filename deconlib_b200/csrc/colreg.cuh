@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
             ok = p < a.per && o < a.nouter;
         }
 
-        Cx<float> v[R2 > R1 ? R2 : R1];
+        C1 v[R2 > R1 ? R2 : R1];
         bool arrived = true;
         if (main) {
             arrived = mbar_wait_bounded(&full, ph, a.flag);

@@ -15,7 +15,7 @@
 // (primal update) in the same form needs 130 registers and was slower than the
 // tile walk (190 vs 90 us), and rows that are not aligned gained nothing
 // consistently (voxels 32 apart: 29.3 vs 29.0 us at 60x150x210).  Float
-// operations and their order are those of hess6 (stencil.cuh): the values are
+// operations and their order are those of hess6_smem (pdhg_tiled.cuh): the values are
 // the same bits.
 #pragma once
 

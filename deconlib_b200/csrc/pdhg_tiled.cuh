@@ -13,8 +13,8 @@
 // working ring (e.g. x_bar = x + theta (x - x_prev)), and one barrier per
 // plane makes the ring visible to the CTA; the 4th ring plane lets a plane be
 // written while slower threads still read the previous three.  The
-// arithmetic is the shared stencil code with shared-memory accessors, so the
-// results equal the untiled kernels bit for bit.
+// arithmetic rounds every operation as the reference's float32 arrays do, so
+// all forms of a stencil give the same bits.
 //
 // The primal update (k_hess_primal_t: six staged y2 components, x and
 // A^T y1) keeps a one-plane register prefetch and static three-plane rings
@@ -41,9 +41,10 @@
 
 namespace dk {
 
-// Hessian components at tile-local (ly, lx) (1-based, halo at 0 and kT+1)
-// from staged planes: clamping is already in the staged values, so the taps
-// are plain neighbours; the float ops are those of hess6.
+// Weighted Hessian [zz, yy, xx, yz, xz, xy] (linops_mlx.py:224-242; d1_cen of
+// d1_cen for the mixed terms) at tile-local (ly, lx) (1-based, halo at 0 and
+// kT+1) from staged planes: clamping is already in the staged values, so the
+// taps are plain neighbours.
 __device__ __forceinline__ void hess6_smem(const float* pm, const float* p0, const float* pp, int ly,
                                            int lx, const float w[6], float h[6]) {
     const int c = ly * kHX + lx;
@@ -385,8 +386,8 @@ __global__ void __launch_bounds__(256) k_hess_regloss_p(PdhgDev* s, const float*
 // H^T y2 over this CTA's tiles from staged planes: components 0, 3, 4 (read
 // at z -+ 1) in rings of three planes, components 1, 2, 5 (read in plane z
 // only) one plane each, a one-plane register prefetch.  body(i, lt, cv)
-// receives the adjoint at interior voxel i (the float operations of
-// hess_adj_gen) and the NC centre operands cen[c][i], which are prefetched
+// receives the adjoint at interior voxel i (the six adjoint stencils of
+// linops_mlx.py:244-259, summed in its order) and the NC centre operands cen[c][i], which are prefetched
 // into registers one plane ahead with the y2 halo values (a load issued in
 // the body would wait a full memory latency per plane).
 //
@@ -541,8 +542,7 @@ __global__ void __launch_bounds__(256) k_hess_primal_t(PdhgDev* s, const float* 
     put_slot(s, s_xn2, xn2);
 }
 
-// Hessian3D.adjoint of six stored components on the staged tile walk:
-// bit-identical to the per-voxel global-memory form (hess_adj_gen).
+// Hessian3D.adjoint of six stored components on the staged tile walk.
 template <class IDX>
 __global__ void __launch_bounds__(256) k_hessian_adj_t(const float* __restrict__ hw, float* __restrict__ out,
                                                        Dims d, W6 w) {

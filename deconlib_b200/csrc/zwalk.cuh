@@ -61,7 +61,7 @@ struct StageSlots {
 // publishes the three values its neighbours' stencils take from it: the
 // field, the half central z-difference (f(z+1) - f(z-1)) / 2 and the second
 // z-difference.  Planes are double-buffered, so a plane costs one CTA
-// barrier.  Every float operation is hess6_smem's (hess6 of stencil.cuh),
+// barrier.  Every float operation is hess6_smem's (pdhg_tiled.cuh),
 // evaluated by the owner of an operand instead of its reader, so the
 // components are bit-identical to the operator's.
 //   raw(i)       -> RawT: the loads behind the fields at linear index i
