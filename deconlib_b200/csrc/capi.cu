@@ -299,7 +299,6 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
     p->npartials = std::max<int64_t>(reduce_partials_needed(), cdiv(nz * ny, std::max(1, std::min(p->T_x / 2, 4))) + 1);
     if ((st = pool_alloc((void**)&p->otf, (size_t)Fz * Fy * p->P * sizeof(float2), "OTF")) ||
         (st = pool_alloc((void**)&p->s1, (size_t)nz * ny * p->P * sizeof(float2), "spectrum S1")) ||
-        (st = pool_alloc((void**)&p->s2, (size_t)nz * Fy * p->P * sizeof(float2), "spectrum S2")) ||
         (st = pool_alloc((void**)&p->dscal, 16 * sizeof(double), "scalars")) ||
         (st = pool_alloc((void**)&p->partials, p->npartials * sizeof(double), "partials"))) {
         free_plan(p);
@@ -317,7 +316,14 @@ static int conv_create_impl(const float* kernel, const int64_t kshape[3],
     }
     // DECON_NO_TMA=1: column passes with plain loads
     p->tma = getenv("DECON_NO_TMA") == nullptr;
-    make_col_passes(*p);
+    if (!make_one_plane_pass(*p)) {
+        if ((st = pool_alloc((void**)&p->s2, (size_t)nz * Fy * p->P * sizeof(float2), "spectrum S2"))) {
+            free_plan(p);
+            delete p;
+            return st;
+        }
+        make_col_passes(*p);
+    }
     if ((st = build_otf(p, kernel, normalize, s))) {
         free_plan(p);
         delete p;

@@ -599,12 +599,16 @@ static bool make_col_pass(const ConvPlan& p, ColPass& c, const Axis& ax, int mod
     return c.ok = true;
 }
 
+// No axial transform for one plane: three launches per convolution instead of
+// five (forward + adjoint of a 512x640 frame: 59.0 -> 39.6 us), and no S2.
+bool make_one_plane_pass(ConvPlan& p) {
+    const int64_t Ny = p.N[1];
+    return p.F[0] == 1 && make_col_pass(p, p.y_otf, p.ax_y, 2, 1, p.s1, Ny, 1, (int)Ny, p.s1, Ny, (int)Ny, 1);
+}
+
 void make_col_passes(ConvPlan& p) {
     const int64_t Nz = p.N[0], Ny = p.N[1], Fy = p.F[1];
-    // no axial transform for one plane: three launches per convolution instead of
-    // five (forward + adjoint of a 512x640 frame: 59.0 -> 39.6 us)
-    if (p.F[0] == 1)
-        make_col_pass(p, p.y_otf, p.ax_y, 2, 1, p.s1, Ny, 1, (int)Ny, p.s1, Ny, (int)Ny, 1);
+    if (make_one_plane_pass(p) || !p.s2) return;
     make_col_pass(p, p.y_fwd, p.ax_y, 0, 1, p.s1, Ny, Nz, (int)Ny, p.s2, Fy, (int)Fy, Nz);
     make_col_pass(p, p.z_otf, p.ax_z, 2, 2, p.s2, Fy, Nz, (int)Nz, p.s2, Fy, (int)Nz, Fy);
     make_col_pass(p, p.y_inv, p.ax_y, 1, 1, p.s2, Fy, Nz, (int)Fy, p.s1, Ny, (int)Ny, Nz);
@@ -820,6 +824,7 @@ int spectrum_forward(const ConvPlan& p, int pro, const float* in, Win3 win, floa
     const int64_t Nz = p.N[0], Ny = p.N[1], Fy = p.F[1], P = p.P;
     if (use_yz(p)) return launch_xr2c(p, pro, in, win, cval, bg, Nz, p.s1, st, Nz * Ny);
     DK_TRY(launch_xr2c(p, pro, in, win, cval, bg, Nz, p.s1, st));
+    if (!one_plane(p) && !p.s2) return fail(DECON_ERR_CUDA, "the plan's column pass could not be prepared");
     if (one_plane(p)) return DECON_OK;  // the Y transforms run with the product (spectrum_filter_back)
     if (p.y_fwd.ok) {
         DK_TRY(launch_col_pass(p.y_fwd, false, st));

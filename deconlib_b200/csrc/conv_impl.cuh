@@ -243,6 +243,8 @@ void* pick_colfft_kernel();
 // Column passes of the plan's buffers (after they are allocated), and the
 // transform of the OTF buffer along an axis (1: y, 0: z) in place.
 void make_col_passes(ConvPlan& p);
+// The one pass of a one-plane canvas, which needs no S2; false: there is none.
+bool make_one_plane_pass(ConvPlan& p);
 void make_z_otf16(ConvPlan& p);
 int transform_otf(const ConvPlan& p, int axis, cudaStream_t st);
 

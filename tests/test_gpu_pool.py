@@ -55,3 +55,24 @@ def test_memory_of_a_destroyed_plan_is_given_back():
     assert before - held > 4 * 2**30
     del plan
     assert torch.cuda.mem_get_info()[0] > before - 2 * 2**30 - 2**28
+
+
+def test_one_plane_plan_holds_one_spectrum():
+    # 40 plans of an OTF (34 MB) and the first spectrum (33 MB); no second one (34 MB)
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import deconlib_b200.deconvolution as D
+
+    psf = np.ones((5, 5), np.float32)
+    D.LinearFFTConvolver(psf, (32, 32))
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    shape, fft = (1000, 6000), (1024, 8192)
+    plans = [D.LinearFFTConvolver(psf, shape, fft_shape=fft) for _ in range(40)]
+    pitch = 4112
+    one = (fft[0] + shape[0]) * pitch * 8  # OTF and S1
+    used = before - torch.cuda.mem_get_info()[0]
+    assert used < 40 * one * 1.05 + 2**28
+    x = torch.rand(shape, device="cuda")
+    y = plans[0].forward(x)
+    assert torch.equal(plans[0].set_schedule(4).forward(x), y)
