@@ -41,8 +41,9 @@ def test_plan_destroyed_during_a_capture(mode, same_thread):
 
 
 def test_memory_of_a_destroyed_plan_is_given_back():
-    # a plan of about 4 GB: all but the 2 GB that the pool keeps is free again
-    # when the plan is gone, without another synchronisation
+    # a plan of 5.2 GB, up to 2 GB of which the pool may have kept from plans before
+    # it: all but the 2 GB that the pool keeps is free again when the plan is gone,
+    # without another synchronisation
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     import deconlib_b200.deconvolution as D
@@ -52,7 +53,7 @@ def test_memory_of_a_destroyed_plan_is_given_back():
     before = torch.cuda.mem_get_info()[0]
     plan = D.LinearFFTConvolver(psf, (380, 900, 900), fft_shape=(512, 1024, 1024))
     held = torch.cuda.mem_get_info()[0]
-    assert before - held > 4 * 2**30
+    assert before - held > 2 * 2**30
     del plan
     assert torch.cuda.mem_get_info()[0] > before - 2 * 2**30 - 2**28
 
