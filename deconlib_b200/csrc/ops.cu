@@ -253,14 +253,17 @@ int decon_window_copy(const float* src, const int64_t* src_shape, const int64_t*
         n *= b.ds[d];
     }
     if (n == 0) return DECON_OK;
-    // a warp along a row (fewer threads for short rows): eight elements or more
-    // for each look-up of a row's place; 256 threads in all
-    int tx = 8;
+    // a warp along a row, down to one thread for the shortest: at least four elements,
+    // or the whole row, for each look-up of a row's place; 256 threads in all.  At most
+    // 32 CTAs per SM, whose threads then take several rows (1048576x3 to x2: 18.4 us;
+    // eight threads on every row in as many CTAs as it took: 66; an element per
+    // thread: 23)
+    int tx = 1;
     while (tx < 32 && 4 * tx < b.ds[3]) tx *= 2;
     const int64_t rows = n / b.ds[3];
     const dim3 block(tx, 256 / tx);
-    const dim3 grid((unsigned)std::min<int64_t>(cdiv(b.ds[3], 32 * tx), sm_count() * 8),
-                    (unsigned)std::min<int64_t>(cdiv(rows, (int64_t)block.y), 65535));
+    const int64_t gx = std::min<int64_t>(cdiv(b.ds[3], 32 * tx), sm_count() * 8);
+    const dim3 grid((unsigned)gx, (unsigned)std::min<int64_t>(cdiv(rows, (int64_t)block.y), sm_count() * 32 / gx));
     if (rows < (int64_t)1 << 31)
         DK_TRY(chain(k_window_copy<uint32_t>, grid, block, 0, as_stream(stream), src, dst, b, (uint32_t)rows));
     else
