@@ -35,8 +35,9 @@ namespace dk {
 constexpr int64_t kPsfChunkVoxels = int64_t(1) << 25;
 
 // Per column x: flags[x] = 1 if the column of the pupil holds a non-zero (or
-// its phase may not be finite: |kz| > 1e100), and the column block's share of
-// sum |P|^2 in FP64.  32 columns per CTA.
+// its phase may not be finite: |kz| > 1e100), and the block's share of sum |P|^2
+// in FP64.  32 columns per CTA; blockIdx.y: a part of the rows, with flags of its
+// own (with all rows in one CTA, 64 CTAs of a 2048x2048 pupil read it alone).
 __global__ void k_psf_support(const float2* __restrict__ pupil, const double* __restrict__ kz, int ny, int nx,
                               int* __restrict__ flags, double* __restrict__ partials) {
     __shared__ int any[32];
@@ -47,7 +48,7 @@ __global__ void k_psf_support(const float2* __restrict__ pupil, const double* __
     bool on = false;
     if (x < nx) {
 #pragma unroll 4
-        for (int y = threadIdx.y; y < ny; y += blockDim.y) {
+        for (int y = blockIdx.y * blockDim.y + threadIdx.y; y < ny; y += gridDim.y * blockDim.y) {
             const int64_t p = (int64_t)y * nx + x;
             const float2 v = pupil[p];
             acc += (double)v.x * v.x + (double)v.y * v.y;
@@ -60,18 +61,18 @@ __global__ void k_psf_support(const float2* __restrict__ pupil, const double* __
     part[threadIdx.y][threadIdx.x] = acc;
     __syncthreads();
     if (threadIdx.y == 0) {
-        if (x < nx) flags[x] = any[threadIdx.x];
+        if (x < nx) flags[(int64_t)blockIdx.y * nx + x] = any[threadIdx.x];
         double t = 0.0;
         for (int i = 0; i < 32; ++i) t += part[i][threadIdx.x];
         for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-        if (threadIdx.x == 0) partials[blockIdx.x] = t;
+        if (threadIdx.x == 0) partials[blockIdx.y * gridDim.x + blockIdx.x] = t;
     }
 }
 
 // One CTA: the columns in use as a list (act) and each column's place in it
 // (pos, -1 for a zero column), and the energy.  Every column is in use when a
 // z is not finite or huge.
-__global__ void __launch_bounds__(1024) k_psf_scan(const int* __restrict__ flags, int nx, const double* __restrict__ z,
+__global__ void __launch_bounds__(1024) k_psf_scan(const int* __restrict__ flags, int nx, int nflags, const double* __restrict__ z,
                                                    int64_t nz, const double* __restrict__ partials, int nparts,
                                                    int* __restrict__ act, int* __restrict__ pos, int* __restrict__ nact,
                                                    double* __restrict__ energy) {
@@ -85,7 +86,10 @@ __global__ void __launch_bounds__(1024) k_psf_scan(const int* __restrict__ flags
     __syncthreads();
     for (int x0 = 0; x0 < nx; x0 += blockDim.x) {
         const int x = x0 + tid;
-        const bool on = x < nx && (all || flags[x]);
+        int f = all;
+        if (x < nx)
+            for (int i = 0; i < nflags; ++i) f |= flags[(int64_t)i * nx + x];
+        const bool on = x < nx && f;
         const unsigned m = __ballot_sync(0xffffffffu, on);
         if (lane == 0) warp_base[w] = __popc(m);
         __syncthreads();
@@ -104,11 +108,12 @@ __global__ void __launch_bounds__(1024) k_psf_scan(const int* __restrict__ flags
         if (on) act[at] = x;
         __syncthreads();
     }
-    if (tid == 0) {
-        *nact = base;
+    if (tid == 0) *nact = base;
+    if (w == 0) {
         double t = 0.0;
-        for (int i = 0; i < nparts; ++i) t += partials[i];
-        *energy = t;
+        for (int i = lane; i < nparts; i += 32) t += partials[i];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) *energy = t;
     }
 }
 
@@ -157,9 +162,12 @@ extern "C" int decon_pupil_to_psf(const float* pupil, const double* kz, const do
     cudaMemPool_t pool;
     DK_TRY(device_pool(&pool));
     // scratch: complex chunk, then energy, partials, and the column lists
-    const int nparts = (int)cdiv(nx, 32);
+    // two rows or more per thread of the support search, and no more than two CTAs per SM
+    const int64_t gx = cdiv(nx, 32);
+    const int gy = (int)std::max<int64_t>(1, std::min(cdiv(ny, 64), 2 * sm_count() / gx));
+    const int nparts = (int)gx * gy;
     const size_t chunk_bytes = (size_t)round_up(chunk * nyx * (int64_t)sizeof(float2), 256);
-    const size_t bytes = chunk_bytes + (1 + nparts) * sizeof(double) + (3 * nx + 1) * sizeof(int);
+    const size_t bytes = chunk_bytes + (1 + nparts) * sizeof(double) + ((gy + 2) * nx + 1) * sizeof(int);
     char* buf = nullptr;
     auto run = [&]() -> int {
         DK_CUDA(cudaMallocFromPoolAsync((void**)&buf, bytes, pool, st));
@@ -170,10 +178,10 @@ extern "C" int decon_pupil_to_psf(const float* pupil, const double* kz, const do
         double* energy = reinterpret_cast<double*>(buf + chunk_bytes);
         double* partials = energy + 1;
         int* flags = reinterpret_cast<int*>(partials + nparts);
-        int *act = flags + nx, *pos = act + nx, *nact = pos + nx;
-        k_psf_support<<<nparts, dim3(32, 32), 0, st>>>(a.pupil, kz, (int)ny, (int)nx, flags, partials);
+        int *act = flags + gy * nx, *pos = act + nx, *nact = pos + nx;
+        k_psf_support<<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 32), 0, st>>>(a.pupil, kz, (int)ny, (int)nx, flags, partials);
         DK_LAUNCHED();
-        k_psf_scan<<<1, 1024, 0, st>>>(flags, (int)nx, z, nz, partials, nparts, act, pos, nact, energy);
+        k_psf_scan<<<1, 1024, 0, st>>>(flags, (int)nx, gy, z, nz, partials, nparts, act, pos, nact, energy);
         DK_LAUNCHED();
         const double inv_n = 1.0 / ((double)nx * (double)ny);
         a.energy = normalize ? energy : nullptr;
@@ -184,6 +192,7 @@ extern "C" int decon_pupil_to_psf(const float* pupil, const double* kz, const do
         a.nact = nact;
         a.nx = (int)nx;
         a.ny = (int)ny;
+        a.fd_L = make_fastdiv(nx);
         const PsfKernel kc = pick(axy, true), kr = pick(axx, false);
         for (int64_t z0 = 0; z0 < nz; z0 += chunk) {
             const int64_t nzc = std::min(chunk, nz - z0);

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(kDynThreads, 1) k_psf_rows_any(const __grid_co
     const int nr = left < T ? (int)left : T;
     const float2* src = a.a + row0 * L;
     for (int q = tid; q < T * L; q += blockDim.x) {
-        const int t = q / L, j = q - t * L;
+        const int t = fdiv(q, a.fd_L), j = q - t * L;
         const int p = a.pos[j];
         sm[phys(j, t, T)] = t < nr && p >= 0 ? src[(int64_t)t * L + p] : make_float2(0.f, 0.f);
     }
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kDynThreads, 1) k_psf_rows_any(const __grid_co
     const float scale = psf_scale(a);
     float* dst = a.psf + row0 * L;
     for (int q = tid; q < nr * L; q += blockDim.x) {
-        const int t = q / L, j = q - t * L;
+        const int t = fdiv(q, a.fd_L), j = q - t * L;
         const float2 v = sm[phys(j, t, T)];
         dst[q] = (v.x * v.x + v.y * v.y) * scale;
     }

@@ -15,6 +15,7 @@ struct PsfArgs {
     float* psf;            // this chunk's first plane
     const int *act, *pos, *nact;  // columns in use, each column's place or -1, their number
     int nx, ny, ntiles, T;  // T: lines per CTA of the pass
+    FastDiv fd_L;           // nx
     int64_t nrows;
     Axis ax;               // axis of the pass
     const double* energy;  // sum |P|^2 (normalize) or nullptr
