@@ -40,6 +40,7 @@ _SIGS = {
     "decon_pdhg_solver_state": (C.c_int, [_p, C.POINTER(_p), C.POINTER(C.c_int)]),
     "decon_pdhg_solver_destroy": (C.c_int, [_p]),
     "decon_test_wait_timeout": (C.c_int, [C.c_uint, _p]),
+    "decon_test_wait_drain": (C.c_int, [_p, _p, C.c_int, _p]),
     "decon_next_smooth": (_i64, [_i64]),
     "decon_fast_padded_shape": (C.c_int, [C.c_int, _i64p, _i64p, _i64p, _i64p]),
     "decon_conv_create": (C.c_int, [_p, _i64p, _i64p, _i64p, C.c_int, _p, C.POINTER(_p)]),

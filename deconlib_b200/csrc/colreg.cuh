@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
     }
 
     uint32_t ph = 0;
+    int pending = -1;  // parity of the row copy a CTA that gives up still waits for
     for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, ph ^= 1) {
         const bool main = !PLAIN && tile < a.nmain;
         const bool more = !PLAIN && tile + (int)gridDim.x < a.nmain;
@@ -167,7 +168,10 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
         // the refill is an async-proxy write over what the threads just read:
         // each orders its reads before it, then the barrier
         fence_proxy_async_smem();
-        if (!__syncthreads_and(arrived)) return;
+        if (!__syncthreads_and(arrived)) {
+            pending = ph;
+            break;
+        }
         if (tid == 0 && more) issue(tile + gridDim.x);
         if (j < R2) {
             dftn<R1, D>(v);
@@ -214,7 +218,10 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
             const float2* tw = a.tw;
             asm volatile("" : "+l"(tw));
             fence_proxy_async_smem();
-            if (!__syncthreads_and(arrived)) return;
+            if (!__syncthreads_and(arrived)) {
+                pending = more ? ph ^ 1 : ph;
+                break;
+            }
             if (tid == 0 && more) issue_otf(tile + gridDim.x);
             if (j < R1) {
                 dftn<R2, +1>(v);
@@ -235,6 +242,10 @@ __global__ void __launch_bounds__(ColRegShape<L, MODE>::NT, ColRegShape<L, MODE>
                     if (j + r * R2 < lim) dst[r * step] = as_f2(v[r]);
             }
         }
+    }
+    if (pending >= 0 && tid == 0) {
+        mbar_drain(&full, pending);
+        if constexpr (OTF) mbar_drain(&obar, ph);
     }
 }
 

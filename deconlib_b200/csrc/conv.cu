@@ -210,6 +210,28 @@ __global__ void k_wait_probe(unsigned polls) {
     if (threadIdx.x == 0) (void)mbar_wait_bounded(&bar, 0, &g_wait_timeout, polls);
 }
 
+// One CTA starts a copy of n values into shared memory, gives its wait up at once
+// and drains, as the column passes do; then hands on what has arrived.
+constexpr int kDrainProbe = 8192;
+__global__ void k_drain_probe(const float* __restrict__ src, float* __restrict__ dst, int n) {
+    __shared__ __align__(128) float buf[kDrainProbe];
+    __shared__ uint64_t bar;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        fence_proxy_async_smem();
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) buf[i] = 0.f;
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mbar_expect_tx(&bar, (uint32_t)n * 4u);
+        bulk_load(buf, src, (uint32_t)n * 4u, &bar);
+        if (!mbar_wait_bounded(&bar, 0, &g_wait_timeout, 0)) mbar_drain(&bar, 0);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = buf[i];
+}
+
 }  // namespace dk
 
 extern "C" int decon_test_wait_timeout(unsigned polls, void* stream) {
@@ -217,6 +239,17 @@ extern "C" int decon_test_wait_timeout(unsigned polls, void* stream) {
     if (polls == 0 || polls > (1u << 16))
         return fail(DECON_ERR_VALUE, "decon_test_wait_timeout: polls must be in [1, 65536]");
     k_wait_probe<<<1, 32, 0, as_stream(stream)>>>(polls);
+    DK_LAUNCHED();
+    return DECON_OK;
+}
+
+extern "C" int decon_test_wait_drain(const float* src, float* dst, int n, void* stream) {
+    using namespace dk;
+    if (!src || !dst) return fail(DECON_ERR_NULL, "null pointer");
+    if (n < 4 || n > kDrainProbe || n % 4 != 0 || (reinterpret_cast<uintptr_t>(src) & 15) != 0)
+        return fail(DECON_ERR_VALUE, "decon_test_wait_drain: n must be a multiple of 4 up to %d, src 16-byte aligned",
+                    kDrainProbe);
+    k_drain_probe<<<1, 128, 0, as_stream(stream)>>>(src, dst, n);
     DK_LAUNCHED();
     return DECON_OK;
 }

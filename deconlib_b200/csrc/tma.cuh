@@ -53,6 +53,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// For a CTA that leaves because a wait gave up: copies of its own may still be on
+// their way into shared memory that another CTA gets next.  Waits for them, bounded
+// too; by one thread, after the CTA's last barrier.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+    for (unsigned i = 0; i < kWaitLimit; ++i)
+        if (mbar_try_wait(bar, parity)) return;
+}
+
 // 3-D tiled bulk tensor load global -> shared, completion on an mbarrier.
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2,
                                             uint64_t* bar) {

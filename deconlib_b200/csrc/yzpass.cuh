@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_yz(const __grid_constant__ YZA
         }
         __syncthreads();
     }
+    if (!ok && tid == 0) mbar_drain(&bar, (uint32_t)((it - 1) & 1));
 }
 
 }  // namespace dk

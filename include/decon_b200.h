@@ -55,6 +55,10 @@ int decon_device_status_clear(void* stream);
  * leaves the context usable; decon_device_status then reports
  * DECON_ERR_TIMEOUT until decon_device_status_clear. */
 int decon_test_wait_timeout(unsigned polls, void* stream);
+/* Test of what a CTA does before it leaves after such a wait: n floats are copied
+ * from src to dst through a copy whose wait gives up at once; they arrive all the
+ * same, and decon_device_status reports the wait. */
+int decon_test_wait_drain(const float* src, float* dst, int n, void* stream);
 /* Kernels launched by this library since load (benchmark accounting). */
 int64_t decon_launch_count(void);
 
