@@ -12,6 +12,8 @@
 //   4. Y IFFT  S2 -> S1, keep the first Ny points
 //   5. X C2R   S1 -> out, keep x < Nx, scale 1/(Fz Fy Fx), fused epilogue
 //
+// On a canvas of one plane passes 2 to 4 are one, in S1, and there is no S2.
+//
 // Zero padding never exists in memory (the loads return zeros) and only the
 // Nz x Fy x (Fx/2+1) part of the spectrum that the crop can see is ever
 // formed ("pruned" FFT).  P is the spectrum row pitch: Fx/2 + 1 rounded up to

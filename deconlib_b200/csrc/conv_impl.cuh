@@ -200,7 +200,7 @@ struct ConvPlan {
     bool tma = true;  // tensor maps (DECON_NO_TMA was not set when the plan was made)
     // Mixed precision (decon_conv_set_precision): the OTF also stored as FP16
     // complex, scaled per kz plane by a power of two (OTF = otf16 * otf_inv[kz]),
-    // read by the pipelined axial pass instead of the FP32 OTF.
+    // read by the axial pass instead of the FP32 OTF.
     int precision = 0;
     __half2* otf16 = nullptr;
     float* otf_inv = nullptr;

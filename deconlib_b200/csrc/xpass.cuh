@@ -1,5 +1,5 @@
-// X passes of the lengths without a register kernel (xreg.cuh), and of the
-// kx-major spectrum of the fused Y / axial pass: real-to-complex FFT of signal
+// X passes of the lengths without a register kernel (xreg.cuh), the kx-major
+// spectrum of the fused Y / axial pass included: real-to-complex FFT of signal
 // rows (pass 1) and complex-to-real FFT back to rows with the fused
 // element-wise epilogues (pass 5), on the runtime-radix engine.
 //
